@@ -24,6 +24,7 @@
 // and walks one j-slice; small n use several j-slices whose partial sums are
 // added by k_reduce_slices (scratch memory).
 #include "aster_internal.cuh"
+#include "fp64_pair.cuh"
 #include "pn.cuh"
 
 namespace {
@@ -109,10 +110,14 @@ __global__ void __launch_bounds__(BLOCK) k_allpairs_fp64(
             for (int k = 0; k < IPT; ++k) {
                 double dx = pj.x - xi[k], dy = pj.y - yi[k], dz = pj.z - zi[k];
                 double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-                double inv = rsqrt(r2);
-                if (GUARD) inv = r2 > 0.0 ? inv : 0.0;
-                double inv2 = inv * inv;
-                double s = pj.w * inv * inv2;
+                double inv = 0.0, inv2 = 0.0, s;
+                if (PNL) {
+                    inv = inv_r(r2);
+                    inv2 = inv * inv;
+                    s = pj.w * inv * inv2;
+                } else {
+                    s = m_inv_r3(pj.w, r2);
+                }
                 ax[k] = fma(dx, s, ax[k]); ay[k] = fma(dy, s, ay[k]); az[k] = fma(dz, s, az[k]);
                 if (PNL) {
                     const double4 vj = sv[q];
@@ -384,6 +389,11 @@ int aster_allpairs_launch_range(aster_ctx* c, const aster_params* p, int precisi
     const int64_t n_src = c->n_src > 0 ? c->n_src : c->n;
     const int64_t lo = src_lo, hi = src_hi < n_src ? src_hi : n_src;
     const int64_t len = hi > lo ? hi - lo : 0;
+    if (precision == ASTER_FP64 && !targets_dev && !out_dev && lo == 0 && len == nt && nt == c->n &&
+        aster_allpairs_sym_fits(c, p)) {
+        const int st = aster_allpairs_sym_launch(c, p, closing_kick);
+        if (st != ASTER_ERR_OOM) return st;
+    }
     // one target per thread in the mixed post-Newtonian kernel, two elsewhere
     const int64_t per_block = (int64_t)BLOCK * (precision == ASTER_MIXED && pn_level(p) > 0 ? IPT_PN : IPT);
     const int64_t iblocks = (nt + per_block - 1) / per_block;

@@ -131,6 +131,8 @@ struct aster_ctx {
     // pm/vel; anything that moves positions or velocities without refreshing
     // them clears it, and a mixed all-pairs launch refreshes them first
     bool mixed_valid = false;
+    // smallest body count whose symmetric FP64 all-pairs partials did not fit
+    int64_t sym_oom_n = INT64_MAX;
     int* err_dev = nullptr;     // device error flags
     int* err_host = nullptr;    // pinned copy
     int* stack_hw_dev = nullptr;  // tree-walk stack high-water mark
@@ -187,6 +189,9 @@ int aster_allpairs_launch(aster_ctx* ctx, const aster_params* p, int precision,
                           double* out_dev /* nt*3 or null: write ctx->acc */);
 int aster_allpairs_launch_range(aster_ctx* ctx, const aster_params* p, int precision, bool closing_kick, int64_t nt,
                                 const int32_t* targets_dev, double* out_dev, int64_t src_lo, int64_t src_hi);
+// allpairs_sym.cu: FP64 forces of all bodies on all bodies, each unordered pair once
+bool aster_allpairs_sym_fits(const aster_ctx* ctx, const aster_params* p);
+int aster_allpairs_sym_launch(aster_ctx* ctx, const aster_params* p, bool closing_kick);
 // integrate.cu
 int aster_kick_drift_launch(aster_ctx* ctx, const aster_params* p, bool want_box, bool want_mixed);
 // Enqueue-only cores of the stepping entry points (argument checks included,
