@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "aster_internal.cuh"
+#include "fp64_pair.cuh"
 #include "pn.cuh"
 
 namespace {
@@ -841,30 +842,74 @@ __device__ __forceinline__ void interact2_f32(const float4 A, const float4 B, co
     az = __ffma2_rn(dz, sN, az);
 }
 
-template <bool GUARD>
-__device__ __forceinline__ void interact_f64(const double4 e, const double4 b, double eps2, double& ax, double& ay,
-                                             double& az) {
-    const double dx = e.x - b.x, dy = e.y - b.y, dz = e.z - b.z;
-    const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-    double inv = rsqrt(r2);
-    if (GUARD) inv = r2 > 0.0 ? inv : 0.0;
-    const double s = e.w * inv * inv * inv;
-    ax = fma(dx, s, ax);
-    ay = fma(dy, s, ay);
-    az = fma(dz, s, az);
+// `count` entries first, first + step, ... of a shared list on one body, FP64,
+// Q at a time so that their dependent chains overlap. CHECK: some r^2 may lie
+// outside the range of the series step (fp64_pair.cuh); one branch for the Q.
+template <bool CHECK, int Q>
+__device__ __forceinline__ void interact_list_f64(const double4* __restrict__ list, int first, int step, int count,
+                                                  const double4 b, double eps2, double& ax, double& ay, double& az) {
+#pragma unroll 1
+    for (int e = 0; e < count; e += Q) {
+        const double4* l = list + first + e * step;
+        double dx[Q], dy[Q], dz[Q], s[Q];
+        bool odd = false;
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+            const double4 c = l[k * step];
+            dx[k] = c.x - b.x; dy[k] = c.y - b.y; dz[k] = c.z - b.z;
+            const double r2 = fma(dx[k], dx[k], fma(dy[k], dy[k], fma(dz[k], dz[k], eps2)));
+            s[k] = inv_r3_fast(r2) * c.w;
+            if (CHECK) odd = odd || !r2_ordinary(r2);
+        }
+        if (CHECK && odd) {
+#pragma unroll 1
+            for (int k = 0; k < Q; ++k) {
+                const double4 c = l[k * step];
+                const double x = c.x - b.x, y = c.y - b.y, z = c.z - b.z;
+                const double t = m_inv_r3(c.w, fma(x, x, fma(y, y, fma(z, z, eps2))));
+                ax = fma(x, t, ax); ay = fma(y, t, ay); az = fma(z, t, az);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < Q; ++k) {
+                ax = fma(dx[k], s[k], ax); ay = fma(dy[k], s[k], ay); az = fma(dz[k], s[k], az);
+            }
+        }
+    }
+}
+
+// 32 list entries (the ones past the list's end massless) on a lane's two
+// bodies: c0 by all of them, c1 (when `two`) by every lps-th from `sub`.
+template <bool CHECK>
+__device__ __forceinline__ void interact32_f64(const double4* __restrict__ list, const double4 c0, const double4 c1,
+                                               bool two, int lps, int sub, double eps2, double& x0, double& y0,
+                                               double& z0, double& x1, double& y1, double& z1) {
+    interact_list_f64<CHECK, 4>(list, 0, 1, 32, c0, eps2, x0, y0, z0);
+    if (!two) return;
+    if (lps <= 8) interact_list_f64<CHECK, 4>(list, sub, lps, 32 / lps, c1, eps2, x1, y1, z1);
+    else interact_list_f64<CHECK, 1>(list, sub, lps, 32 / lps, c1, eps2, x1, y1, z1);
+}
+
+// Softened, and the root's box far inside FP64's range: every r^2 of the walk
+// lies in [1e-200, 1e200] and needs no test.
+__device__ __forceinline__ bool walk_r2_ordinary(int64_t n, const float4* __restrict__ bmin,
+                                                 const float4* __restrict__ bmax, double eps2) {
+    if (n < 2 || !(eps2 >= 1e-199 && eps2 < 1e199)) return false;
+    const float4 a = bmin[n], b = bmax[n];
+    return fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)), fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fabsf(b.z))) <
+           1e30f;
 }
 
 // One entry with a post-Newtonian force law, FP64: the Newtonian term as
 // interact_f64 forms it plus the terms pk selects (pn.cuh), all divided by G.
 // Entry e (position, mass; velocity ev) acts on the body b (velocity vi).
-template <int PNL, bool GUARD>
+template <int PNL>
 __device__ __forceinline__ void interact_pn_f64(const double4 e, const double4 ev, const double4 b, const double4 vi,
                                                 double eps2, double G, const PnK<double>& k, double& ax, double& ay,
                                                 double& az) {
     const double dx = e.x - b.x, dy = e.y - b.y, dz = e.z - b.z;
     const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-    double inv = rsqrt(r2);
-    if (GUARD) inv = r2 > 0.0 ? inv : 0.0;
+    const double inv = inv_r(r2);
     const double s = e.w * inv * inv * inv;
     ax = fma(dx, s, ax); ay = fma(dy, s, ay); az = fma(dz, s, az);
     PnPair<double> w;
@@ -952,7 +997,7 @@ __device__ __forceinline__ float2 box_dist2_pair(const float2 cx, const float2 c
 // PNL > 0: the post-Newtonian walk (the terms pk selects, with the nodes'
 // velocities node_v); PNL == 0 is the Newtonian kernel.
 template <bool MIXED, bool GUARD, bool KICK, int PNL = 0>
-__global__ void __launch_bounds__(WALK_WARPS * 32, PNL ? 4 : (MIXED ? ASTER_WALK_MINBLOCKS : 6)) k_walk(
+__global__ void __launch_bounds__(WALK_WARPS * 32, PNL ? 4 : ASTER_WALK_MINBLOCKS) k_walk(
     int64_t n, const int2* __restrict__ groups, const unsigned int* __restrict__ ngroups_p,
     unsigned int* __restrict__ work,
     const float4* __restrict__ crec, const double4* __restrict__ node_cm, const int2* __restrict__ child,
@@ -960,7 +1005,7 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, PNL ? 4 : (MIXED ? ASTER_WALK
     double4* __restrict__ vel, int* __restrict__ err, int* __restrict__ stack_hw, int stack_limit,
     int32_t* __restrict__ body_counts, unsigned long long* __restrict__ inter_count,
     const double4* __restrict__ node_v, PnK<double> pk, double4* __restrict__ pm_next, double dt_next,
-    unsigned long long* __restrict__ box_next) {
+    unsigned long long* __restrict__ box_next, const float4* __restrict__ bmin, const float4* __restrict__ bmax) {
     using Shared = typename std::conditional<PNL != 0, WalkSharedPn<MIXED>, WalkShared<MIXED>>::type;
     __shared__ Shared sm;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -971,7 +1016,8 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, PNL ? 4 : (MIXED ? ASTER_WALK
     int* stack = sm.stack[warp];
     int hw = 1;
     unsigned long long wtotal = 0;
-    double bmax = 0.0;  // fused next drift: max |coordinate| of the drifted bodies
+    double box = 0.0;  // fused next drift: max |coordinate| of the drifted bodies
+    const bool plain = !MIXED && PNL == 0 && walk_r2_ordinary(n, bmin, bmax, eps2);
 
     for (;;) {
         unsigned int g = 0;
@@ -1137,11 +1183,11 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, PNL ? 4 : (MIXED ? ASTER_WALK
                     if (two) body(nb1x, nb1y, nb1z, vf1, h1.w, sub, lps, sx1, sy1, sz1, p1, q1);
                 } else {
                     for (int e = 0; e < cnt; ++e)
-                        interact_pn_f64<PNL, GUARD>(sm.lcm[warp][e], sm.lvd[warp][e], c0, vd0, eps2, G, pk, dx0, dy0,
+                        interact_pn_f64<PNL>(sm.lcm[warp][e], sm.lvd[warp][e], c0, vd0, eps2, G, pk, dx0, dy0,
                                                     dz0);
                     if (two)
                         for (int e = sub; e < cnt; e += lps)
-                            interact_pn_f64<PNL, GUARD>(sm.lcm[warp][e], sm.lvd[warp][e], c1, vd1, eps2, G, pk, dx1,
+                            interact_pn_f64<PNL>(sm.lcm[warp][e], sm.lvd[warp][e], c1, vd1, eps2, G, pk, dx1,
                                                         dy1, dz1);
                 }
                 total += cnt;
@@ -1176,12 +1222,9 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, PNL ? 4 : (MIXED ? ASTER_WALK
                     sx1.add(ax1.x + ax1.y); sy1.add(ay1.x + ay1.y); sz1.add(az1.x + az1.y);
                 }
             } else {
-#pragma unroll 4
-                for (int e = 0; e < cnt; ++e) interact_f64<GUARD>(sm.lcm[warp][e], c0, eps2, dx0, dy0, dz0);
-                if (two) {
-#pragma unroll 4
-                    for (int e = sub; e < cnt; e += lps) interact_f64<GUARD>(sm.lcm[warp][e], c1, eps2, dx1, dy1, dz1);
-                }
+                // cnt = 32, or the rest of the list, padded to 32 by the caller
+                if (plain) interact32_f64<false>(sm.lcm[warp], c0, c1, two, lps, sub, eps2, dx0, dy0, dz0, dx1, dy1, dz1);
+                else interact32_f64<true>(sm.lcm[warp], c0, c1, two, lps, sub, eps2, dx0, dy0, dz0, dx1, dy1, dz1);
             }
             total += cnt;
         };
@@ -1303,6 +1346,7 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, PNL ? 4 : (MIXED ? ASTER_WALK
             if (lane == 0) atomicOr(err, ASTER_DEVERR_STACK);
             break;
         }
+        if (!MIXED && PNL == 0 && lane >= lc) sm.lcm[warp][lane] = make_double4(0, 0, 0, 0);  // the last 32, padded
         if (MIXED && (lc & 1) && lane == 0) {  // zero mass, zero offset: contributes nothing
             float* A = reinterpret_cast<float*>(&sm.lpa[warp][0]);
             float* B = reinterpret_cast<float*>(&sm.lpb[warp][0]);
@@ -1375,16 +1419,16 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, PNL ? 4 : (MIXED ? ASTER_WALK
                     double4 pp = pm_next[b];
                     pp.x += vv.x * dt_next; pp.y += vv.y * dt_next; pp.z += vv.z * dt_next;
                     pm_next[b] = pp;
-                    bmax = fmax(bmax, fmax(fabs(pp.x), fmax(fabs(pp.y), fabs(pp.z))));
+                    box = fmax(box, fmax(fabs(pp.x), fmax(fabs(pp.y), fabs(pp.z))));
                 }
                 vel[b] = vv;
             }
         }
     }
     if (box_next) {
-        for (int o = 16; o > 0; o >>= 1) bmax = fmax(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
+        for (int o = 16; o > 0; o >>= 1) box = fmax(box, __shfl_xor_sync(0xffffffffu, box, o));
         // non-negative doubles order like their bit patterns
-        if (lane == 0) atomicMax(box_next, (unsigned long long)__double_as_longlong(bmax));
+        if (lane == 0) atomicMax(box_next, (unsigned long long)__double_as_longlong(box));
     }
     if (lane == 0) {
         atomicMax(stack_hw, hw);
@@ -1392,9 +1436,344 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, PNL ? 4 : (MIXED ? ASTER_WALK
     }
 }
 
+// Team walk: a block of TEAM_WARPS warps per group, for trees with too few
+// groups to fill the GPU with one warp each. Warp 0 traverses (the rounds of
+// k_walk, the same lists in the same order) and hands the list over in batches
+// of WARPS - 1 chunks through a double buffer; the other warps evaluate
+// one chunk each while it goes on. A chunk is WALK_FLUSH_MIXED entries, as in
+// k_walk, so that every FP32 partial sum is the same as there; only the order
+// in which the chunks' sums are added differs (compensated FP32 per warp, FP64
+// over the warps). FP64: the list holds node ids, and each evaluating warp
+// gathers the nodes of its chunk 32 at a time, so that the traversal does not
+// wait for them. Bound by the traversal's ~85 dependent rounds a group (mixed)
+// or by the FP64 pipe (FP64); chunk, warps and resident teams are the best of
+// 64 / 96 / 128 entries, 3 to 8 warps and 2 to 6 teams per SM at 1000 to
+// 262,144 bodies (fewer teams leave FP64 the registers it would spill).
+template <bool MIXED>
+struct TeamSize {
+    static constexpr int WARPS = MIXED ? 4 : 5;
+    static constexpr int CHUNK = MIXED ? WALK_FLUSH_MIXED : 64;
+    static constexpr int BATCH = (WARPS - 1) * CHUNK;
+    static constexpr int LIST = BATCH + 64;  // a round appends up to 64 entries
+    static_assert(CHUNK >= 64 && CHUNK % 32 == 0, "the rest of a list is at most WARPS chunks");
+};
+
+template <bool MIXED>
+struct TeamShared {
+    int stack[WALK_STACK];
+    float4 lpa[2][MIXED ? TeamSize<MIXED>::LIST / 2 : 1];  // as WalkShared::lpa, lpb
+    float4 lpb[2][MIXED ? TeamSize<MIXED>::LIST / 2 : 1];
+    int lid[2][MIXED ? 1 : TeamSize<MIXED>::LIST];                // node ids
+    double4 lcm[TeamSize<MIXED>::WARPS][MIXED ? 1 : 32];          // the entries a warp evaluates
+    double sum[TeamSize<MIXED>::WARPS][6][32];
+    int cnt[2];    // entries in each buffer
+    int state[2];  // of each buffer: 0 more to come, 1 last batch, 2 stack overflow
+    unsigned int next;
+};
+
+template <bool MIXED, bool GUARD, bool KICK>
+__global__ void __launch_bounds__(TeamSize<MIXED>::WARPS * 32, MIXED ? 5 : 3) k_walk_team(
+    int64_t n, const int2* __restrict__ groups, const unsigned int* __restrict__ ngroups_p,
+    unsigned int* __restrict__ work, const float4* __restrict__ crec, const double4* __restrict__ node_cm,
+    const int2* __restrict__ child, const int32_t* __restrict__ perm, double G, double eps2, double half_dt,
+    double4* __restrict__ acc, double4* __restrict__ vel, int* __restrict__ err, int* __restrict__ stack_hw,
+    int stack_limit, int32_t* __restrict__ body_counts, unsigned long long* __restrict__ inter_count,
+    double4* __restrict__ pm_next, double dt_next, unsigned long long* __restrict__ box_next,
+    const float4* __restrict__ bmin, const float4* __restrict__ bmax) {
+    __shared__ TeamShared<MIXED> sm;
+    constexpr int TEAM_WARPS = TeamSize<MIXED>::WARPS, TEAM_CHUNK = TeamSize<MIXED>::CHUNK,
+                  TEAM_BATCH = TeamSize<MIXED>::BATCH;
+    const bool plain = !MIXED && walk_r2_ordinary(n, bmin, bmax, eps2);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    const unsigned int nbig = ngroups_p[0], ngroups = nbig + ngroups_p[3];
+    const int nI = (int)n;
+    int hw = 1;
+    unsigned long long wtotal = 0;
+    double box = 0.0;
+    if (threadIdx.x == 0) sm.next = atomicAdd(work, 1u);
+    __syncthreads();
+    for (;;) {
+        const unsigned int g = sm.next;
+        __syncthreads();
+        if (g >= ngroups) break;
+        if (threadIdx.x == 32) sm.next = atomicAdd(work, 1u);  // read after this group's barriers
+        const int2 gr = groups[g < nbig ? (int64_t)g : n - 1 - (int64_t)(g - nbig)];
+        const int r = gr.y > 32 ? gr.y - 32 : 0;
+        const bool two = r > 0;
+        int lps = 32;
+        while (lps > 1 && lps * r > 32) lps >>= 1;
+        const int sb = lane / lps, sub = lane & (lps - 1);
+        const bool v0 = lane < gr.y, v1 = two && sb < r;
+        const int64_t k0 = (int64_t)gr.x + (v0 ? lane : 0);
+        const int64_t k1 = (int64_t)gr.x + (v1 ? 32 + sb : 0);
+        const double4 c0 = node_cm[k0], c1 = two ? node_cm[k1] : c0;
+        float4 h0, l0, h1, l1;
+        leaf_trav(c0, h0, l0);
+        leaf_trav(c1, h1, l1);
+        const float glox = warp_min_f(fminf(v0 ? h0.x : INFINITY, v1 ? h1.x : INFINITY));
+        const float gloy = warp_min_f(fminf(v0 ? h0.y : INFINITY, v1 ? h1.y : INFINITY));
+        const float gloz = warp_min_f(fminf(v0 ? h0.z : INFINITY, v1 ? h1.z : INFINITY));
+        const float ghix = warp_max_f(fmaxf(v0 ? h0.x : -INFINITY, v1 ? h1.x : -INFINITY));
+        const float ghiy = warp_max_f(fmaxf(v0 ? h0.y : -INFINITY, v1 ? h1.y : -INFINITY));
+        const float ghiz = warp_max_f(fmaxf(v0 ? h0.z : -INFINITY, v1 ? h1.z : -INFINITY));
+        const float cgx = 0.5f * (glox + ghix), cgy = 0.5f * (gloy + ghiy), cgz = 0.5f * (gloz + ghiz);
+        const float3 b0 = make_float3((h0.x - cgx) + l0.x, (h0.y - cgy) + l0.y, (h0.z - cgz) + l0.z);
+        const float3 b1 = make_float3((h1.x - cgx) + l1.x, (h1.y - cgy) + l1.y, (h1.z - cgz) + l1.z);
+        CompSum sx0, sy0, sz0, sx1, sy1, sz1;
+        double dx0 = 0, dy0 = 0, dz0 = 0, dx1 = 0, dy1 = 0, dz1 = 0;
+
+        // one chunk: cnt entries from entry `from` of buffer b
+        auto evaluate = [&](int b, int from, int cnt) {
+            if constexpr (MIXED) {
+                const float4* A = sm.lpa[b] + from / 2;
+                const float4* B = sm.lpb[b] + from / 2;
+                const float2 e2 = make_float2((float)eps2, (float)eps2);
+                const float2 nb0x = make_float2(-b0.x, -b0.x), nb0y = make_float2(-b0.y, -b0.y),
+                             nb0z = make_float2(-b0.z, -b0.z);
+                const float2 nb1x = make_float2(-b1.x, -b1.x), nb1y = make_float2(-b1.y, -b1.y),
+                             nb1z = make_float2(-b1.z, -b1.z);
+                const int np = (cnt + 1) >> 1;  // an odd list has its last half slot zeroed
+                float2 ax0 = make_float2(0.f, 0.f), ay0 = ax0, az0 = ax0, ax1 = ax0, ay1 = ax0, az1 = ax0;
+                if (two && lps == 1) {
+#pragma unroll 4
+                    for (int q = 0; q < np; ++q) {
+                        interact2_f32<GUARD>(A[q], B[q], nb0x, nb0y, nb0z, e2, ax0, ay0, az0);
+                        interact2_f32<GUARD>(A[q], B[q], nb1x, nb1y, nb1z, e2, ax1, ay1, az1);
+                    }
+                } else {
+#pragma unroll WALK_UNROLL
+                    for (int q = 0; q < np; ++q)
+                        interact2_f32<GUARD>(A[q], B[q], nb0x, nb0y, nb0z, e2, ax0, ay0, az0);
+                    if (two) {
+#pragma unroll 4
+                        for (int q = sub; q < np; q += lps)
+                            interact2_f32<GUARD>(A[q], B[q], nb1x, nb1y, nb1z, e2, ax1, ay1, az1);
+                    }
+                }
+                sx0.add(ax0.x + ax0.y); sy0.add(ay0.x + ay0.y); sz0.add(az0.x + az0.y);
+                if (two) { sx1.add(ax1.x + ax1.y); sy1.add(ay1.x + ay1.y); sz1.add(az1.x + az1.y); }
+            } else {
+                const int* id = sm.lid[b] + from;
+                double4* st = sm.lcm[warp];
+                double4 nx = lane < cnt ? node_cm[id[lane]] : make_double4(0, 0, 0, 0);
+                for (int e0 = 0; e0 < cnt; e0 += 32) {
+                    __syncwarp();
+                    st[lane] = nx;
+                    __syncwarp();
+                    nx = e0 + 32 + lane < cnt ? node_cm[id[e0 + 32 + lane]] : make_double4(0, 0, 0, 0);
+                    if (plain) interact32_f64<false>(st, c0, c1, two, lps, sub, eps2, dx0, dy0, dz0, dx1, dy1, dz1);
+                    else interact32_f64<true>(st, c0, c1, two, lps, sub, eps2, dx0, dy0, dz0, dx1, dy1, dz1);
+                }
+            }
+        };
+        auto put = [&](int b, int pos, float x, float y, float z, float mass) {
+            float* A = reinterpret_cast<float*>(sm.lpa[b]);
+            float* B = reinterpret_cast<float*>(sm.lpb[b]);
+            const int o = ((pos >> 1) << 2) | (pos & 1);
+            A[o] = x;
+            A[o + 2] = y;
+            B[o] = z;
+            B[o + 2] = mass;
+        };
+
+        // the traversing warp's state
+        int top = 0, lc = 0, total = 0;
+        bool overflow = false;
+        const float2 lox2 = make_float2(glox, glox), loy2 = make_float2(gloy, gloy), loz2 = make_float2(gloz, gloz);
+        const float2 nhix2 = make_float2(-ghix, -ghix), nhiy2 = make_float2(-ghiy, -ghiy),
+                     nhiz2 = make_float2(-ghiz, -ghiz);
+        const float2 ncgx2 = make_float2(-cgx, -cgx), ncgy2 = make_float2(-cgy, -cgy), ncgz2 = make_float2(-cgz, -cgz);
+        if (warp == 0) {
+            if (n >= 2) {
+                if (lane == 0) sm.stack[0] = nI;
+                top = 1;
+            } else {
+                if (lane == 0) {
+                    if (MIXED) put(0, 0, b0.x, b0.y, b0.z, h0.w);
+                    else sm.lid[0][0] = 0;
+                }
+                lc = 1;
+            }
+            __syncwarp();
+        }
+        // traverses until buffer b holds a batch or nothing is left to open
+        auto fill = [&](int b) {
+            while (top > 0 && lc < TEAM_BATCH) {
+                const int cnt = top < 32 ? top : 32;
+                const bool act = lane < cnt;
+                int v = nI;
+                if (act) v = sm.stack[top - 1 - lane];
+                __syncwarp();
+                top -= cnt;
+                const float4* rec = crec + 4 * (int64_t)(v - nI);
+                const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2], r3 = rec[3];
+                const int2 ch = child[v];
+                const float2 cx = make_float2(r0.x, r0.y), cy = make_float2(r0.z, r0.w), cz = make_float2(r1.x, r1.y);
+                const float2 d2 = box_dist2_pair(cx, cy, cz, lox2, loy2, loz2, nhix2, nhiy2, nhiz2);
+                const bool fL = ch.x < nI || d2.x > r3.z, fR = ch.y < nI || d2.y > r3.w;
+                const bool aL = act && fL, aR = act && fR, oL = act && !fL, oR = act && !fR;
+                const uint32_t mAL = __ballot_sync(0xffffffffu, aL), mAR = __ballot_sync(0xffffffffu, aR);
+                const uint32_t mOL = __ballot_sync(0xffffffffu, oL), mOR = __ballot_sync(0xffffffffu, oR);
+                const int npush = __popc(mOL) + __popc(mOR);
+                if (top + npush > stack_limit) {
+                    overflow = true;
+                    return;
+                }
+                {
+                    const int pos = top + __popc(mOL & lt) + __popc(mOR & lt);
+                    if (oL) sm.stack[pos] = ch.x;
+                    if (oR) sm.stack[pos + (oL ? 1 : 0)] = ch.y;
+                }
+                top += npush;
+                hw = top > hw ? top : hw;
+                const int pos = lc + __popc(mAL & lt) + __popc(mAR & lt);
+                if (MIXED) {
+                    const float2 ex = __fadd2_rn(__fadd2_rn(cx, ncgx2), make_float2(r2.x, r2.y));
+                    const float2 ey = __fadd2_rn(__fadd2_rn(cy, ncgy2), make_float2(r2.z, r2.w));
+                    const float2 ez = __fadd2_rn(__fadd2_rn(cz, ncgz2), make_float2(r3.x, r3.y));
+                    if (aL) put(b, pos, ex.x, ey.x, ez.x, r1.z);
+                    if (aR) put(b, pos + (aL ? 1 : 0), ex.y, ey.y, ez.y, r1.w);
+                } else {
+                    if (aL) sm.lid[b][pos] = ch.x;
+                    if (aR) sm.lid[b][pos + (aL ? 1 : 0)] = ch.y;
+                }
+                lc += __popc(mAL) + __popc(mAR);
+                __syncwarp();
+            }
+        };
+        int b = 0;
+        bool fail = false;
+        for (;;) {
+            if (warp == 0) {
+                fill(b);
+                const bool last = overflow || top == 0;
+                if (MIXED && top == 0 && (lc & 1) && lane == 0) put(b, lc, 0.f, 0.f, 0.f, 0.f);
+                if (lane == 0) {
+                    sm.cnt[b] = lc;
+                    sm.state[b] = overflow ? 2 : last ? 1 : 0;
+                }
+            }
+            __syncthreads();  // buffer b is full; the other one has been evaluated
+            const int cnt = sm.cnt[b], state = sm.state[b];
+            if (state != 0) {
+                fail = state == 2;
+                // the rest: up to TEAM_WARPS chunks (warp 0 takes the fourth)
+                const int from = ((warp + TEAM_WARPS - 1) % TEAM_WARPS) * TEAM_CHUNK;
+                if (!fail && from < cnt) evaluate(b, from, cnt - from < TEAM_CHUNK ? cnt - from : TEAM_CHUNK);
+                total += cnt;
+                break;
+            }
+            total += TEAM_BATCH;
+            if (warp == 0) {  // carry the entries beyond the batch over
+                const int rest = lc - TEAM_BATCH;  // < 64
+                if (MIXED) {
+                    if (lane < (rest + 1) >> 1) {
+                        sm.lpa[b ^ 1][lane] = sm.lpa[b][TEAM_BATCH / 2 + lane];
+                        sm.lpb[b ^ 1][lane] = sm.lpb[b][TEAM_BATCH / 2 + lane];
+                    }
+                } else {
+                    if (lane < rest) sm.lid[b ^ 1][lane] = sm.lid[b][TEAM_BATCH + lane];
+                    if (lane + 32 < rest) sm.lid[b ^ 1][lane + 32] = sm.lid[b][TEAM_BATCH + 32 + lane];
+                }
+                lc = rest;
+                __syncwarp();
+            } else {
+                evaluate(b, (warp - 1) * TEAM_CHUNK, TEAM_CHUNK);
+            }
+            b ^= 1;  // (sm.cnt, sm.state of a buffer are rewritten two barriers after they are read)
+        }
+        if (fail) {
+            if (threadIdx.x == 0) atomicOr(err, ASTER_DEVERR_STACK);
+            break;
+        }
+        {
+            double(*s)[32] = sm.sum[warp];
+            s[0][lane] = MIXED ? sx0.value() : dx0; s[1][lane] = MIXED ? sy0.value() : dy0;
+            s[2][lane] = MIXED ? sz0.value() : dz0; s[3][lane] = MIXED ? sx1.value() : dx1;
+            s[4][lane] = MIXED ? sy1.value() : dy1; s[5][lane] = MIXED ? sz1.value() : dz1;
+        }
+        __syncthreads();
+        if (warp == 0) wtotal += (unsigned long long)total * (unsigned long long)gr.y;
+        // warp 0: bodies 0..31; warp 1: the secondary bodies
+        if (warp < 2 && (warp == 0 || two)) {
+            double ax = 0, ay = 0, az = 0;
+#pragma unroll
+            for (int w = 0; w < TEAM_WARPS; ++w) {
+                ax += sm.sum[w][3 * warp][lane];
+                ay += sm.sum[w][3 * warp + 1][lane];
+                az += sm.sum[w][3 * warp + 2][lane];
+            }
+            if (warp == 1)
+                for (int o = lps >> 1; o >= 1; o >>= 1) {
+                    ax += __shfl_xor_sync(0xffffffffu, ax, o);
+                    ay += __shfl_xor_sync(0xffffffffu, ay, o);
+                    az += __shfl_xor_sync(0xffffffffu, az, o);
+                }
+            if (warp == 0 ? v0 : (v1 && sub == 0)) {
+                ax *= G; ay *= G; az *= G;
+                const int32_t body = perm[warp == 0 ? k0 : k1];
+                acc[body] = make_double4(ax, ay, az, 0.0);
+                if (body_counts) body_counts[body] = total;
+                if (KICK) {
+                    double4 vv = vel[body];
+                    vv.x += ax * half_dt; vv.y += ay * half_dt; vv.z += az * half_dt;
+                    if (pm_next) {  // the next step's opening kick and drift, as in k_walk
+                        vv.x += ax * half_dt; vv.y += ay * half_dt; vv.z += az * half_dt;
+                        double4 pp = pm_next[body];
+                        pp.x += vv.x * dt_next; pp.y += vv.y * dt_next; pp.z += vv.z * dt_next;
+                        pm_next[body] = pp;
+                        box = fmax(box, fmax(fabs(pp.x), fmax(fabs(pp.y), fabs(pp.z))));
+                    }
+                    vel[body] = vv;
+                }
+            }
+        }
+        // the next group's first barrier orders these reads of sm.sum before its writes
+    }
+    if (box_next && warp < 2) {
+        for (int o = 16; o > 0; o >>= 1) box = fmax(box, __shfl_xor_sync(0xffffffffu, box, o));
+        if (lane == 0) atomicMax(box_next, (unsigned long long)__double_as_longlong(box));
+    }
+    if (threadIdx.x == 0) {
+        atomicMax(stack_hw, hw);
+        atomicAdd(inter_count, wtotal);
+    }
+}
+
+// Up to these sizes a tree has too few groups for one warp each (mixed: 740
+// resident teams against 2960 warps, about 3000 groups at 10^5 bodies).
+// Walk at theta = 0.5, k_walk against the team, us: mixed 5000 bodies 82, 46;
+// 20,011: 125, 66; 60,000: 196, 135; 100,000: 238, 201; 131,073: 244, 248;
+// 262,144: 432, 480. FP64 5000: 164, 64; 20,011: 225, 98; 60,000: 391, 236;
+// 131,073: 580, 492; 262,144: 942, 948; 1,048,576: 3556, 4002.
+constexpr int64_t TEAM_MAX_MIXED = 120000, TEAM_MAX_FP64 = 200000;
+
+template <bool MIXED, bool GUARD, bool KICK>
+int launch_team(aster_ctx* c, const aster_params* p, int32_t* counts, bool fuse_next) {
+    LbvhBufs& t = c->tree;
+    auto kern = k_walk_team<MIXED, GUARD, KICK>;
+    int per_sm = 0;
+    ASTER_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TeamSize<MIXED>::WARPS * 32, 0));
+    if (per_sm < 1) per_sm = 1;
+    const int64_t blocks = std::min<int64_t>((int64_t)c->sm_count * per_sm, c->n);  // groups <= n
+    unsigned int* gcount = red_groups(c);
+    kern<<<(unsigned)blocks, TeamSize<MIXED>::WARPS * 32, 0, c->stream>>>(
+        c->n, t.groups.as<int2>(), gcount, gcount + 1, t.crec.as<float4>(), t.node_cm.as<double4>(),
+        t.child.as<int2>(), t.perm.as<int32_t>(), p->G, p->eps2, 0.5 * p->dt, c->acc.as<double4>(),
+        c->vel.as<double4>(), c->err_dev, c->stack_hw_dev, c->walk_stack_limit, counts, red_inter(c),
+        KICK && fuse_next ? c->pm.as<double4>() : nullptr, p->dt, KICK && fuse_next ? red_box(c) : nullptr,
+        t.bmin.as<float4>(), t.bmax.as<float4>());
+    ASTER_CUDA(cudaGetLastError());
+    return ASTER_OK;
+}
+
 template <bool MIXED, bool GUARD, bool KICK, int PNL = 0>
 int launch_walk(aster_ctx* c, const aster_params* p, int32_t* counts, bool fuse_next) {
     LbvhBufs& t = c->tree;
+    if constexpr (PNL == 0) {
+        if (c->n <= (MIXED ? TEAM_MAX_MIXED : TEAM_MAX_FP64)) return launch_team<MIXED, GUARD, KICK>(c, p, counts, fuse_next);
+    }
     auto kern = k_walk<MIXED, GUARD, KICK, PNL>;
     int per_sm = 0;
     ASTER_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WALK_WARPS * 32, 0));
@@ -1408,7 +1787,8 @@ int launch_walk(aster_ctx* c, const aster_params* p, int32_t* counts, bool fuse_
         t.crec.as<float4>(), t.node_cm.as<double4>(), t.child.as<int2>(), t.perm.as<int32_t>(), p->G, p->eps2, 0.5 * p->dt,
         c->acc.as<double4>(), c->vel.as<double4>(), c->err_dev, c->stack_hw_dev, c->walk_stack_limit, counts,
         red_inter(c), PNL > 0 ? t.node_v.as<double4>() : nullptr, make_pn(p),
-        KICK && fuse_next ? c->pm.as<double4>() : nullptr, p->dt, KICK && fuse_next ? red_box(c) : nullptr);
+        KICK && fuse_next ? c->pm.as<double4>() : nullptr, p->dt, KICK && fuse_next ? red_box(c) : nullptr,
+        t.bmin.as<float4>(), t.bmax.as<float4>());
     ASTER_CUDA(cudaGetLastError());
     return ASTER_OK;
 }
