@@ -69,7 +69,7 @@ struct LbvhBufs {
     DevBuf codes, codes_alt, sorted_codes, perm, perm_alt, hist, digit_off;
     DevBuf parent, sib, rlo, rhi, counters;
     DevBuf node_cm, bmin, bmax;  // node_cm: double4 (com x, y, z, mass)
-    DevBuf child, groups, crec, front;
+    DevBuf child, groups, crec, front, dl;
     DevBuf node_v;  // double4 (vx, vy, vz, 0) per node: post-Newtonian walk only
     int64_t n = 0;
     bool built = false;
@@ -213,7 +213,8 @@ int64_t aster_energy_parts(const aster_ctx* ctx);
 int aster_kick_drift_coef(aster_ctx* ctx, double kick_dt, double drift_dt, bool kick, bool want_box,
                           bool want_mixed);
 // lbvh.cu
-int aster_lbvh_build_dev(aster_ctx* ctx, const aster_params* p, bool box_ready);
+// links: also parents, siblings and leaf ranges (the exported tree; post-Newtonian laws imply it)
+int aster_lbvh_build_dev(aster_ctx* ctx, const aster_params* p, bool box_ready, bool links = false);
 // fuse_next (with closing_kick): the walk also applies the next step's
 // opening kick and drift to every body and leaves their bounding box in
 // red_box, so that step's kick-drift launch is left out.

@@ -12,14 +12,12 @@
 //   sort     stable LSD radix sort of (code, body index), 8-bit digits:
 //            per pass a tile histogram, a per-digit scan over tiles, a stable
 //            scatter (warp match-any ranking). Ties keep body-index order.
-//   karras   Karras (2012) node split exactly as barnes_hut.cpp:338-396
-//            (tie-break 32 + clz(i ^ j) on sorted positions), children,
-//            parents and leaf ranges; the same kernel gathers the leaves.
-//   bottomup one thread per leaf climbs with an atomic arrival counter per
-//            node; the second arrival merges the children: FP64 mass and
-//            centre of mass in NodesArray::unite order (barnes_hut.cpp:137-152,
-//            bit-exact), FP32 AABB, squared opening radius
-//            r_crit = l/theta + |com - box centre| (rounded up to FP32).
+//   tree     Karras' (2012) tree exactly as barnes_hut.cpp:338-396 (tie-break
+//            32 + clz(i ^ j) on sorted positions), built bottom up: climbs
+//            meet at their parent's split and the second arrival merges the
+//            children: FP64 mass and centre of mass in NodesArray::unite order
+//            (barnes_hut.cpp:137-152, bit-exact), FP32 AABB, squared opening
+//            radius r_crit = l/theta + |com - box centre| (rounded up to FP32).
 //   walk     one warp per group (a subtree of <= 64 leaves whose parent holds
 //            more): a shared-memory stack walk that opens a node for the whole
 //            group unless its FP32 centre of mass lies farther than r_crit
@@ -376,14 +374,43 @@ __device__ __forceinline__ void put_child_record(float4* __restrict__ dst, int64
     dst[3] = make_float4(lL.z, lR.z, lL.w, lR.w);
 }
 
-// -------------------------------------------------------------- karras
+// ---------------------------------------------------------------- tree
+// The tree Karras (2012) builds top down (barnes_hut.cpp:338-396), built bottom
+// up together with the node data: a node [lo, hi] of the radix tree over the
+// sorted codes is its parent's left child when delta(hi, hi+1) > delta(lo-1, lo)
+// (delta: common prefix of neighbouring augmented keys), so a climb finds its
+// parent's split, hi or lo - 1, from two values, and the two children of a node
+// meet at its split (Apetrei 2014). Node numbers are Karras': a left child has
+// its last leaf's index, a right child its first leaf's, the root 0 (each + n).
+// The same trees bit for bit, without the searches of the top-down form (57 us
+// of the build at 2^20 bodies) and without links to read on the way up.
+//
+// k_tree_local: a block merges what it can of TREE_LEAVES consecutive leaves;
+// the subtrees left over ("frontier": their sibling lies outside) go out in leaf
+// order. k_tree_merge, launched until one block is left: a block takes the
+// frontiers of several neighbouring blocks as items and merges on, climbs again
+// meeting through shared memory. Rank r of an item and its first leaf lo(r)
+// give every range: items tile their region. What bounds it: a chain of
+// dependent merges (about 31 levels at 2^20 bodies, three divisions each);
+// before, every level between the 64-leaf blocks and the root was an
+// acquire-release atomic and a dependent load at L2 (54 us at 131,072 bodies,
+// 59 at 2^20). Climbing through global memory in these kernels took as long
+// again; with node data, deltas and exchanges in shared memory a level is about
+// 0.5 us. Build per graph-replayed step, before and after: 2000 bodies 98.7 ->
+// 71.6 us, 20,011 115.6 -> 93.7, 131,073 132.5 -> 108.9, 2^20 315 -> 273.
+constexpr int TREE_LEAVES = 64;
+constexpr int MERGE_FAN_MAX = 256;  // input blocks per block at most
+// Items a merge holds in shared memory: 512 leave two blocks per SM, 1344 take
+// one block's 227 KB (the last merge). More items (clustered bodies) go through
+// global memory.
+constexpr int MERGE_CAP = 512, MERGE_CAP_LAST = 1344;
+constexpr int MERGE_THREADS = 512;
+
+// delta of the neighbours at sorted positions i, i + 1 (codes a, b, bodies pa, pb)
 template <class KeyT, bool COMPAT>
-__device__ __forceinline__ int kdelta(const KeyT* __restrict__ codes, const int32_t* __restrict__ perm,
-                                      int64_t n, int64_t i, int64_t j) {
-    if (j < 0 || j >= n) return -1;
-    const KeyT a = codes[i], b = codes[j];
+__device__ __forceinline__ int neighbour_delta(KeyT a, KeyT b, int64_t i, int32_t pa, int32_t pb) {
     if (a == b) {
-        const uint32_t t = COMPAT ? (uint32_t)(perm[i] ^ perm[j]) : (uint32_t)(i ^ j);
+        const uint32_t t = COMPAT ? (uint32_t)(pa ^ pb) : (uint32_t)(i ^ (i + 1));
         return (sizeof(KeyT) == 8 ? 64 : 32) + __clz((int)t);
     }
     return sizeof(KeyT) == 8 ? __clzll((long long)(a ^ b)) : __clz((int)(uint32_t)(a ^ b));
@@ -393,14 +420,11 @@ __device__ __forceinline__ int kdelta(const KeyT* __restrict__ codes, const int3
 // parent's holds more (the root when n <= GROUP_MAX). Its leaves are a
 // contiguous sorted run sharing a Morton prefix, so the group is spatially
 // compact (a fixed run of consecutive sorted bodies is not: it can straddle a
-// Morton jump and span the whole system). Listed here as (first leaf, size):
-// internal node n + i knows its own range and both children's, and thread i
-// lists the groups among its children, so groups come roughly in sorted-leaf
-// order, which keeps consecutive walk groups close in space. Groups of more
-// than 32 bodies (a second pass over the list, or two bodies per lane) fill
-// the array from the front, groups of at most 32 (one pass) from the back;
-// the walk takes the front part first, so its last wave is made of the
-// cheaper groups and warps finish closer together.
+// Morton jump and span the whole system). Listed here as (first leaf, size)
+// where the parent is merged. Groups of more than 32 bodies (a second pass over
+// the list, or two bodies per lane) fill the array from the front, groups of at
+// most 32 (one pass) from the back; the walk takes the front part first, so its
+// last wave is made of the cheaper groups and warps finish closer together.
 constexpr int GROUP_SMALL = 32;
 __device__ __forceinline__ void list_group(int2* groups, unsigned int* ngroups, int64_t n, int64_t first,
                                            int64_t size) {
@@ -409,92 +433,47 @@ __device__ __forceinline__ void list_group(int2* groups, unsigned int* ngroups, 
     else
         groups[n - 1 - atomicAdd(&ngroups[3], 1u)] = make_int2((int32_t)first, (int32_t)size);
 }
-template <class KeyT, bool COMPAT>
-__global__ void __launch_bounds__(256) k_karras(int64_t n, const KeyT* __restrict__ codes, const int32_t* __restrict__ perm,
-                                                const double4* __restrict__ pm, int32_t* __restrict__ parent,
-                                                int32_t* __restrict__ sib, int32_t* __restrict__ rlo, int32_t* __restrict__ rhi,
-                                                int2* __restrict__ child, uint32_t* __restrict__ counters,
-                                                double4* __restrict__ node_cm, int2* __restrict__ groups,
-                                                unsigned int* __restrict__ ngroups) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        // leaf i: gather body perm[i]
-        {
-            node_cm[i] = pm[perm[i]];
-            rlo[i] = (int32_t)i;
-            rhi[i] = (int32_t)i;
-            if (n == 1) {
-                parent[0] = -1;
-                list_group(groups, ngroups, n, 0, 1);
-            }
-        }
-        if (i == n - 1) {
-            parent[n] = -1;  // root (n >= 2) or unused slot
-            continue;
-        }
-        const int dl = i == 0 ? -1 : kdelta<KeyT, COMPAT>(codes, perm, n, i, i - 1);
-        const int dr = kdelta<KeyT, COMPAT>(codes, perm, n, i, i + 1);
-        const int64_t d = dr > dl ? 1 : -1;
-        const int dmin = d == 1 ? dl : dr;
-        int64_t lmax = 2;
-        while (kdelta<KeyT, COMPAT>(codes, perm, n, i, i + lmax * d) > dmin) lmax *= 2;
-        int64_t l = 0;
-        for (int64_t t = lmax / 2; t >= 1; t /= 2)
-            if (kdelta<KeyT, COMPAT>(codes, perm, n, i, i + (l + t) * d) > dmin) l += t;
-        const int64_t j = i + l * d;
-        const int dnode = kdelta<KeyT, COMPAT>(codes, perm, n, i, j);
-        int64_t s = 0;
-        const int64_t range = j > i ? j - i : i - j;
-        for (int64_t t = (range + 1) / 2; t >= 1; t = (t + 1) / 2) {
-            if (kdelta<KeyT, COMPAT>(codes, perm, n, i, i + (s + t) * d) > dnode) s += t;
-            if (t == 1) break;
-        }
-        const int64_t gamma = i + s * d + (d < 0 ? d : 0);
-        const int64_t lo = i < j ? i : j, hi = i < j ? j : i;
-        const int64_t node = n + i;
-        const int32_t L = (int32_t)(lo == gamma ? gamma : n + gamma);
-        const int32_t R = (int32_t)(hi == gamma + 1 ? gamma + 1 : n + gamma + 1);
-        child[node] = make_int2(L, R);
-        parent[L] = (int32_t)node;
-        parent[R] = (int32_t)node;
-        sib[L] = R;   // >= 0: the node is a left child
-        sib[R] = ~L;  // <  0: a right child, sibling ~sib
-        rlo[node] = (int32_t)lo;
-        rhi[node] = (int32_t)hi;
-        counters[i] = 0u;
-        if (hi - lo + 1 > GROUP_MAX) {
-            const int64_t szL = gamma - lo + 1, szR = hi - gamma;
-            if (szL <= GROUP_MAX) list_group(groups, ngroups, n, lo, szL);
-            if (szR <= GROUP_MAX) list_group(groups, ngroups, n, gamma + 1, szR);
-        } else if (i == 0) {  // the root holds at most GROUP_MAX leaves
-            list_group(groups, ngroups, n, 0, n);
-        }
+
+// (x, y, z) / m, each correctly rounded as __ddiv_rn, from one correctly rounded
+// reciprocal: q = a y, then q + (a - m q) y twice with fused multiply-adds. The
+// first correction leaves q within an ulp of a / m, and from there, y being the
+// rounded 1 / m, the second one gives the rounded quotient (Markstein 1990).
+// Components or masses outside [2^-400, 2^400), where a step could leave the
+// normal range, take the division itself. Three divisions were the longest part
+// of a merge's serial chain.
+__device__ __forceinline__ bool mid_range(double v) {
+    return (unsigned)((__double2hiint(v) & 0x7fffffff) - ((1023 - 400) << 20)) < (800u << 20);
+}
+__device__ __forceinline__ void div3_rn(double& x, double& y, double& z, double m) {
+    const double r = __drcp_rn(m);
+    double qx = __dmul_rn(x, r), qy = __dmul_rn(y, r), qz = __dmul_rn(z, r);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        qx = __fma_rn(__fma_rn(-m, qx, x), r, qx);
+        qy = __fma_rn(__fma_rn(-m, qy, y), r, qy);
+        qz = __fma_rn(__fma_rn(-m, qz, z), r, qz);
     }
+    if (!(mid_range(x) && mid_range(y) && mid_range(z) && mid_range(m))) {
+        qx = __ddiv_rn(x, m);
+        qy = __ddiv_rn(y, m);
+        qz = __ddiv_rn(z, m);
+    }
+    x = qx;
+    y = qy;
+    z = qz;
 }
 
-// ------------------------------------------------------------ bottom-up
-__device__ __forceinline__ double4 ld_cg(const double4* p) {
-    const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
-    const double2 b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
-    return make_double4(a.x, a.y, b.x, b.y);
+// Exchange on a shared-memory slot where two climbs meet: its release half
+// publishes the climb's node data (shared memory), its acquire half makes the
+// first arrival's visible to the second.
+__device__ __forceinline__ int meet(int* slot, int mine) {
+    int old;
+    asm volatile("atom.acq_rel.cta.shared.exch.b32 %0, [%1], %2;"
+                 : "=r"(old)
+                 : "r"((unsigned)__cvta_generic_to_shared(slot)), "r"(mine)
+                 : "memory");
+    return old;
 }
-__device__ __forceinline__ float4 ld_cg(const float4* p) { return __ldcg(p); }
-
-// Bottom-up merge: every leaf climbs towards the root; at each internal node
-// the first arrival stops and the second merges the two children in
-// NodesArray::unite order. Two phases, so that the climbs through global
-// memory are short and all in flight at once:
-//  1. k_bottom_up_local: a block owns BU_LEAVES consecutive sorted leaves and
-//     completes every node whose leaf range lies inside them, with arrival
-//     counters and node data in shared memory (block-scope fences). A node
-//     whose parent's range leaves the block is a frontier node.
-//  2. k_bottom_up_front: one climb per frontier node through the remaining
-//     (boundary-crossing) nodes with global counters and device-scope fences.
-// sib[v] names v's sibling and side (>= 0: v is a left child), so a climb
-// reads both children without loading child[parent] first.
-#ifndef ASTER_BU_LEAVES
-#define ASTER_BU_LEAVES 64
-#endif
-constexpr int BU_LEAVES = ASTER_BU_LEAVES;
 
 __device__ __forceinline__ void bu_merge(const double4 cl, const double4 cr, const float4 l0, const float4 l1,
                                          const float4 h0, const float4 h1, double4& cm, float4& lo, float4& hi) {
@@ -504,9 +483,10 @@ __device__ __forceinline__ void bu_merge(const double4 cl, const double4 cr, con
     // finite too (unite leaves such a node's previous contents in place).
     const double M = __dadd_rn(cr.w, cl.w);
     if (M > 0.0) {
-        cm.x = __ddiv_rn(__dadd_rn(__dmul_rn(cr.x, cr.w), __dmul_rn(cl.x, cl.w)), M);
-        cm.y = __ddiv_rn(__dadd_rn(__dmul_rn(cr.y, cr.w), __dmul_rn(cl.y, cl.w)), M);
-        cm.z = __ddiv_rn(__dadd_rn(__dmul_rn(cr.z, cr.w), __dmul_rn(cl.z, cl.w)), M);
+        cm.x = __dadd_rn(__dmul_rn(cr.x, cr.w), __dmul_rn(cl.x, cl.w));
+        cm.y = __dadd_rn(__dmul_rn(cr.y, cr.w), __dmul_rn(cl.y, cl.w));
+        cm.z = __dadd_rn(__dmul_rn(cr.z, cr.w), __dmul_rn(cl.z, cl.w));
+        div3_rn(cm.x, cm.y, cm.z, M);
     } else {
         cm.x = __dmul_rn(0.5, __dadd_rn(cr.x, cl.x));
         cm.y = __dmul_rn(0.5, __dadd_rn(cr.y, cl.y));
@@ -517,173 +497,396 @@ __device__ __forceinline__ void bu_merge(const double4 cl, const double4 cr, con
     hi = make_float4(fmaxf(h0.x, h1.x), fmaxf(h0.y, h1.y), fmaxf(h0.z, h1.z), 0.f);
 }
 
-__global__ void __launch_bounds__(BU_LEAVES, 1024 / BU_LEAVES) k_bottom_up_local(
-    int64_t n, const int32_t* __restrict__ parent, const int32_t* __restrict__ sib, const int32_t* __restrict__ rlo,
-    const int32_t* __restrict__ rhi, double4* __restrict__ node_cm, float4* __restrict__ bmin,
-    float4* __restrict__ bmax, int32_t* __restrict__ front, unsigned int* __restrict__ nfront, int* __restrict__ err,
-    double theta, const int2* __restrict__ child, float4* __restrict__ crec) {
-    // [0][j]: leaf B0 + j; [1][j]: internal node n + B0 + j (Karras numbering:
-    // an internal node inside the block has its index inside the block too)
-    __shared__ double4 s_cm[2][BU_LEAVES];
-    __shared__ float4 s_lo[2][BU_LEAVES], s_hi[2][BU_LEAVES];
-    __shared__ int32_t s_par[2][BU_LEAVES], s_sib[2][BU_LEAVES];
-    __shared__ int32_t s_rlo[BU_LEAVES], s_rhi[BU_LEAVES];
-    __shared__ unsigned int s_cnt[BU_LEAVES];
-    __shared__ int32_t s_front[BU_LEAVES];  // frontier nodes are disjoint subtrees: at most one per leaf
-    __shared__ unsigned int s_nf, s_fbase;
-    const int j = threadIdx.x;
-    const int64_t B0 = (int64_t)blockIdx.x * BU_LEAVES;
-    const int64_t B1 = (B0 + BU_LEAVES < n ? B0 + BU_LEAVES : n) - 1;
-    const int64_t k = B0 + j;
-    s_cnt[j] = 0u;
-    if (j == 0) s_nf = 0u;
-    if (k < n) {
-        const double4 lc = node_cm[k];
-        s_cm[0][j] = lc;
-        s_lo[0][j] = leaf_lo(lc);
-        s_hi[0][j] = leaf_hi(lc);
-        s_par[0][j] = parent[k];
-        s_sib[0][j] = sib[k];
+// The node arrays. LINKS: also parent, sib (>= 0: a left child's sibling; < 0: a
+// right child's, complemented) and the leaf ranges, which only the exported
+// tree and the post-Newtonian node velocities read.
+struct TreeOut {
+    double4* node_cm;
+    float4 *bmin, *bmax;
+    int2* child;
+    float4* crec;
+    int32_t *parent, *sib, *rlo, *rhi;
+    int2* groups;
+    unsigned int* ngroups;
+    int* err;
+};
+
+// lists the walk groups among a node's children [l0, l1) and [l1, l2)
+__device__ __forceinline__ void list_children(const TreeOut& o, int64_t n, int64_t l0, int64_t l1, int64_t l2) {
+    if (l2 - l0 <= GROUP_MAX) return;
+    if (l1 - l0 <= GROUP_MAX) list_group(o.groups, o.ngroups, n, l0, l1 - l0);
+    if (l2 - l1 <= GROUP_MAX) list_group(o.groups, o.ngroups, n, l1, l2 - l1);
+}
+
+template <bool LINKS>
+__device__ __forceinline__ void put_links(const TreeOut& o, int32_t id, int32_t L, int32_t R, int64_t lo, int64_t hi) {
+    if (LINKS) {
+        o.parent[L] = id;
+        o.parent[R] = id;
+        o.sib[L] = R;
+        o.sib[R] = ~L;
+        o.rlo[id] = (int32_t)lo;
+        o.rhi[id] = (int32_t)hi;
     }
-    if (k < n - 1) {
-        s_par[1][j] = parent[n + k];
-        s_sib[1][j] = sib[n + k];
-        s_rlo[j] = rlo[n + k];
-        s_rhi[j] = rhi[n + k];
+}
+
+// front[B0 + r] = (node, first leaf) of the block's r-th frontier subtree,
+// nfront[block] their number; dl[k] = delta(k, k + 1), -1 at the end.
+template <class KeyT, bool COMPAT, bool LINKS>
+__global__ void __launch_bounds__(TREE_LEAVES, 1024 / TREE_LEAVES) k_tree_local(
+    int64_t n, double theta, const KeyT* __restrict__ codes, const int32_t* __restrict__ perm,
+    const double4* __restrict__ pm, TreeOut o, signed char* __restrict__ dl, int2* __restrict__ front,
+    int32_t* __restrict__ nfront) {
+    // [0][j]: leaf B0 + j; [1][j]: the node whose children meet between leaves B0 + j and B0 + j + 1
+    __shared__ double4 s_cm[2][TREE_LEAVES];
+    __shared__ float4 s_lo[2][TREE_LEAVES], s_hi[2][TREE_LEAVES];
+    __shared__ int s_slot[TREE_LEAVES], s_kids[TREE_LEAVES];
+    __shared__ int32_t s_id[TREE_LEAVES], s_fid[TREE_LEAVES];
+    __shared__ int s_rng[TREE_LEAVES];
+    __shared__ signed char s_dl[TREE_LEAVES + 1];  // [j]: delta(B0 + j - 1, B0 + j)
+    __shared__ int s_warp[TREE_LEAVES / 32];
+    const int j = threadIdx.x;
+    const int64_t B0 = (int64_t)blockIdx.x * TREE_LEAVES, k = B0 + j;
+    const int cnt = (int)(n - B0 < TREE_LEAVES ? n - B0 : TREE_LEAVES);
+    const bool in = j < cnt;
+    s_slot[j] = 0;
+    s_id[j] = -1;
+    s_fid[j] = -1;
+    double4 cm = make_double4(0, 0, 0, 0);
+    float4 blo = make_float4(0, 0, 0, 0), bhi = blo;
+    if (in) {
+        const int32_t pk = perm[k];
+        const KeyT ck = codes[k];
+        const int d = k == 0 ? -1 : neighbour_delta<KeyT, COMPAT>(codes[k - 1], ck, k - 1, COMPAT ? perm[k - 1] : 0, pk);
+        s_dl[j] = (signed char)d;
+        if (k > 0) dl[k - 1] = (signed char)d;
+        if (k == n - 1) dl[k] = -1;
+        if (j == cnt - 1)
+            s_dl[cnt] = (signed char)(k == n - 1 ? -1
+                                                 : neighbour_delta<KeyT, COMPAT>(ck, codes[k + 1], k, pk,
+                                                                                 COMPAT ? perm[k + 1] : 0));
+        cm = pm[pk];
+        blo = leaf_lo(cm);
+        bhi = leaf_hi(cm);
+        o.node_cm[k] = cm;
+        s_cm[0][j] = cm;
+        s_lo[0][j] = blo;
+        s_hi[0][j] = bhi;
+        if (LINKS) o.rlo[k] = o.rhi[k] = (int32_t)k;
     }
     __syncthreads();
-    int side = 0, slot = j;
-    int32_t cur = (int32_t)k;
-    double4 cm = make_double4(0, 0, 0, 0);
-    float4 lo = make_float4(0, 0, 0, 0), hi = lo;
-    if (k < n) {
-        cm = s_cm[0][j];
-        lo = s_lo[0][j];
-        hi = s_hi[0][j];
-    }
-    for (int level = 0; k < n; ++level) {
-        const int32_t par = s_par[side][slot];
-        if (par < 0) break;  // the root
-        const int64_t ip = (int64_t)par - n;
-        const bool local = ip >= B0 && ip <= B1 && s_rlo[ip - B0] >= B0 && s_rhi[ip - B0] <= B1;
-        if (!local) {
-            s_front[atomicAdd(&s_nf, 1u)] = cur;  // its data is in global memory already
+    int lo = j, hi = j, loc = j;
+    int32_t id = (int32_t)k;
+    for (int level = 0; in; ++level) {
+        const int dL = s_dl[lo], dR = s_dl[hi + 1];
+        if (dL < 0 && dR < 0) {  // the root
+            if (n <= GROUP_MAX) list_group(o.groups, o.ngroups, n, 0, n);
+            if (LINKS) {
+                o.parent[n] = -1;
+                if (n == 1) o.parent[0] = -1;
+            }
             break;
         }
+        const bool left = dR > dL;
+        const int s = left ? hi : lo - 1;
+        s_fid[lo] = id;  // on the frontier unless it is merged below
+        if (s < 0 || s >= cnt - 1) break;
         if (level >= MAX_CLIMB) {
-            atomicOr(err, ASTER_DEVERR_TREE);
+            atomicOr(o.err, ASTER_DEVERR_TREE);
             break;
         }
-        const int pslot = (int)(ip - B0);
-        __threadfence_block();  // own node data (shared) before the arrival count
-        if (atomicAdd(&s_cnt[pslot], 1u) == 0u) break;
-        __threadfence_block();
-        const int32_t sb = s_sib[side][slot];
-        const int32_t so = sb >= 0 ? sb : ~sb;
-        const int oside = so >= n ? 1 : 0;
-        const int oslot = (int)(oside ? (int64_t)so - n - B0 : (int64_t)so - B0);
-        const double4 oc = s_cm[oside][oslot];
-        const float4 ol = s_lo[oside][oslot], oh = s_hi[oside][oslot];
-        const bool right = sb < 0;  // cur is the right child
+        const int old = meet(&s_slot[s], 1 + (left ? lo : hi) + TREE_LEAVES * loc);
+        if (old == 0) break;  // the sibling merges
+        const int e = (old - 1) % TREE_LEAVES, sl = (old - 1) / TREE_LEAVES;
+        const int sw = sl / TREE_LEAVES, si = sl % TREE_LEAVES;
+        const double4 oc = s_cm[sw][si];
+        const float4 ol = s_lo[sw][si], oh = s_hi[sw][si];
         double4 pc;
         float4 plo, phi;
-        bu_merge(right ? oc : cm, right ? cm : oc, right ? ol : lo, right ? lo : ol, right ? oh : hi, right ? hi : oh,
-                 pc, plo, phi);
-        s_cm[1][pslot] = pc;
-        s_lo[1][pslot] = plo;
-        s_hi[1][pslot] = phi;
+        bu_merge(left ? cm : oc, left ? oc : cm, left ? blo : ol, left ? ol : blo, left ? bhi : oh, left ? oh : bhi, pc,
+                 plo, phi);
+        s_fid[s + 1] = -1;
+        s_kids[s] = left ? loc + 256 * sl : sl + 256 * loc;
+        if (left) hi = e;
+        else lo = e;
+        loc = TREE_LEAVES + s;
         cm = pc;
-        lo = plo;
-        hi = phi;
-        side = 1;
-        slot = pslot;
-        cur = par;
-    }
-    __syncthreads();  // one global reservation per block for its frontier nodes
-    if (j == 0) s_fbase = s_nf ? atomicAdd(nfront, s_nf) : 0u;
-    // the block's completed internal nodes (both children arrived) go to global
-    // memory in one coalesced pass, not from inside the climb, so that the
-    // block-scope fences there wait for shared-memory stores only; with them
-    // their child records, from the children's data still in shared memory
-    // (a completed node's children lie in the block: leaves B0..B1, internal
-    // nodes n + B0..B1)
-    if (k < n - 1 && s_cnt[j] == 2u) {
-        node_cm[n + k] = s_cm[1][j];
-        bmin[n + k] = s_lo[1][j];
-        bmax[n + k] = s_hi[1][j];
-        const int2 ch = child[n + k];
-        const int sL = (int)(ch.x < n ? ch.x - B0 : ch.x - n - B0), sR = (int)(ch.y < n ? ch.y - B0 : ch.y - n - B0);
-        const int tL = ch.x < n ? 0 : 1, tR = ch.y < n ? 0 : 1;
-        put_child_record(crec + 4 * k, n, theta, ch.x, s_cm[tL][sL], s_lo[tL][sL], s_hi[tL][sL], ch.y, s_cm[tR][sR],
-                         s_lo[tR][sR], s_hi[tR][sR]);
+        blo = plo;
+        bhi = phi;
+        s_cm[1][s] = cm;
+        s_lo[1][s] = blo;
+        s_hi[1][s] = bhi;
+        s_rng[s] = lo + 256 * hi;
+        const int nL = s_dl[lo], nR = s_dl[hi + 1];
+        id = (int32_t)(n + (nL < 0 && nR < 0 ? 0 : B0 + (nR > nL ? hi : lo)));
+        s_id[s] = id;
     }
     __syncthreads();
-    if ((unsigned)j < s_nf) front[s_fbase + j] = s_front[j];
+    const unsigned fm = __ballot_sync(0xffffffffu, s_fid[j] >= 0);
+    if ((j & 31) == 0) s_warp[j >> 5] = __popc(fm);
+    if (s_id[j] >= 0) {
+        const int32_t v = s_id[j];
+        const int kL = s_kids[j] & 255, kR = s_kids[j] >> 8;
+        const int tL = kL / TREE_LEAVES, iL = kL % TREE_LEAVES, tR = kR / TREE_LEAVES, iR = kR % TREE_LEAVES;
+        const int32_t L = tL ? s_id[iL] : (int32_t)(B0 + iL), R = tR ? s_id[iR] : (int32_t)(B0 + iR);
+        o.node_cm[v] = s_cm[1][j];
+        o.bmin[v] = s_lo[1][j];
+        o.bmax[v] = s_hi[1][j];
+        o.child[v] = make_int2(L, R);
+        put_links<LINKS>(o, v, L, R, B0 + (s_rng[j] & 255), B0 + (s_rng[j] >> 8));
+        put_child_record(o.crec + 4 * (v - n), n, theta, L, s_cm[tL][iL], s_lo[tL][iL], s_hi[tL][iL], R, s_cm[tR][iR],
+                         s_lo[tR][iR], s_hi[tR][iR]);
+    }
+    __syncthreads();
+    if (s_fid[j] >= 0) {
+        const int r = (j >= 32 ? s_warp[0] : 0) + __popc(fm & ((1u << (j & 31)) - 1u));
+        front[B0 + r] = make_int2(s_fid[j], (int32_t)(B0 + j));
+    }
+    if (j == 0) nfront[blockIdx.x] = s_warp[0] + s_warp[1];
 }
 
-// Arrival at a node in the global phase: one atomic with acquire-release
-// semantics at GPU scope. Its release half publishes this climb's node data
-// (written before it) to the climb that arrives second; its acquire half
-// makes the sibling's data, published by the first arrival's release, visible
-// to the loads that follow. (ASTER_BU_FENCES=1: the equivalent form with a
-// full fence on either side of a relaxed atomicAdd.)
-#ifndef ASTER_BU_FENCES
-#define ASTER_BU_FENCES 0
-#endif
-__device__ __forceinline__ unsigned int bu_arrive(unsigned int* counter) {
-#if ASTER_BU_FENCES
-    __threadfence();
-    const unsigned int old = atomicAdd(counter, 1u);
-    __threadfence();
-    return old;
-#else
-    unsigned int old;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
-    return old;
-#endif
-}
+// One block's share of a merge: `T` items (node, first leaf) in leaf order that
+// tile the leaves [base, end).
+struct MergeItems {
+    int64_t n, end;
+    int T;
+    const signed char* dl;
+};
 
-__global__ void __launch_bounds__(256) k_bottom_up_front(int64_t n, const int32_t* __restrict__ front,
-                                                         const unsigned int* __restrict__ nfront,
-                                                         const int32_t* __restrict__ parent,
-                                                         const int32_t* __restrict__ sib,
-                                                         uint32_t* __restrict__ counters, double4* __restrict__ node_cm,
-                                                         float4* __restrict__ bmin, float4* __restrict__ bmax,
-                                                         int* __restrict__ err) {
-    const int64_t nf = *nfront;
-    for (int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; f < nf; f += (int64_t)gridDim.x * blockDim.x) {
-        int32_t cur = front[f];
-        // the climb's own node data stays in registers; only the sibling's is loaded
-        double4 cm = ld_cg(node_cm + cur);
-        float4 lo = cur < n ? leaf_lo(cm) : ld_cg(bmin + cur), hi = cur < n ? leaf_hi(cm) : ld_cg(bmax + cur);
-        int32_t par = parent[cur], sb = sib[cur];
-        for (int level = 0; par >= 0; ++level) {
+// The climb of a merge whose items exceed the shared memory (`cap`): the same
+// with node data, and the climb state per leaf of the region, in global memory.
+struct MergeSpill {
+    unsigned long long* slot;
+    int32_t *lo, *done, *fid;
+};
+template <bool LINKS>
+__device__ __noinline__ void merge_spilled(const MergeItems m, double theta, const TreeOut o, unsigned long long* slot,
+                                           int32_t* ilo, int32_t* done, int32_t* fid) {
+    const int64_t n = m.n;
+    const int T = m.T;
+    auto first = [&](int r) -> int64_t { return r < T ? (int64_t)ilo[r] : m.end; };
+    auto delta = [&](int r) -> int {  // across the boundary before item r
+        const int64_t l = first(r);
+        return l == 0 ? -1 : (int)m.dl[l - 1];
+    };
+    for (int r = threadIdx.x; r < T; r += MERGE_THREADS) {
+        int a = r, b = r;
+        int32_t id = fid[r];
+        double4 cm = o.node_cm[id];
+        float4 lo = id < n ? leaf_lo(cm) : o.bmin[id], hi = id < n ? leaf_hi(cm) : o.bmax[id];
+        int dL = delta(r), dR = delta(r + 1);
+        for (int level = 0;; ++level) {
+            if (dL < 0 && dR < 0) break;  // the root
+            const bool left = dR > dL;
+            const int s = left ? b : a - 1;
+            fid[a] = id;
+            if (s < 0 || s >= T - 1) break;
             if (level >= MAX_CLIMB) {
-                atomicOr(err, ASTER_DEVERR_TREE);
+                atomicOr(o.err, ASTER_DEVERR_TREE);
                 break;
             }
-            // the next level's links load while this level synchronises
-            const int32_t par_next = parent[par], sb_next = sib[par];
-            if (bu_arrive(&counters[par - n]) == 0u) break;  // first arrival: the sibling finishes it
-            const int32_t so = sb >= 0 ? sb : ~sb;
-            const double4 oc = ld_cg(node_cm + so);
-            const float4 ol = so < n ? leaf_lo(oc) : ld_cg(bmin + so), oh = so < n ? leaf_hi(oc) : ld_cg(bmax + so);
-            const bool right = sb < 0;  // cur is the right child
+            __threadfence_block();
+            const unsigned long long mine =
+                ((unsigned long long)(unsigned)((left ? a : b) + 1) << 32) | (unsigned long long)(unsigned)id;
+            const unsigned long long old = atomicExch(&slot[s], mine);
+            if (old == 0ull) break;
+            __threadfence_block();
+            const int e = (int)(old >> 32) - 1;
+            const int32_t so = (int32_t)(unsigned)old;
+            const double4 oc = o.node_cm[so];
+            const float4 ol = so < n ? leaf_lo(oc) : o.bmin[so], oh = so < n ? leaf_hi(oc) : o.bmax[so];
+            if (left) b = e;
+            else a = e;
+            dL = delta(a);
+            dR = delta(b + 1);
             double4 pc;
             float4 plo, phi;
-            bu_merge(right ? oc : cm, right ? cm : oc, right ? ol : lo, right ? lo : ol, right ? oh : hi,
-                     right ? hi : oh, pc, plo, phi);
-            node_cm[par] = pc;
-            bmin[par] = plo;
-            bmax[par] = phi;
+            bu_merge(left ? cm : oc, left ? oc : cm, left ? lo : ol, left ? ol : lo, left ? hi : oh, left ? oh : hi, pc,
+                     plo, phi);
+            const int64_t l0 = first(a), l1 = first(s + 1), l2 = first(b + 1);  // children [l0, l1), [l1, l2)
+            const int32_t L = left ? id : so, R = left ? so : id;
+            id = (int32_t)(n + (dL < 0 && dR < 0 ? 0 : dR > dL ? l2 - 1 : l0));
+            fid[s + 1] = -1;
+            done[s] = id;
             cm = pc;
             lo = plo;
             hi = phi;
-            cur = par;
-            par = par_next;
-            sb = sb_next;
+            o.node_cm[id] = cm;
+            o.bmin[id] = lo;
+            o.bmax[id] = hi;
+            o.child[id] = make_int2(L, R);
+            put_links<LINKS>(o, id, L, R, l0, l2 - 1);
+            list_children(o, n, l0, l1, l2);
         }
     }
+    __syncthreads();
+    // the records of the nodes merged here, off the climbs' serial path
+    for (int s = threadIdx.x; s < T - 1; s += MERGE_THREADS) {
+        const int32_t v = done[s];
+        if (v < 0) continue;
+        const int2 ch = o.child[v];
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        put_child_record(o.crec + 4 * (v - n), n, theta, ch.x, o.node_cm[ch.x], ch.x < n ? z : o.bmin[ch.x],
+                         ch.x < n ? z : o.bmax[ch.x], ch.y, o.node_cm[ch.y], ch.y < n ? z : o.bmin[ch.y],
+                         ch.y < n ? z : o.bmax[ch.y]);
+    }
+}
+
+// Shared memory of a merge of up to `cap` items: per location (item r, or cap +
+// the node whose children meet between items s and s + 1) the node's data and
+// number; per item its first leaf and the climb state.
+__host__ __device__ inline size_t merge_smem_bytes(int cap) {
+    return (size_t)cap * (2 * (sizeof(double4) + 2 * sizeof(float4) + sizeof(int32_t)) + 5 * sizeof(int32_t) + 1) + 16;
+}
+
+template <bool LINKS>
+__global__ void __launch_bounds__(MERGE_THREADS, 1) k_tree_merge(int64_t n, double theta, int64_t region, int64_t sub,
+                                                                 int cap, const signed char* __restrict__ dl, TreeOut o,
+                                                                 const int2* __restrict__ front_in,
+                                                                 const int32_t* __restrict__ nfront_in,
+                                                                 int2* __restrict__ front_out,
+                                                                 int32_t* __restrict__ nfront_out, MergeSpill spill) {
+    extern __shared__ double4 merge_smem[];
+    __shared__ int s_off[MERGE_FAN_MAX];
+    __shared__ uint32_t s32[32];
+    const int64_t base = (int64_t)blockIdx.x * region, end = base + region < n ? base + region : n;
+    const int nin = (int)((end - base + sub - 1) / sub);
+    const int32_t* nf = nfront_in + base / sub;
+    uint32_t total;
+    const uint32_t off = block_exclusive_scan((int)threadIdx.x < nin ? (uint32_t)nf[threadIdx.x] : 0u, s32, &total);
+    if ((int)threadIdx.x < nin) s_off[threadIdx.x] = (int)off;
+    const int T = (int)total;
+    const bool fits = T <= cap;
+    double4* s_cm = merge_smem;
+    float4* s_lo = reinterpret_cast<float4*>(s_cm + 2 * cap);
+    float4* s_hi = s_lo + 2 * cap;
+    int32_t* s_id = reinterpret_cast<int32_t*>(s_hi + 2 * cap);
+    int32_t* s_kids = s_id + 2 * cap;
+    int32_t* s_rng = s_kids + cap;
+    int32_t* s_slot = s_rng + cap;
+    int32_t* ilo = fits ? s_slot + cap : spill.lo + base;
+    int32_t* fid = fits ? s_slot + 2 * cap : spill.fid + base;
+    signed char* s_dl = reinterpret_cast<signed char*>(s_slot + 3 * cap);  // [r]: delta before item r
+    __syncthreads();
+    for (int q = threadIdx.x >> 5; q < nin; q += MERGE_THREADS / 32) {
+        const int2* f = front_in + base + q * sub;
+        const int c = (q + 1 < nin ? s_off[q + 1] : T) - s_off[q];
+        for (int i = threadIdx.x & 31; i < c; i += 32) {
+            const int2 it = f[i];
+            const int r = s_off[q] + i;
+            ilo[r] = it.y;
+            fid[r] = fits ? -1 : it.x;
+            if (fits) {
+                const double4 cm = o.node_cm[it.x];
+                s_cm[r] = cm;
+                s_lo[r] = it.x < n ? leaf_lo(cm) : o.bmin[it.x];
+                s_hi[r] = it.x < n ? leaf_hi(cm) : o.bmax[it.x];
+                s_dl[r] = it.y == 0 ? (signed char)-1 : dl[it.y - 1];
+                s_id[r] = it.x;
+                s_id[cap + r] = -1;
+                s_slot[r] = 0;
+            } else {
+                spill.slot[base + r] = 0ull;
+                spill.done[base + r] = -1;
+            }
+        }
+    }
+    if (fits && threadIdx.x == 0) s_dl[T] = dl[end - 1];
+    __syncthreads();
+    if (!fits) {
+        merge_spilled<LINKS>(MergeItems{n, end, T, dl}, theta, o, spill.slot + base, ilo, spill.done + base, fid);
+    } else {
+        for (int r = threadIdx.x; r < T; r += MERGE_THREADS) {
+            int a = r, b = r, loc = r;
+            int32_t id = s_id[r];
+            double4 cm = s_cm[r];
+            float4 lo = s_lo[r], hi = s_hi[r];
+            int dL = s_dl[r], dR = s_dl[r + 1];
+            for (int level = 0;; ++level) {
+                if (dL < 0 && dR < 0) break;  // the root
+                const bool left = dR > dL;
+                const int s = left ? b : a - 1;
+                fid[a] = id;  // on the frontier unless it is merged below
+                if (s < 0 || s >= T - 1) break;
+                if (level >= MAX_CLIMB) {
+                    atomicOr(o.err, ASTER_DEVERR_TREE);
+                    break;
+                }
+                const int old = meet(&s_slot[s], 1 + (left ? a : b) + (loc << 12));
+                if (old == 0) break;  // the sibling merges
+                const int e = (old - 1) & 4095, sl = (old - 1) >> 12;
+                const double4 oc = s_cm[sl];
+                const float4 ol = s_lo[sl], oh = s_hi[sl];
+                if (left) b = e;
+                else a = e;
+                dL = s_dl[a];
+                dR = s_dl[b + 1];
+                double4 pc;
+                float4 plo, phi;
+                bu_merge(left ? cm : oc, left ? oc : cm, left ? lo : ol, left ? ol : lo, left ? hi : oh, left ? oh : hi,
+                         pc, plo, phi);
+                fid[s + 1] = -1;
+                s_kids[s] = left ? loc | sl << 16 : sl | loc << 16;
+                s_rng[s] = a | b << 16;
+                id = (int32_t)(n + (dL < 0 && dR < 0 ? 0 : dR > dL ? (b + 1 < T ? (int64_t)ilo[b + 1] : end) - 1 : ilo[a]));
+                loc = cap + s;
+                cm = pc;
+                lo = plo;
+                hi = phi;
+                s_id[loc] = id;
+                s_cm[loc] = cm;
+                s_lo[loc] = lo;
+                s_hi[loc] = hi;
+            }
+        }
+        __syncthreads();
+        // the merged nodes to global memory, their records, groups and links
+        for (int s = threadIdx.x; s < T - 1; s += MERGE_THREADS) {
+            const int32_t v = s_id[cap + s];
+            if (v < 0) continue;
+            const int kL = s_kids[s] & 0xffff, kR = s_kids[s] >> 16, a = s_rng[s] & 0xffff, b = s_rng[s] >> 16;
+            const int32_t L = s_id[kL], R = s_id[kR];
+            const int64_t l0 = ilo[a], l1 = ilo[s + 1], l2 = b + 1 < T ? (int64_t)ilo[b + 1] : end;
+            o.node_cm[v] = s_cm[cap + s];
+            o.bmin[v] = s_lo[cap + s];
+            o.bmax[v] = s_hi[cap + s];
+            o.child[v] = make_int2(L, R);
+            put_links<LINKS>(o, v, L, R, l0, l2 - 1);
+            list_children(o, n, l0, l1, l2);
+            put_child_record(o.crec + 4 * (v - n), n, theta, L, s_cm[kL], s_lo[kL], s_hi[kL], R, s_cm[kR], s_lo[kR],
+                             s_hi[kR]);
+        }
+    }
+    if (gridDim.x == 1) {  // the root is done
+        if (LINKS && threadIdx.x == 0) o.parent[n] = -1;
+        return;
+    }
+    uint32_t at = 0;
+    for (int r0 = 0; r0 < T; r0 += MERGE_THREADS) {
+        const int r = r0 + (int)threadIdx.x;
+        const bool f = r < T && fid[r] >= 0;
+        uint32_t sum;
+        const uint32_t p = block_exclusive_scan(f ? 1u : 0u, s32, &sum);
+        if (f) front_out[base + at + p] = make_int2(fid[r], ilo[r]);
+        at += sum;
+    }
+    if (threadIdx.x == 0) nfront_out[blockIdx.x] = (int32_t)at;
+}
+
+// Arrival at a node of the node-velocity climb: one atomic with
+// acquire-release semantics at GPU scope. Its release half publishes this
+// climb's node data (written before it) to the climb that arrives second; its
+// acquire half makes the sibling's data, published by the first arrival's
+// release, visible to the loads that follow.
+__device__ __forceinline__ unsigned int bu_arrive(unsigned int* counter) {
+    unsigned int old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
+    return old;
+}
+__device__ __forceinline__ double4 ld_cg(const double4* p) {
+    const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
+    const double2 b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
+    return make_double4(a.x, a.y, b.x, b.y);
 }
 
 // Node velocities for the post-Newtonian walk, in NodesArray::unite form
@@ -733,54 +936,6 @@ __global__ void __launch_bounds__(256) k_node_vel(int64_t n, const int32_t* __re
             par = parent[cur];
             sb = sib[cur];
         }
-    }
-}
-
-// Child records of the internal nodes completed by the global phase of the
-// bottom-up merge (their arrival counters read 2; the block-local phase writes
-// the records of the nodes it completes and leaves their counters at 0).
-// Those nodes are sparse (~10% of the internal nodes at N = 2^20), so each block
-// first compacts the ones in its span of REC_SPAN counters into shared memory
-// and then gives them to consecutive threads: the latency-bound loads of the
-// children's data run in full warps instead of one lane per warp.
-constexpr int REC_SPAN = 2048;
-__global__ void __launch_bounds__(256) k_front_records(int64_t n, double theta, const uint32_t* __restrict__ counters,
-                                                       const int2* __restrict__ child,
-                                                       const double4* __restrict__ node_cm,
-                                                       const float4* __restrict__ bmin,
-                                                       const float4* __restrict__ bmax, float4* __restrict__ crec) {
-    __shared__ int32_t s_list[REC_SPAN];
-    __shared__ unsigned int s_n;
-    const int lane = threadIdx.x & 31;
-    const int64_t m = n - 1;  // internal nodes 0 .. n - 2
-    for (int64_t base = (int64_t)blockIdx.x * REC_SPAN; base < m; base += (int64_t)gridDim.x * REC_SPAN) {
-        if (threadIdx.x == 0) s_n = 0u;
-        __syncthreads();
-        bool hit[REC_SPAN / 256];
-#pragma unroll
-        for (int r = 0; r < REC_SPAN / 256; ++r) {
-            const int64_t i = base + r * 256 + threadIdx.x;
-            hit[r] = i < m && counters[i] == 2u;
-        }
-#pragma unroll
-        for (int r = 0; r < REC_SPAN / 256; ++r) {
-            const uint32_t mask = __ballot_sync(0xffffffffu, hit[r]);
-            unsigned int wb = 0u;
-            if (lane == 0 && mask) wb = atomicAdd(&s_n, (unsigned int)__popc(mask));
-            wb = __shfl_sync(0xffffffffu, wb, 0);
-            if (hit[r]) s_list[wb + __popc(mask & ((1u << lane) - 1u))] = r * 256 + (int)threadIdx.x;
-        }
-        __syncthreads();
-        const unsigned int cnt = s_n;
-        for (unsigned int k = threadIdx.x; k < cnt; k += blockDim.x) {
-            const int64_t i = base + s_list[k];
-            const int2 ch = child[n + i];
-            const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-            put_child_record(crec + 4 * i, n, theta, ch.x, node_cm[ch.x], ch.x < n ? z : bmin[ch.x],
-                             ch.x < n ? z : bmax[ch.x], ch.y, node_cm[ch.y], ch.y < n ? z : bmin[ch.y],
-                             ch.y < n ? z : bmax[ch.y]);
-        }
-        __syncthreads();  // s_n and s_list are reused by the next span
     }
 }
 
@@ -1823,27 +1978,49 @@ int run_sort(aster_ctx* c, int bits) {
     return ASTER_OK;
 }
 
-int launch_bottom_up(aster_ctx* c, int64_t n, double theta) {
+template <class KeyT, bool COMPAT, bool LINKS>
+int run_tree(aster_ctx* c, const aster_params* p) {
     LbvhBufs& t = c->tree;
-    unsigned int* nfront = red_groups(c) + 2;  // zeroed at the start of the build
-    const int64_t blocks = (n + BU_LEAVES - 1) / BU_LEAVES;
-    k_bottom_up_local<<<(unsigned)blocks, BU_LEAVES, 0, c->stream>>>(
-        n, t.parent.as<int32_t>(), t.sib.as<int32_t>(), t.rlo.as<int32_t>(), t.rhi.as<int32_t>(),
-        t.node_cm.as<double4>(), t.bmin.as<float4>(), t.bmax.as<float4>(), t.front.as<int32_t>(), nfront, c->err_dev,
-        theta, t.child.as<int2>(), t.crec.as<float4>());
+    const int64_t n = c->n;
+    int64_t nb = (n + TREE_LEAVES - 1) / TREE_LEAVES, sub = TREE_LEAVES;
+    const TreeOut o{t.node_cm.as<double4>(), t.bmin.as<float4>(), t.bmax.as<float4>(), t.child.as<int2>(),
+                    t.crec.as<float4>(), LINKS ? t.parent.as<int32_t>() : nullptr, LINKS ? t.sib.as<int32_t>() : nullptr,
+                    LINKS ? t.rlo.as<int32_t>() : nullptr, LINKS ? t.rhi.as<int32_t>() : nullptr,
+                    t.groups.as<int2>(), red_groups(c), c->err_dev};
+    // frontiers alternate between two arrays; the sort's alternate keys, histogram and the leaves' unused boxes are free
+    int2* fr[2] = {t.front.as<int2>(), t.codes_alt.as<int2>()};
+    int32_t* nfr[2] = {t.hist.as<int32_t>(), t.hist.as<int32_t>() + nb};
+    const MergeSpill spill{t.bmax.as<unsigned long long>(), t.perm_alt.as<int32_t>(), t.counters.as<int32_t>(),
+                           t.bmin.as<int32_t>()};
+    signed char* dl = t.dl.as<signed char>();
+    k_tree_local<KeyT, COMPAT, LINKS><<<(unsigned)nb, TREE_LEAVES, 0, c->stream>>>(
+        n, p->theta, t.sorted_codes.as<KeyT>(), t.perm.as<int32_t>(), c->pm.as<double4>(), o, dl, fr[0], nfr[0]);
     ASTER_CUDA(cudaGetLastError());
-    const int64_t fb = std::min<int64_t>(blocks, (int64_t)c->sm_count * 8);
-    k_bottom_up_front<<<(unsigned)fb, 256, 0, c->stream>>>(n, t.front.as<int32_t>(), nfront, t.parent.as<int32_t>(),
-                                                           t.sib.as<int32_t>(), t.counters.as<uint32_t>(),
-                                                           t.node_cm.as<double4>(), t.bmin.as<float4>(),
-                                                           t.bmax.as<float4>(), c->err_dev);
-    ASTER_CUDA(cudaGetLastError());
-    c->stats.kernels += 2;
+    c->stats.kernels += 1;
+    ASTER_CUDA(cudaFuncSetAttribute(k_tree_merge<LINKS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)merge_smem_bytes(MERGE_CAP_LAST)));
+    for (int cur = 0; nb > 1; cur ^= 1) {
+        // a block of R leaves leaves about log2(R) + 0.3 subtrees over (Plummer, 2^20 bodies: 6.3 of 64 leaves, 8.3 of
+        // 256): one block takes the rest when its items fit, else each takes as many as fit
+        const double items = 1.2 * (std::log2((double)sub) + 0.3);
+        const bool last = nb <= MERGE_FAN_MAX && (double)nb * items <= MERGE_CAP_LAST;
+        int64_t fan = nb;
+        if (!last)
+            for (fan = 4; fan < 64 && 2 * fan * items <= MERGE_CAP;) fan *= 2;
+        const int cap = last && (double)nb * items > MERGE_CAP ? MERGE_CAP_LAST : MERGE_CAP;
+        const int64_t region = sub * fan, out = (n + region - 1) / region;
+        k_tree_merge<LINKS><<<(unsigned)out, MERGE_THREADS, merge_smem_bytes(cap), c->stream>>>(
+            n, p->theta, region, sub, cap, dl, o, fr[cur], nfr[cur], fr[cur ^ 1], nfr[cur ^ 1], spill);
+        ASTER_CUDA(cudaGetLastError());
+        c->stats.kernels += 1;
+        sub = region;
+        nb = out;
+    }
     return ASTER_OK;
 }
 
 template <class KeyT>
-int run_build(aster_ctx* c, const aster_params* p) {
+int run_build(aster_ctx* c, const aster_params* p, bool links) {
     LbvhBufs& t = c->tree;
     const int64_t n = c->n;
     const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)c->sm_count * 16);
@@ -1869,30 +2046,11 @@ int run_build(aster_ctx* c, const aster_params* p) {
                                            // [3] small groups
     ASTER_CUDA(cudaMemsetAsync(gcount, 0, 4 * sizeof(unsigned int), c->stream));
     ASTER_TRY(aster_apply_pending_mass(c));  // the leaf gather below is the first reader of the masses
-    const KeyT* sc = t.sorted_codes.as<KeyT>();
-    if (p->compat_mode)
-        k_karras<KeyT, true><<<grid, 256, 0, c->stream>>>(
-            n, sc, t.perm.as<int32_t>(), c->pm.as<double4>(), t.parent.as<int32_t>(), t.sib.as<int32_t>(),
-            t.rlo.as<int32_t>(), t.rhi.as<int32_t>(), t.child.as<int2>(), t.counters.as<uint32_t>(),
-            t.node_cm.as<double4>(), t.groups.as<int2>(), gcount);
-    else
-        k_karras<KeyT, false><<<grid, 256, 0, c->stream>>>(
-            n, sc, t.perm.as<int32_t>(), c->pm.as<double4>(), t.parent.as<int32_t>(), t.sib.as<int32_t>(),
-            t.rlo.as<int32_t>(), t.rhi.as<int32_t>(), t.child.as<int2>(), t.counters.as<uint32_t>(),
-            t.node_cm.as<double4>(), t.groups.as<int2>(), gcount);
-    ASTER_CUDA(cudaGetLastError());
-    ASTER_TRY(launch_bottom_up(c, n, p->theta));
-    const int64_t spans = (n - 2 + REC_SPAN) / REC_SPAN;  // ceil((n - 1) / REC_SPAN); 0 for n == 1
-    const int rgrid = (int)std::max<int64_t>(1, std::min<int64_t>(spans, (int64_t)c->sm_count * 8));
-    k_front_records<<<rgrid, 256, 0, c->stream>>>(n, p->theta, t.counters.as<uint32_t>(), t.child.as<int2>(),
-                                                 t.node_cm.as<double4>(), t.bmin.as<float4>(), t.bmax.as<float4>(),
-                                                 t.crec.as<float4>());
-    ASTER_CUDA(cudaGetLastError());
-    c->stats.kernels += 2;
-    return ASTER_OK;
+    if (p->compat_mode) return links ? run_tree<KeyT, true, true>(c, p) : run_tree<KeyT, true, false>(c, p);
+    return links ? run_tree<KeyT, false, true>(c, p) : run_tree<KeyT, false, false>(c, p);
 }
 
-int ensure_tree(aster_ctx* c) {
+int ensure_tree(aster_ctx* c, bool links) {
     LbvhBufs& t = c->tree;
     const int64_t n = c->n, m = 2 * n;  // 2n-1 nodes, +1 slot so parent[n] exists for n == 1
     const int64_t nblocks = (n + SORT_TILE - 1) / SORT_TILE;
@@ -1903,11 +2061,14 @@ int ensure_tree(aster_ctx* c) {
     ASTER_TRY(t.perm_alt.ensure((size_t)n * 4));
     ASTER_TRY(t.hist.ensure((size_t)nblocks * RADIX * 4));
     ASTER_TRY(t.digit_off.ensure((size_t)RADIX * 4));
-    ASTER_TRY(t.parent.ensure((size_t)m * 4));
-    ASTER_TRY(t.sib.ensure((size_t)m * 4));
-    ASTER_TRY(t.front.ensure((size_t)n * 4));
-    ASTER_TRY(t.rlo.ensure((size_t)m * 4));
-    ASTER_TRY(t.rhi.ensure((size_t)m * 4));
+    if (links) {
+        ASTER_TRY(t.parent.ensure((size_t)m * 4));
+        ASTER_TRY(t.sib.ensure((size_t)m * 4));
+        ASTER_TRY(t.rlo.ensure((size_t)m * 4));
+        ASTER_TRY(t.rhi.ensure((size_t)m * 4));
+    }
+    ASTER_TRY(t.front.ensure((size_t)n * sizeof(int2)));
+    ASTER_TRY(t.dl.ensure((size_t)n));
     ASTER_TRY(t.counters.ensure((size_t)n * 4));
     ASTER_TRY(t.node_cm.ensure((size_t)m * sizeof(double4)));
     ASTER_TRY(t.bmin.ensure((size_t)m * sizeof(float4)));
@@ -1922,8 +2083,9 @@ int ensure_tree(aster_ctx* c) {
 
 }  // namespace
 
-int aster_lbvh_build_dev(aster_ctx* c, const aster_params* p, bool box_ready) {
-    ASTER_TRY(ensure_tree(c));
+int aster_lbvh_build_dev(aster_ctx* c, const aster_params* p, bool box_ready, bool links) {
+    links = links || pn_level(p) > 0;  // the node velocities climb by parent and sibling
+    ASTER_TRY(ensure_tree(c, links));
     if (!box_ready) {
         unsigned long long* box = red_box(c);
         ASTER_CUDA(cudaMemsetAsync(box, 0, sizeof(unsigned long long), c->stream));
@@ -1932,8 +2094,8 @@ int aster_lbvh_build_dev(aster_ctx* c, const aster_params* p, bool box_ready) {
         ASTER_CUDA(cudaGetLastError());
         c->stats.kernels += 1;
     }
-    if (p->morton_bits == 63) ASTER_TRY(run_build<uint64_t>(c, p));
-    else ASTER_TRY(run_build<uint32_t>(c, p));
+    if (p->morton_bits == 63) ASTER_TRY(run_build<uint64_t>(c, p, links));
+    else ASTER_TRY(run_build<uint32_t>(c, p, links));
     c->tree.built = true;
     return ASTER_OK;
 }
@@ -2079,7 +2241,7 @@ extern "C" int aster_lbvh_build(aster_ctx* c, const aster_params* p, aster_tree_
     ASTER_TRY(aster_begin(c));
     c->stats = aster_stats{};
     cudaEventRecord(c->ev[0], c->stream);
-    ASTER_TRY(aster_lbvh_build_dev(c, p, false));
+    ASTER_TRY(aster_lbvh_build_dev(c, p, false, view != nullptr));
     cudaEventRecord(c->ev[1], c->stream);
     ASTER_TRY(aster_finish(c));
     float ms = 0.f;
@@ -2102,7 +2264,7 @@ extern "C" int aster_lbvh_forces(aster_ctx* c, const aster_params* p, int precis
         ASTER_TRY(c->targets.ensure((size_t)c->n * 4));
         cnt = c->targets.as<int32_t>();
     }
-    ASTER_TRY(ensure_tree(c));
+    ASTER_TRY(ensure_tree(c, pn_level(p) > 0));
     unsigned long long* inter = red_inter(c);
     ASTER_CUDA(cudaMemsetAsync(inter, 0, 8, c->stream));
     cudaEventRecord(c->ev[0], c->stream);
