@@ -161,8 +161,7 @@ struct aster_ctx {
 inline unsigned long long* red_box(aster_ctx* c) { return c->red.as<unsigned long long>(); }         // byte 0
 inline double* red_energy(aster_ctx* c) { return c->red.as<double>() + 8; }                         // byte 64
 inline unsigned long long* red_inter(aster_ctx* c) { return c->red.as<unsigned long long>() + 64; } // byte 512
-inline unsigned int* red_groups(aster_ctx* c) {  // [0] large-group count, [1] walk work counter, [2] bottom-up
-                                                 // frontier, [3] small-group count
+inline unsigned int* red_groups(aster_ctx* c) {  // [0] large-group count, [1] walk work counter, [3] small-group count
     return reinterpret_cast<unsigned int*>(c->red.as<char>() + 1024);
 }
 
@@ -213,8 +212,11 @@ int64_t aster_energy_parts(const aster_ctx* ctx);
 int aster_kick_drift_coef(aster_ctx* ctx, double kick_dt, double drift_dt, bool kick, bool want_box,
                           bool want_mixed);
 // lbvh.cu
-// links: also parents, siblings and leaf ranges (the exported tree; post-Newtonian laws imply it)
-int aster_lbvh_build_dev(aster_ctx* ctx, const aster_params* p, bool box_ready, bool links = false);
+// links: also parents, siblings and leaf ranges (the exported tree; post-Newtonian laws imply it).
+// zero_box: red_box is zero afterwards, as a walk with fuse_next needs it. The walk's work counter is zero
+// afterwards: one walk per build.
+int aster_lbvh_build_dev(aster_ctx* ctx, const aster_params* p, bool box_ready, bool links = false,
+                         bool zero_box = false);
 // fuse_next (with closing_kick): the walk also applies the next step's
 // opening kick and drift to every body and leaves their bounding box in
 // red_box, so that step's kick-drift launch is left out.

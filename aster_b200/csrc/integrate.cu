@@ -220,7 +220,7 @@ static int force_eval(aster_ctx* c, const aster_params* p, int solver, int preci
         if (tm) pairs[0] = e0, pairs[1] = e0, pairs[2] = tm->mark(c->stream);
         return ASTER_OK;
     }
-    ASTER_TRY(aster_lbvh_build_dev(c, p, box_ready));
+    ASTER_TRY(aster_lbvh_build_dev(c, p, box_ready, false, closing_kick && fuse_next));
     int e1 = tm ? tm->mark(c->stream) : -1;
     ASTER_TRY(aster_lbvh_walk_launch(c, p, precision, closing_kick, nullptr, fuse_next));
     if (tm) pairs[0] = e0, pairs[1] = e1, pairs[2] = tm->mark(c->stream);

@@ -31,6 +31,8 @@
 #include <cstring>
 #include <type_traits>
 
+#include <cooperative_groups.h>
+
 #include "aster_internal.cuh"
 #include "fp64_pair.cuh"
 #include "pn.cuh"
@@ -128,25 +130,30 @@ __device__ __forceinline__ uint32_t quantize_compat(double x, double B) {
 }
 
 template <class KeyT, int MODE>  // MODE 0: 30-bit, 1: 63-bit, 2: 30-bit compat
+__device__ __forceinline__ KeyT morton_code(const double4 p, double B) {
+    if (MODE == 0) {
+        uint32_t ix = quantize(p.x, B, 1024.0, 1023u), iy = quantize(p.y, B, 1024.0, 1023u),
+                 iz = quantize(p.z, B, 1024.0, 1023u);
+        return (KeyT)((part1by2_32(iz) << 2) | (part1by2_32(iy) << 1) | part1by2_32(ix));
+    }
+    if (MODE == 1) {
+        uint64_t ix = quantize(p.x, B, 2097152.0, 2097151u), iy = quantize(p.y, B, 2097152.0, 2097151u),
+                 iz = quantize(p.z, B, 2097152.0, 2097151u);
+        return (KeyT)((part1by2_64(iz) << 2) | (part1by2_64(iy) << 1) | part1by2_64(ix));
+    }
+    uint32_t ix = quantize_compat(p.x, B), iy = quantize_compat(p.y, B), iz = quantize_compat(p.z, B);
+    return (KeyT)(part1by2_32(ix) | (part1by2_32(iy) << 1) | (part1by2_32(iz) << 2));
+}
+
+// (and the build's counters, four from gcount, to zero)
+template <class KeyT, int MODE>
 __global__ void __launch_bounds__(256) k_morton(int64_t n, const double4* __restrict__ pm,
                                                 const unsigned long long* __restrict__ box_bits,
-                                                KeyT* __restrict__ codes) {
+                                                KeyT* __restrict__ codes, unsigned int* __restrict__ gcount) {
+    if (blockIdx.x == 0 && threadIdx.x < 4) gcount[threadIdx.x] = 0u;
     const double B = __longlong_as_double((long long)*box_bits);
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double4 p = pm[i];
-        if (MODE == 0) {
-            uint32_t ix = quantize(p.x, B, 1024.0, 1023u), iy = quantize(p.y, B, 1024.0, 1023u),
-                     iz = quantize(p.z, B, 1024.0, 1023u);
-            codes[i] = (KeyT)((part1by2_32(iz) << 2) | (part1by2_32(iy) << 1) | part1by2_32(ix));
-        } else if (MODE == 1) {
-            uint64_t ix = quantize(p.x, B, 2097152.0, 2097151u), iy = quantize(p.y, B, 2097152.0, 2097151u),
-                     iz = quantize(p.z, B, 2097152.0, 2097151u);
-            codes[i] = (KeyT)((part1by2_64(iz) << 2) | (part1by2_64(iy) << 1) | part1by2_64(ix));
-        } else {
-            uint32_t ix = quantize_compat(p.x, B), iy = quantize_compat(p.y, B), iz = quantize_compat(p.z, B);
-            codes[i] = (KeyT)(part1by2_32(ix) | (part1by2_32(iy) << 1) | (part1by2_32(iz) << 2));
-        }
-    }
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        codes[i] = morton_code<KeyT, MODE>(pm[i], B);
 }
 
 // ---------------------------------------------------------------- sort
@@ -304,6 +311,129 @@ __global__ void __launch_bounds__(SORT_THREADS, 4) k_sort_scatter(int64_t n, con
     }
 }
 
+// Morton codes and their whole stable sort in one launch, for up to 16 blocks'
+// worth of bodies: a cluster of up to 16 blocks keeps the keys on chip (ITEMS
+// per thread) and exchanges them through distributed shared memory, one 8-bit
+// digit a pass. Per pass: warps rank their keys with match-any as k_sort_scatter
+// does, every block publishes its digit counts to the others, and the keys go
+// straight to their new block and place; the last pass writes to global memory.
+// Bound by latency (two cluster barriers a pass). The general sort takes three
+// launches a pass, ~3.3 us each below 10^5 keys, whatever the size.
+constexpr int CSORT_THREADS = 1024, CSORT_WARPS = CSORT_THREADS / 32, CSORT_BLOCKS = 16;
+
+template <class KeyT>
+constexpr size_t cluster_sort_smem(int items) {
+    return (size_t)CSORT_THREADS * items * (sizeof(KeyT) + 4) + (size_t)CSORT_WARPS * RADIX * 2 +
+           (size_t)CSORT_BLOCKS * RADIX * 4 + 2 * RADIX * 4;
+}
+
+template <class KeyT, int MODE, int ITEMS>
+__global__ void __launch_bounds__(CSORT_THREADS, 1) k_sort_cluster(int64_t n, const double4* __restrict__ pm,
+                                                                   const unsigned long long* __restrict__ box_bits,
+                                                                   KeyT* __restrict__ codes, KeyT* __restrict__ kout,
+                                                                   int32_t* __restrict__ vout,
+                                                                   unsigned int* __restrict__ gcount) {
+    namespace cg = cooperative_groups;
+    constexpr int PASSES = sizeof(KeyT) == 8 ? 8 : 4;
+    constexpr int PER_BLOCK = CSORT_THREADS * ITEMS;
+    extern __shared__ __align__(16) unsigned char csort_smem[];
+    KeyT* bkey = reinterpret_cast<KeyT*>(csort_smem);
+    uint32_t* bval = reinterpret_cast<uint32_t*>(bkey + PER_BLOCK);
+    uint32_t* ctot = bval + PER_BLOCK;            // [block][digit] counts of every block
+    uint32_t* stot = ctot + CSORT_BLOCKS * RADIX;  // [digit] this block's counts
+    uint32_t* sbase = stot + RADIX;                // [digit] place of this block's first key
+    uint16_t* wh = reinterpret_cast<uint16_t*>(sbase + RADIX);  // [warp][digit]
+    __shared__ uint32_t s32[32];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), nblk = (int)cluster.num_blocks();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    const int64_t tile0 = (int64_t)rank * PER_BLOCK;
+    if (rank == 0 && threadIdx.x < 4) gcount[threadIdx.x] = 0u;  // the build's counters
+    const int local0 = warp * 32 * ITEMS + lane;
+    const double B = __longlong_as_double((long long)*box_bits);
+    KeyT key[ITEMS];
+    uint32_t val[ITEMS];
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const int64_t i = tile0 + local0 + 32 * r;
+        key[r] = 0;
+        val[r] = (uint32_t)i;
+        if (i < n) {
+            key[r] = morton_code<KeyT, MODE>(pm[i], B);
+            if (codes) codes[i] = key[r];
+        }
+    }
+    cluster.sync();  // every block runs before its shared memory is written from outside
+#pragma unroll 1
+    for (int pass = 0; pass < PASSES; ++pass) {
+        if (pass > 0) {
+#pragma unroll
+            for (int r = 0; r < ITEMS; ++r) {
+                key[r] = bkey[local0 + 32 * r];
+                val[r] = bval[local0 + 32 * r];
+            }
+        }
+        for (int d = threadIdx.x; d < CSORT_WARPS * RADIX / 2; d += CSORT_THREADS) reinterpret_cast<uint32_t*>(wh)[d] = 0u;
+        __syncthreads();
+        uint32_t rk[ITEMS], dig[ITEMS];
+        uint16_t* w = wh + warp * RADIX;
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            const bool ok = tile0 + local0 + 32 * r < n;
+            const uint32_t d = ok ? (uint32_t)(key[r] >> (8 * pass)) & (RADIX - 1) : 0xFFFFu;
+            dig[r] = d;
+            const uint32_t peers = __match_any_sync(0xffffffffu, d);
+            uint32_t before = 0;
+            if (ok) before = w[d];
+            __syncwarp();
+            rk[r] = before + __popc(peers & lt);
+            if (ok && (peers & lt) == 0) w[d] = (uint16_t)(before + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        if (threadIdx.x < RADIX) {  // exclusive prefix of the digit over the warps
+            uint32_t tot = 0;
+#pragma unroll 8
+            for (int q = 0; q < CSORT_WARPS; ++q) {
+                const uint32_t t = wh[q * RADIX + threadIdx.x];
+                wh[q * RADIX + threadIdx.x] = (uint16_t)tot;
+                tot += t;
+            }
+            stot[threadIdx.x] = tot;
+        }
+        __syncthreads();
+        for (int x = threadIdx.x; x < nblk * RADIX; x += CSORT_THREADS)
+            cluster.map_shared_rank(ctot, x / RADIX)[rank * RADIX + x % RADIX] = stot[x % RADIX];
+        cluster.sync();  // every block's counts are here; every block has read its keys
+        uint32_t all = 0, mine = 0;
+        if (threadIdx.x < RADIX) {
+            for (int q = 0; q < nblk; ++q) {
+                const uint32_t t = ctot[q * RADIX + threadIdx.x];
+                all += t;
+                mine += q < rank ? t : 0u;
+            }
+        }
+        const uint32_t start = block_exclusive_scan(all, s32, nullptr);
+        if (threadIdx.x < RADIX) sbase[threadIdx.x] = start + mine;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            if (dig[r] >= RADIX) continue;
+            const uint32_t g = sbase[dig[r]] + w[dig[r]] + rk[r];
+            if (pass == PASSES - 1) {
+                kout[g] = key[r];
+                vout[g] = (int32_t)val[r];
+            } else {
+                const int to = (int)(g / PER_BLOCK), at = (int)(g % PER_BLOCK);
+                cluster.map_shared_rank(bkey, to)[at] = key[r];
+                cluster.map_shared_rank(bval, to)[at] = val[r];
+            }
+        }
+        if (pass < PASSES - 1) cluster.sync();  // the keys have arrived
+    }
+}
+
 template <class KeyT>
 __global__ void k_reverse(int64_t n, const KeyT* __restrict__ kin, const int32_t* __restrict__ vin,
                           KeyT* __restrict__ kout, int32_t* __restrict__ vout) {
@@ -400,10 +530,17 @@ __device__ __forceinline__ void put_child_record(float4* __restrict__ dst, int64
 // 71.6 us, 20,011 115.6 -> 93.7, 131,073 132.5 -> 108.9, 2^20 315 -> 273.
 constexpr int TREE_LEAVES = 64;
 constexpr int MERGE_FAN_MAX = 256;  // input blocks per block at most
-// Items a merge holds in shared memory: 512 leave two blocks per SM, 1344 take
-// one block's 227 KB (the last merge). More items (clustered bodies) go through
-// global memory.
-constexpr int MERGE_CAP = 512, MERGE_CAP_LAST = 1344;
+// Items a merge holds in shared memory: 512 leave two blocks per SM, 256 (the
+// first merge of up to MERGE_MANY input blocks, 32 blocks' worth of items) five.
+// More items (clustered bodies) go through global memory. A merge's time grows
+// with its items (400 items 28 us, 200 some 15), a further launch costs as much
+// as those save: build per step with 512 / 256 in the first merge, us: 10,000
+// bodies 72.8 / 67.0, 20,011 81.2 / 75.0, 262,144 136.0 / 132.2, 524,288 178.1 /
+// 188.5, 2^20 265.7 / 284.0; one last merge of up to 1344 items instead of 512:
+// 10,000 bodies 80.5, 262,144 140.9. 256 threads a merge are slower than 512
+// (20,011 bodies 77.6, 262,144 142.4).
+constexpr int MERGE_CAP0 = 256, MERGE_CAP = 512;
+constexpr int64_t MERGE_MANY = 6000;
 constexpr int MERGE_THREADS = 512;
 
 // delta of the neighbours at sorted positions i, i + 1 (codes a, b, bodies pa, pb)
@@ -536,7 +673,7 @@ template <class KeyT, bool COMPAT, bool LINKS>
 __global__ void __launch_bounds__(TREE_LEAVES, 1024 / TREE_LEAVES) k_tree_local(
     int64_t n, double theta, const KeyT* __restrict__ codes, const int32_t* __restrict__ perm,
     const double4* __restrict__ pm, TreeOut o, signed char* __restrict__ dl, int2* __restrict__ front,
-    int32_t* __restrict__ nfront) {
+    int32_t* __restrict__ nfront, unsigned long long* __restrict__ zero_box) {
     // [0][j]: leaf B0 + j; [1][j]: the node whose children meet between leaves B0 + j and B0 + j + 1
     __shared__ double4 s_cm[2][TREE_LEAVES];
     __shared__ float4 s_lo[2][TREE_LEAVES], s_hi[2][TREE_LEAVES];
@@ -549,6 +686,7 @@ __global__ void __launch_bounds__(TREE_LEAVES, 1024 / TREE_LEAVES) k_tree_local(
     const int64_t B0 = (int64_t)blockIdx.x * TREE_LEAVES, k = B0 + j;
     const int cnt = (int)(n - B0 < TREE_LEAVES ? n - B0 : TREE_LEAVES);
     const bool in = j < cnt;
+    if (zero_box && k == 0) *zero_box = 0ull;  // read by the codes; the walk's fused drift refills it
     s_slot[j] = 0;
     s_id[j] = -1;
     s_fid[j] = -1;
@@ -1978,8 +2116,50 @@ int run_sort(aster_ctx* c, int bits) {
     return ASTER_OK;
 }
 
+// One cluster's launch; false (nothing launched) where the device cannot hold
+// such a cluster.
+template <class KeyT, int MODE, int ITEMS>
+bool launch_sort_cluster(aster_ctx* c, bool want_codes, int* st) {
+    LbvhBufs& t = c->tree;
+    auto kern = k_sort_cluster<KeyT, MODE, ITEMS>;
+    const size_t smem = cluster_sort_smem<KeyT>(ITEMS);
+    const int blocks = (int)((c->n + (int64_t)CSORT_THREADS * ITEMS - 1) / ((int64_t)CSORT_THREADS * ITEMS));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(CSORT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)blocks;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) != cudaSuccess || fit < 1) {
+        cudaGetLastError();
+        return false;
+    }
+    const cudaError_t e =
+        cudaLaunchKernelEx(&cfg, kern, c->n, (const double4*)c->pm.as<double4>(),
+                           (const unsigned long long*)red_box(c), want_codes ? t.codes.as<KeyT>() : (KeyT*)nullptr,
+                           t.sorted_codes.as<KeyT>(), t.perm.as<int32_t>(), red_groups(c));
+    *st = e == cudaSuccess ? ASTER_OK : aster_cuda_fail(e, "k_sort_cluster", __FILE__, __LINE__);
+    c->stats.kernels += 1;
+    return true;
+}
+template <class KeyT, int MODE>
+bool sort_cluster(aster_ctx* c, bool want_codes, int* st) {
+    const int64_t per = (c->n + (int64_t)CSORT_THREADS * CSORT_BLOCKS - 1) / ((int64_t)CSORT_THREADS * CSORT_BLOCKS);
+    if (per <= 1) return launch_sort_cluster<KeyT, MODE, 1>(c, want_codes, st);
+    if (per <= 2) return launch_sort_cluster<KeyT, MODE, 2>(c, want_codes, st);
+    return false;  // four keys a thread: 98 us a build at 40,000 bodies, as the general sort's
+}
+
 template <class KeyT, bool COMPAT, bool LINKS>
-int run_tree(aster_ctx* c, const aster_params* p) {
+int run_tree(aster_ctx* c, const aster_params* p, bool zero_box) {
     LbvhBufs& t = c->tree;
     const int64_t n = c->n;
     int64_t nb = (n + TREE_LEAVES - 1) / TREE_LEAVES, sub = TREE_LEAVES;
@@ -1994,20 +2174,21 @@ int run_tree(aster_ctx* c, const aster_params* p) {
                            t.bmin.as<int32_t>()};
     signed char* dl = t.dl.as<signed char>();
     k_tree_local<KeyT, COMPAT, LINKS><<<(unsigned)nb, TREE_LEAVES, 0, c->stream>>>(
-        n, p->theta, t.sorted_codes.as<KeyT>(), t.perm.as<int32_t>(), c->pm.as<double4>(), o, dl, fr[0], nfr[0]);
+        n, p->theta, t.sorted_codes.as<KeyT>(), t.perm.as<int32_t>(), c->pm.as<double4>(), o, dl, fr[0], nfr[0],
+        zero_box ? red_box(c) : nullptr);
     ASTER_CUDA(cudaGetLastError());
     c->stats.kernels += 1;
     ASTER_CUDA(cudaFuncSetAttribute(k_tree_merge<LINKS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)merge_smem_bytes(MERGE_CAP_LAST)));
+                                    (int)merge_smem_bytes(MERGE_CAP)));
     for (int cur = 0; nb > 1; cur ^= 1) {
         // a block of R leaves leaves about log2(R) + 0.3 subtrees over (Plummer, 2^20 bodies: 6.3 of 64 leaves, 8.3 of
         // 256): one block takes the rest when its items fit, else each takes as many as fit
         const double items = 1.2 * (std::log2((double)sub) + 0.3);
-        const bool last = nb <= MERGE_FAN_MAX && (double)nb * items <= MERGE_CAP_LAST;
+        const bool last = nb <= MERGE_FAN_MAX && (double)nb * items <= MERGE_CAP;
+        const int cap = last || sub > TREE_LEAVES || nb > MERGE_MANY ? MERGE_CAP : MERGE_CAP0;
         int64_t fan = nb;
         if (!last)
-            for (fan = 4; fan < 64 && 2 * fan * items <= MERGE_CAP;) fan *= 2;
-        const int cap = last && (double)nb * items > MERGE_CAP ? MERGE_CAP_LAST : MERGE_CAP;
+            for (fan = 4; 2 * fan * items <= cap && fan < 64;) fan *= 2;
         const int64_t region = sub * fan, out = (n + region - 1) / region;
         k_tree_merge<LINKS><<<(unsigned)out, MERGE_THREADS, merge_smem_bytes(cap), c->stream>>>(
             n, p->theta, region, sub, cap, dl, o, fr[cur], nfr[cur], fr[cur ^ 1], nfr[cur ^ 1], spill);
@@ -2020,18 +2201,29 @@ int run_tree(aster_ctx* c, const aster_params* p) {
 }
 
 template <class KeyT>
-int run_build(aster_ctx* c, const aster_params* p, bool links) {
+int run_build(aster_ctx* c, const aster_params* p, bool links, bool zero_box) {
     LbvhBufs& t = c->tree;
     const int64_t n = c->n;
     const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)c->sm_count * 16);
     const unsigned long long* box = red_box(c);
     const int mode = p->compat_mode ? 2 : (p->morton_bits == 63 ? 1 : 0);
-    if (mode == 0) k_morton<KeyT, 0><<<grid, 256, 0, c->stream>>>(n, c->pm.as<double4>(), box, t.codes.as<KeyT>());
-    else if (mode == 1) k_morton<KeyT, 1><<<grid, 256, 0, c->stream>>>(n, c->pm.as<double4>(), box, t.codes.as<KeyT>());
-    else k_morton<KeyT, 2><<<grid, 256, 0, c->stream>>>(n, c->pm.as<double4>(), box, t.codes.as<KeyT>());
-    ASTER_CUDA(cudaGetLastError());
-    c->stats.kernels += 1;
-    ASTER_TRY(run_sort<KeyT>(c, p->morton_bits == 63 ? 64 : 32));
+    unsigned int* gcount = red_groups(c);  // [0] large groups, [1] walk work counter, [3] small groups: zeroed with
+                                           // the codes
+    int cst = ASTER_OK;
+    bool sorted = false;
+    if constexpr (sizeof(KeyT) == 8) sorted = sort_cluster<KeyT, 1>(c, links, &cst);
+    else sorted = mode == 2 ? sort_cluster<KeyT, 2>(c, links, &cst) : sort_cluster<KeyT, 0>(c, links, &cst);
+    if (cst != ASTER_OK) return cst;
+    if (!sorted) {
+        const double4* pm = c->pm.as<double4>();
+        KeyT* codes = t.codes.as<KeyT>();
+        if constexpr (sizeof(KeyT) == 8) k_morton<KeyT, 1><<<grid, 256, 0, c->stream>>>(n, pm, box, codes, gcount);
+        else if (mode == 2) k_morton<KeyT, 2><<<grid, 256, 0, c->stream>>>(n, pm, box, codes, gcount);
+        else k_morton<KeyT, 0><<<grid, 256, 0, c->stream>>>(n, pm, box, codes, gcount);
+        ASTER_CUDA(cudaGetLastError());
+        c->stats.kernels += 1;
+        ASTER_TRY(run_sort<KeyT>(c, p->morton_bits == 63 ? 64 : 32));
+    }
     if (p->compat_mode) {
         // OpenCL order is descending by (code, index): reverse the ascending sort
         k_reverse<KeyT><<<grid, 256, 0, c->stream>>>(n, t.sorted_codes.as<KeyT>(), t.perm.as<int32_t>(),
@@ -2042,12 +2234,10 @@ int run_build(aster_ctx* c, const aster_params* p, bool links) {
                                    c->stream));
         c->stats.kernels += 1;
     }
-    unsigned int* gcount = red_groups(c);  // [0] large groups, [1] walk work counter, [2] bottom-up frontier,
-                                           // [3] small groups
-    ASTER_CUDA(cudaMemsetAsync(gcount, 0, 4 * sizeof(unsigned int), c->stream));
     ASTER_TRY(aster_apply_pending_mass(c));  // the leaf gather below is the first reader of the masses
-    if (p->compat_mode) return links ? run_tree<KeyT, true, true>(c, p) : run_tree<KeyT, true, false>(c, p);
-    return links ? run_tree<KeyT, false, true>(c, p) : run_tree<KeyT, false, false>(c, p);
+    if (p->compat_mode) return links ? run_tree<KeyT, true, true>(c, p, zero_box)
+                                        : run_tree<KeyT, true, false>(c, p, zero_box);
+    return links ? run_tree<KeyT, false, true>(c, p, zero_box) : run_tree<KeyT, false, false>(c, p, zero_box);
 }
 
 int ensure_tree(aster_ctx* c, bool links) {
@@ -2083,7 +2273,7 @@ int ensure_tree(aster_ctx* c, bool links) {
 
 }  // namespace
 
-int aster_lbvh_build_dev(aster_ctx* c, const aster_params* p, bool box_ready, bool links) {
+int aster_lbvh_build_dev(aster_ctx* c, const aster_params* p, bool box_ready, bool links, bool zero_box) {
     links = links || pn_level(p) > 0;  // the node velocities climb by parent and sibling
     ASTER_TRY(ensure_tree(c, links));
     if (!box_ready) {
@@ -2094,8 +2284,8 @@ int aster_lbvh_build_dev(aster_ctx* c, const aster_params* p, bool box_ready, bo
         ASTER_CUDA(cudaGetLastError());
         c->stats.kernels += 1;
     }
-    if (p->morton_bits == 63) ASTER_TRY(run_build<uint64_t>(c, p, links));
-    else ASTER_TRY(run_build<uint32_t>(c, p, links));
+    if (p->morton_bits == 63) ASTER_TRY(run_build<uint64_t>(c, p, links, zero_box));
+    else ASTER_TRY(run_build<uint32_t>(c, p, links, zero_box));
     c->tree.built = true;
     return ASTER_OK;
 }
@@ -2104,9 +2294,7 @@ int aster_lbvh_walk_launch(aster_ctx* c, const aster_params* p, int precision, b
                            bool fuse_next) {
     if (kick) c->mixed_valid = false;  // the closing kick moves the velocities
     fuse_next = fuse_next && kick;
-    ASTER_CUDA(cudaMemsetAsync(red_groups(c) + 1, 0, sizeof(unsigned int), c->stream));  // work counter
-    // the fused drift's box (the build that just ran has read the previous one)
-    if (fuse_next) ASTER_CUDA(cudaMemsetAsync(red_box(c), 0, sizeof(unsigned long long), c->stream));
+    // the work counter and, with fuse_next, the box are zero: the build that just ran left them so
     const bool guard = !(p->eps2 > 0.0);
     if (precision != ASTER_MIXED && precision != ASTER_FP64) return ASTER_ERR_INVALID_ARG;
     const bool mixed = precision == ASTER_MIXED;
