@@ -322,17 +322,46 @@ __global__ void __launch_bounds__(BLOCK) k_allpairs_mixed2(
                          acc, out3, kick);
 }
 
+// The next step's opening kick and drift, applied where the slices are added
+// (the operations of the kick-drift kernel in its order, so that it need not
+// run); phi, plo, vf: the FP32 copies to refresh (mixed), or null.
+struct NextDrift {
+    double4* pm;  // null: none
+    double dt;
+    float4 *phi, *plo, *vf;
+};
+
 __global__ void k_reduce_slices(int64_t nt, int nslices, const double4* __restrict__ partial,
                                 const int32_t* __restrict__ targets, double G, double4* __restrict__ acc,
-                                double* __restrict__ out3, KickArgs kick) {
+                                double* __restrict__ out3, KickArgs kick, NextDrift next) {
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nt; t += (int64_t)gridDim.x * blockDim.x) {
         double ax = 0, ay = 0, az = 0;
+#pragma unroll 4
         for (int s = 0; s < nslices; ++s) {
             double4 p = partial[(int64_t)s * nt + t];
             ax += p.x; ay += p.y; az += p.z;
         }
         int64_t body = targets ? (int64_t)targets[t] : t;
         store_result(t, body, ax, ay, az, G, 1, 0, nt, nullptr, acc, out3, kick);
+        if (next.pm) {
+            const double4 a = acc[body];
+            double4 p = next.pm[body], v = kick.vel[body];
+            v.x += a.x * kick.half_dt; v.y += a.y * kick.half_dt; v.z += a.z * kick.half_dt;
+            p.x += v.x * next.dt; p.y += v.y * next.dt; p.z += v.z * next.dt;
+            next.pm[body] = p;
+            kick.vel[body] = v;
+            if (next.phi) {
+                float4 h, l;
+                ds_split(p.x, h.x, l.x);
+                ds_split(p.y, h.y, l.y);
+                ds_split(p.z, h.z, l.z);
+                h.w = __double2float_rn(p.w);
+                l.w = 0.f;
+                next.phi[body] = h;
+                next.plo[body] = l;
+                next.vf[body] = make_float4((float)v.x, (float)v.y, (float)v.z, 0.f);
+            }
+        }
     }
 }
 
@@ -374,32 +403,18 @@ void launch_pnl(int precision, bool guard, dim3 grid, cudaStream_t st, int64_t j
 
 }  // namespace
 
-// Launch one all-pairs evaluation. Targets: every body (targets_dev == null,
-// nt == n) or an explicit list. Output: ctx->acc (out_dev == null) with an
-// optional closing kick, or out_dev[nt*3].
-// Launch one all-pairs evaluation over the sources [src_lo, src_hi) (bodies
-// beyond the last massive one are dropped: they attract nothing under any of
-// the force laws). Targets: every body (targets_dev == null, nt == n) or an
-// explicit list. Output: ctx->acc (out_dev == null) with an optional closing
-// kick, or out_dev[nt*3].
-int aster_allpairs_launch_range(aster_ctx* c, const aster_params* p, int precision, bool closing_kick, int64_t nt,
-                                const int32_t* targets_dev, double* out_dev, int64_t src_lo, int64_t src_hi) {
-    if (precision != ASTER_FP64 && precision != ASTER_MIXED) return ASTER_ERR_INVALID_ARG;
-    if (precision == ASTER_MIXED && !c->mixed_valid) ASTER_TRY(aster_refresh_mixed(c));
-    const int64_t n_src = c->n_src > 0 ? c->n_src : c->n;
-    const int64_t lo = src_lo, hi = src_hi < n_src ? src_hi : n_src;
-    const int64_t len = hi > lo ? hi - lo : 0;
-    if (precision == ASTER_FP64 && !targets_dev && !out_dev && lo == 0 && len == nt && nt == c->n &&
-        aster_allpairs_sym_fits(c, p)) {
-        const int st = aster_allpairs_sym_launch(c, p, closing_kick);
-        if (st != ASTER_ERR_OOM) return st;
-    }
+// Source slices of an evaluation of nt targets against len sources.
+struct SliceGrid {
+    int64_t iblocks, ns, slice_len;
+};
+static SliceGrid slice_grid(const aster_ctx* c, const aster_params* p, int precision, int64_t nt, int64_t len) {
+    SliceGrid g;
     // one target per thread in the mixed post-Newtonian kernel, two elsewhere
     const int64_t per_block = (int64_t)BLOCK * (precision == ASTER_MIXED && pn_level(p) > 0 ? IPT_PN : IPT);
-    const int64_t iblocks = (nt + per_block - 1) / per_block;
+    g.iblocks = (nt + per_block - 1) / per_block;
     // j-slices so that small n still fill the GPU (>= ASTER_SLICE_BLOCKS_PER_SM blocks per SM).
     int64_t want = ASTER_SLICE_BLOCKS_PER_SM * (int64_t)c->sm_count;
-    int64_t ns = iblocks >= want ? 1 : (want + iblocks - 1) / iblocks;
+    int64_t ns = g.iblocks >= want ? 1 : (want + g.iblocks - 1) / g.iblocks;
     // each slice at least one j-tile; the mixed kernel's at least
     // ASTER_SLICE_MIN_MIXED sources (its partial-sum reduction outweighs more
     // parallelism below that)
@@ -412,6 +427,32 @@ int aster_allpairs_launch_range(aster_ctx* c, const aster_params* p, int precisi
     if (slice_len < BLOCK) slice_len = BLOCK;
     ns = (len + slice_len - 1) / slice_len;
     if (ns < 1) ns = 1;  // no sources: one slice that writes zeros
+    g.ns = ns;
+    g.slice_len = slice_len;
+    return g;
+}
+
+// Launch one all-pairs evaluation over the sources [src_lo, src_hi) (bodies
+// beyond the last massive one are dropped: they attract nothing under any of
+// the force laws). Targets: every body (targets_dev == null, nt == n) or an
+// explicit list. Output: ctx->acc (out_dev == null) with an optional closing
+// kick, or out_dev[nt*3]. fuse_next: aster_allpairs_can_fuse.
+int aster_allpairs_launch_range(aster_ctx* c, const aster_params* p, int precision, bool closing_kick, int64_t nt,
+                                const int32_t* targets_dev, double* out_dev, int64_t src_lo, int64_t src_hi,
+                                bool fuse_next) {
+    if (precision != ASTER_FP64 && precision != ASTER_MIXED) return ASTER_ERR_INVALID_ARG;
+    if (precision == ASTER_MIXED && !c->mixed_valid) ASTER_TRY(aster_refresh_mixed(c));
+    const int64_t n_src = c->n_src > 0 ? c->n_src : c->n;
+    const int64_t lo = src_lo, hi = src_hi < n_src ? src_hi : n_src;
+    const int64_t len = hi > lo ? hi - lo : 0;
+    if (precision == ASTER_FP64 && !targets_dev && !out_dev && lo == 0 && len == nt && nt == c->n &&
+        aster_allpairs_sym_fits(c, p)) {
+        const int st = aster_allpairs_sym_launch(c, p, closing_kick, fuse_next);
+        if (st != ASTER_ERR_OOM || fuse_next) return st;
+    }
+    const SliceGrid sg = slice_grid(c, p, precision, nt, len);
+    const int64_t ns = sg.ns, slice_len = sg.slice_len;
+    if (fuse_next && (ns < 2 || !closing_kick || out_dev || targets_dev)) return ASTER_ERR_UNSUPPORTED;
     double4* partial = nullptr;
     if (ns > 1) {
         ASTER_TRY(c->scratch.ensure((size_t)ns * nt * sizeof(double4)));
@@ -419,7 +460,7 @@ int aster_allpairs_launch_range(aster_ctx* c, const aster_params* p, int precisi
     }
     KickArgs kick{closing_kick && !out_dev, 0.5 * p->dt, c->vel.as<double4>()};
     if (kick.on) c->mixed_valid = false;  // the closing kick moves the velocities
-    dim3 grid((unsigned)iblocks, (unsigned)ns);
+    dim3 grid((unsigned)sg.iblocks, (unsigned)ns);
     const bool guard = !(p->eps2 > 0.0);
     const int pnl = pn_level(p);
     const int64_t j_hi = lo + len;
@@ -429,11 +470,16 @@ int aster_allpairs_launch_range(aster_ctx* c, const aster_params* p, int precisi
     ASTER_CUDA(cudaGetLastError());
     c->stats.kernels += 1;
     if (ns > 1) {
-        int g = (int)((nt + 255) / 256);
-        k_reduce_slices<<<g, 256, 0, c->stream>>>(nt, (int)ns, partial, targets_dev, p->G, c->acc.as<double4>(),
-                                                  out_dev, kick);
+        const bool mixed = precision == ASTER_MIXED;
+        const NextDrift next{fuse_next ? c->pm.as<double4>() : nullptr, p->dt, mixed ? c->phi.as<float4>() : nullptr,
+                             mixed ? c->plo.as<float4>() : nullptr, mixed ? c->vf.as<float4>() : nullptr};
+        // few targets: small blocks, so that the reduction's latency spreads over the SMs
+        const int rb = nt < 40000 ? 64 : 256;
+        k_reduce_slices<<<(unsigned)((nt + rb - 1) / rb), rb, 0, c->stream>>>(nt, (int)ns, partial, targets_dev, p->G,
+                                                                             c->acc.as<double4>(), out_dev, kick, next);
         ASTER_CUDA(cudaGetLastError());
         c->stats.kernels += 1;
+        if (fuse_next && mixed) c->mixed_valid = true;  // refreshed with the drift
     }
     c->stats.interactions += (double)nt * (double)len;
     return ASTER_OK;
@@ -441,8 +487,18 @@ int aster_allpairs_launch_range(aster_ctx* c, const aster_params* p, int precisi
 
 // Every source body [0, n).
 int aster_allpairs_launch(aster_ctx* c, const aster_params* p, int precision, bool closing_kick, int64_t nt,
-                          const int32_t* targets_dev, double* out_dev) {
-    return aster_allpairs_launch_range(c, p, precision, closing_kick, nt, targets_dev, out_dev, 0, c->n);
+                          const int32_t* targets_dev, double* out_dev, bool fuse_next) {
+    return aster_allpairs_launch_range(c, p, precision, closing_kick, nt, targets_dev, out_dev, 0, c->n, fuse_next);
+}
+
+// Whether an evaluation of all bodies ends in a kernel that adds partial sums,
+// where the next step's opening kick and drift can follow (no other block then
+// reads positions any more). Allocates the symmetric path's partials.
+bool aster_allpairs_can_fuse(aster_ctx* c, const aster_params* p, int precision) {
+    if (precision == ASTER_FP64 && aster_allpairs_sym_fits(c, p))
+        if (aster_allpairs_sym_prepare(c, p) == ASTER_OK) return true;
+    const int64_t n_src = c->n_src > 0 ? c->n_src : c->n;
+    return slice_grid(c, p, precision, c->n, n_src).ns > 1;
 }
 
 extern "C" int aster_allpairs(aster_ctx* c, const aster_params* p, int precision, double* acc_out) {

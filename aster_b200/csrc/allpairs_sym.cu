@@ -246,10 +246,12 @@ __global__ void __launch_bounds__(32 * W, U == 2 ? 8 : 2) k_allpairs_sym(SymArgs
 }
 
 // Sum of a body's slots in slot order, one thread per component (a warp takes
-// 32 bodies of one component), scaled by G; then the closing kick.
+// 32 bodies of one component), scaled by G; then the closing kick and, with pm,
+// the next step's opening kick and drift (the operations of the kick-drift
+// kernel in its order, so that it need not run).
 __global__ void __launch_bounds__(192) k_sym_reduce(int64_t n, int64_t npad, int slots, const double* __restrict__ part,
                                                     double G, double4* __restrict__ acc, double4* __restrict__ vel,
-                                                    double kick_dt) {
+                                                    double kick_dt, double4* __restrict__ pm, double drift_dt) {
     const int c = (threadIdx.x >> 5) % 3;
     const int64_t b = ((int64_t)blockIdx.x * 2 + threadIdx.x / 96) * 32 + (threadIdx.x & 31);
     if (b >= n) return;
@@ -262,8 +264,15 @@ __global__ void __launch_bounds__(192) k_sym_reduce(int64_t n, int64_t npad, int
     o[c] = a;
     if (c == 2) o[3] = 0.0;
     if (vel) {
-        double* v = reinterpret_cast<double*>(vel + b) + c;
-        *v += a * kick_dt;
+        double* vp = reinterpret_cast<double*>(vel + b) + c;
+        double v = *vp;
+        v += a * kick_dt;
+        if (pm) {
+            double* x = reinterpret_cast<double*>(pm + b) + c;
+            v += a * kick_dt;
+            *x += v * drift_dt;
+        }
+        *vp = v;
     }
 }
 
@@ -303,16 +312,12 @@ bool aster_allpairs_sym_fits(const aster_ctx* c, const aster_params* p) {
     return pn_level(p) <= 1 && c->n >= SYM_MIN && c->n_src == c->n && c->n < c->sym_oom_n;
 }
 
-// ASTER_ERR_OOM: no room for the partial array; nothing was launched, and the
-// context's evaluations of this size go to the directed kernel from then on.
-int aster_allpairs_sym_launch(aster_ctx* c, const aster_params* p, bool closing_kick) {
+static SymArgs sym_args(const aster_ctx* c, const aster_params* p) {
     const int pnl = pn_level(p);
-    const int64_t n = c->n;
-    const bool small = n < SYM_SMALL;
-    const int set = small ? 64 : pnl ? 128 : 256;
+    const int set = c->n < SYM_SMALL ? 64 : pnl ? 128 : 256;
     SymArgs g;
-    g.n = n;
-    g.npad = (n + set - 1) / set * set;
+    g.n = c->n;
+    g.npad = (c->n + set - 1) / set * set;
     const int64_t sets = g.npad / set;
     g.tile = (int)((sets + SYM_SLOTS - 1) / SYM_SLOTS) * set;
     if (g.tile > JT) g.tile = (g.tile + JT - 1) / JT * JT;
@@ -322,18 +327,32 @@ int aster_allpairs_sym_launch(aster_ctx* c, const aster_params* p, bool closing_
     g.eps2 = p->eps2;
     g.G = p->G;
     g.c2 = make_pn(p).c2;
+    g.part = nullptr;
+    return g;
+}
+
+// Room for the partial array. ASTER_ERR_OOM: there is none, and the context's
+// evaluations of this size go to the directed kernel from then on.
+int aster_allpairs_sym_prepare(aster_ctx* c, const aster_params* p) {
+    const SymArgs g = sym_args(c, p);
     const int st = c->scratch.ensure((size_t)g.slots * 3 * g.npad * sizeof(double));
-    if (st != ASTER_OK) {
-        if (st == ASTER_ERR_OOM) c->sym_oom_n = n;
-        return st;
-    }
+    if (st == ASTER_ERR_OOM) c->sym_oom_n = c->n;
+    return st;
+}
+
+// One evaluation (ASTER_ERR_OOM: nothing was launched), with the closing kick
+// and, fuse_next, the next step's opening kick and drift.
+int aster_allpairs_sym_launch(aster_ctx* c, const aster_params* p, bool closing_kick, bool fuse_next) {
+    ASTER_TRY(aster_allpairs_sym_prepare(c, p));
+    SymArgs g = sym_args(c, p);
     g.part = c->scratch.as<double>();
-    if (pnl) ASTER_TRY(small ? launch_sym<1, 2, 2>(c, g) : launch_sym<1, 4, 4>(c, g));
+    const int64_t n = c->n;
+    const bool small = n < SYM_SMALL;
+    if (pn_level(p)) ASTER_TRY(small ? launch_sym<1, 2, 2>(c, g) : launch_sym<1, 4, 4>(c, g));
     else ASTER_TRY(small ? launch_sym<0, 2, 2>(c, g) : launch_sym<0, 8, 4>(c, g));
-    k_sym_reduce<<<(unsigned)((n + 63) / 64), 192, 0, c->stream>>>(n, g.npad, g.slots, g.part, p->G,
-                                                                  c->acc.as<double4>(),
-                                                                  closing_kick ? c->vel.as<double4>() : nullptr,
-                                                                  0.5 * p->dt);
+    k_sym_reduce<<<(unsigned)((n + 63) / 64), 192, 0, c->stream>>>(
+        n, g.npad, g.slots, g.part, p->G, c->acc.as<double4>(), closing_kick ? c->vel.as<double4>() : nullptr,
+        0.5 * p->dt, closing_kick && fuse_next ? c->pm.as<double4>() : nullptr, p->dt);
     ASTER_CUDA(cudaGetLastError());
     if (closing_kick) c->mixed_valid = false;  // the closing kick moves the velocities
     c->stats.kernels += 2;

@@ -185,12 +185,17 @@ int aster_copy_acc_out(aster_ctx* ctx, double* acc_out);
 // allpairs.cu
 int aster_allpairs_launch(aster_ctx* ctx, const aster_params* p, int precision,
                           bool closing_kick, int64_t nt, const int32_t* targets_dev,
-                          double* out_dev /* nt*3 or null: write ctx->acc */);
+                          double* out_dev /* nt*3 or null: write ctx->acc */, bool fuse_next = false);
 int aster_allpairs_launch_range(aster_ctx* ctx, const aster_params* p, int precision, bool closing_kick, int64_t nt,
-                                const int32_t* targets_dev, double* out_dev, int64_t src_lo, int64_t src_hi);
+                                const int32_t* targets_dev, double* out_dev, int64_t src_lo, int64_t src_hi,
+                                bool fuse_next = false);
+// fuse_next (with closing_kick, every body): the evaluation also applies the next step's opening kick and drift
+// (and refreshes the FP32 copies, mixed); only where aster_allpairs_can_fuse says so
+bool aster_allpairs_can_fuse(aster_ctx* ctx, const aster_params* p, int precision);
 // allpairs_sym.cu: FP64 forces of all bodies on all bodies, each unordered pair once
 bool aster_allpairs_sym_fits(const aster_ctx* ctx, const aster_params* p);
-int aster_allpairs_sym_launch(aster_ctx* ctx, const aster_params* p, bool closing_kick);
+int aster_allpairs_sym_prepare(aster_ctx* ctx, const aster_params* p);
+int aster_allpairs_sym_launch(aster_ctx* ctx, const aster_params* p, bool closing_kick, bool fuse_next);
 // integrate.cu
 int aster_kick_drift_launch(aster_ctx* ctx, const aster_params* p, bool want_box, bool want_mixed);
 // Enqueue-only cores of the stepping entry points (argument checks included,

@@ -19,9 +19,11 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "aster_internal.cuh"
+#include "fp64_pair.cuh"
 
 namespace {
 
@@ -73,43 +75,97 @@ __global__ void __launch_bounds__(256) k_kick_drift(int64_t n, double half_dt, d
     }
 }
 
-// FP64 energy/momentum: per-block partials (ke, pe, px, py, pz), then one
-// block adds them in a fixed order (deterministic).
+// 1 / r of a pair's potential: r = sqrt(d.d + eps2), or the reference formula's
+// sqrt(d.d) + eps2 (collectors.cpp:43). x = d.d (+ eps2 unless REF_FORM).
 template <bool REF_FORM>
-// Block (x, slice y): bodies i of block x against the sources of slice y,
-// [y * slice_len, (y + 1) * slice_len); the kinetic energy and momentum of i
-// come with slice 0. Partials in part[(y * gridDim.x + x) * 5 + k].
-__global__ void __launch_bounds__(256) k_energy_partial(int64_t n, const double4* __restrict__ pm,
-                                                        const double4* __restrict__ vel, double eps2,
-                                                        int64_t slice_len, double* __restrict__ part) {
-    __shared__ double4 sp[256];
-    __shared__ double red[5][8];
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t j0 = (int64_t)blockIdx.y * slice_len, j1 = min(n, j0 + slice_len);
-    double4 pi = i < n ? pm[i] : make_double4(0, 0, 0, 0);
-    double pot = 0.0;
-    for (int64_t base = j0; base < j1; base += 256) {
+__device__ __forceinline__ double inv_pot_any(double x, double eps2) {
+    return REF_FORM ? 1.0 / (sqrt(x) + eps2) : 1.0 / sqrt(x);
+}
+// The same for an ordinary x (fp64_pair.cuh) and 0 <= eps2 < 1e100. The reference
+// formula: with z the hardware's approximate reciprocal of b = r + eps2 and
+// e = 1 - b z, 1 / b = z (1 + e + e^2 + O(e^3)).
+template <bool REF_FORM>
+__device__ __forceinline__ double inv_pot_fast(double x, double eps2) {
+    const double y = inv_r_fast(x);
+    if (!REF_FORM) return y;
+    const double b = fma(x, y, eps2);
+    double z;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(z) : "d"(b));
+    const double e = fma(-b, z, 1.0);
+    return fma(z, fma(e, e, e), z);
+}
+
+// FP64 energy/momentum: per-block partials (ke, pe, px, py, pz), then one
+// block adds them in a fixed order (deterministic). Block (x, slice y): bodies
+// i of block x (U per thread) with the later ones, j > i, of slice y, so that
+// every pair is formed once: 12 FP64 operations a pair (17 by the reference
+// formula), against about 40 per directed pair with the library's square root
+// and division. The kinetic energy and momentum of i come with slice 0. Partials
+// in part[(y * gridDim.x + x) * 5 + k].
+constexpr int EN_THREADS = 128;
+template <bool REF_FORM, int U>
+__global__ void __launch_bounds__(EN_THREADS) k_energy_partial(int64_t n, const double4* __restrict__ pm,
+                                                               const double4* __restrict__ vel, double eps2,
+                                                               int64_t slice_len, double* __restrict__ part) {
+    __shared__ double4 sp[EN_THREADS];
+    __shared__ double red[5][EN_THREADS / 32];
+    const int64_t i0 = (int64_t)blockIdx.x * EN_THREADS * U;
+    const int64_t j1 = min(n, ((int64_t)blockIdx.y + 1) * slice_len);
+    const bool plain = eps2 < 1e100;
+    const double add = REF_FORM ? 0.0 : eps2;
+    double4 pi[U];
+    double pot[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int64_t i = i0 + u * EN_THREADS + threadIdx.x;
+        pi[u] = i < n ? pm[i] : make_double4(0, 0, 0, 0);
+        pot[u] = 0.0;
+    }
+    for (int64_t base = max((int64_t)blockIdx.y * slice_len, i0); base < j1; base += EN_THREADS) {
         __syncthreads();
         const int64_t j = base + threadIdx.x;
-        sp[threadIdx.x] = j < j1 ? pm[j] : make_double4(0, 0, 0, 0);
+        if (j < j1) sp[threadIdx.x] = pm[j];
         __syncthreads();
-        const int lim = (int)min((int64_t)256, j1 - base);
-        for (int q = 0; q < lim; ++q) {
-            if (base + q == i) continue;
-            const double4 pj = sp[q];
-            double dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-            double r2 = dx * dx + dy * dy + dz * dz;
-            double inv = REF_FORM ? 1.0 / (sqrt(r2) + eps2) : 1.0 / sqrt(r2 + eps2);
-            pot += pj.w * inv;
-        }
+        const int lim = (int)min((int64_t)EN_THREADS, j1 - base);
+        auto tile = [&](auto diag) {  // diag: some j <= i
+            const int i = (int)(i0 - base) + (int)threadIdx.x;  // bodies i, i + EN_THREADS, ... from base
+#pragma unroll 2
+            for (int q = 0; q < lim; ++q) {
+                const double4 pj = sp[q];
+                double x[U], w[U];
+                bool odd = false;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const double dx = pj.x - pi[u].x, dy = pj.y - pi[u].y, dz = pj.z - pi[u].z;
+                    x[u] = fma(dx, dx, fma(dy, dy, fma(dz, dz, add)));
+                    // a body and itself (left out below): keep it off the slow path
+                    if (decltype(diag)::value && q == i + u * EN_THREADS) x[u] = 1.0;
+                    w[u] = inv_pot_fast<REF_FORM>(x[u], eps2);
+                    odd = odd || !r2_ordinary(x[u]);
+                }
+                if (odd || !plain) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (!(plain && r2_ordinary(x[u]))) w[u] = inv_pot_any<REF_FORM>(x[u], eps2);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (!decltype(diag)::value || q > i + u * EN_THREADS) pot[u] = fma(pj.w, w[u], pot[u]);
+            }
+        };
+        if (base < i0 + EN_THREADS * U) tile(std::true_type{});
+        else tile(std::false_type{});
     }
     double v[5] = {0, 0, 0, 0, 0};
-    if (i < n) {
-        v[1] = -0.5 * pi.w * pot;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int64_t i = i0 + u * EN_THREADS + threadIdx.x;
+        if (i >= n) continue;
+        v[1] -= pi[u].w * pot[u];
         if (blockIdx.y == 0) {
             const double4 vi = vel[i];
-            v[0] = 0.5 * pi.w * (vi.x * vi.x + vi.y * vi.y + vi.z * vi.z);
-            v[2] = pi.w * vi.x; v[3] = pi.w * vi.y; v[4] = pi.w * vi.z;
+            v[0] += 0.5 * pi[u].w * (vi.x * vi.x + vi.y * vi.y + vi.z * vi.z);
+            v[2] += pi[u].w * vi.x; v[3] += pi[u].w * vi.y; v[4] += pi[u].w * vi.z;
         }
     }
     for (int k = 0; k < 5; ++k) {
@@ -120,7 +176,7 @@ __global__ void __launch_bounds__(256) k_energy_partial(int64_t n, const double4
     __syncthreads();
     if (threadIdx.x < 5) {
         double s = 0;
-        for (int w = 0; w < 8; ++w) s += red[threadIdx.x][w];
+        for (int w = 0; w < EN_THREADS / 32; ++w) s += red[threadIdx.x][w];
         part[((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * 5 + threadIdx.x] = s;
     }
 }
@@ -134,6 +190,7 @@ __global__ void __launch_bounds__(160) k_energy_final(int nparts, const double* 
     const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (k < 5) {
         double a = 0;
+#pragma unroll 8
         for (int b = lane; b < nparts; b += 32) a += part[(int64_t)b * 5 + k];
         for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
         if (lane == 0) s[k] = a;
@@ -216,7 +273,7 @@ static int force_eval(aster_ctx* c, const aster_params* p, int solver, int preci
                       bool fuse_next = false) {
     int e0 = tm ? tm->mark(c->stream) : -1;
     if (solver == ASTER_SOLVER_ALLPAIRS) {
-        ASTER_TRY(aster_allpairs_launch(c, p, precision, closing_kick, c->n, nullptr, nullptr));
+        ASTER_TRY(aster_allpairs_launch(c, p, precision, closing_kick, c->n, nullptr, nullptr, fuse_next));
         if (tm) pairs[0] = e0, pairs[1] = e0, pairs[2] = tm->mark(c->stream);
         return ASTER_OK;
     }
@@ -408,13 +465,14 @@ static int kdk_core(aster_ctx* c, const aster_params* p, int solver, int precisi
         ASTER_TRY(aster_kick_drift_launch(c, p, solver == ASTER_SOLVER_LBVH, mixed_ap));
         return force_eval(c, p, solver, precision, true, true, tm, nullptr, nullptr, last);
     };
-    // Tree steps: every walk but the last also applies the next step's opening
-    // kick and drift (and its bounding box), so only the first step launches
-    // the kick-drift kernel: first = kick-drift + build + walk(fused), middle =
-    // build + walk(fused) (captured and replayed), last = build + walk.
-    const bool fuse = solver == ASTER_SOLVER_LBVH && nsteps >= 2;
+    // Every force evaluation but the last also applies the next step's opening
+    // kick and drift (tree: in the walk, with the bounding box; all-pairs:
+    // where the partial sums are added), so only the first step launches the
+    // kick-drift kernel: first = kick-drift + force(fused), middle =
+    // force(fused) (captured and replayed), last = force.
+    const bool fuse = nsteps >= 2 && (solver == ASTER_SOLVER_LBVH || aster_allpairs_can_fuse(c, p, precision));
     auto first = [&]() -> int {
-        ASTER_TRY(aster_kick_drift_launch(c, p, true, false));
+        ASTER_TRY(aster_kick_drift_launch(c, p, solver == ASTER_SOLVER_LBVH, mixed_ap));
         return force_eval(c, p, solver, precision, true, true, tm, nullptr, nullptr, last, true);
     };
     auto middle = [&]() -> int { return force_eval(c, p, solver, precision, true, true, tm, nullptr, nullptr, last, true); };
@@ -726,36 +784,44 @@ extern "C" int aster_saba_steps(aster_ctx* c, const aster_params* p, int solver,
     return st;
 }
 
-// FP64 energy and momentum of the resident state into out4 (device:
-// energy, px, py, pz); part holds (n + 255) / 256 * 5 doubles. No sync.
-// Source slices of the energy sum: enough blocks to fill the GPU when n is
-// small (each slice a whole number of 256-body tiles).
-static int energy_slices(const aster_ctx* c, int64_t n) {
-    const int64_t tiles = (n + 255) / 256;
-    int64_t ns = ((int64_t)4 * c->sm_count + tiles - 1) / tiles;
-    if (ns > tiles) ns = tiles;
-    if (ns > 64) ns = 64;
-    if (ns < 1) ns = 1;
-    return (int)ns;
+// Shape of the energy sum: bodies per thread, blocks of bodies and slices of
+// sources (whole 128-body tiles), enough blocks to fill the GPU when n is small.
+struct EnergyGrid {
+    int u;
+    int64_t blocks, slices, slice_len;
+};
+static EnergyGrid energy_grid(const aster_ctx* c, int64_t n) {
+    EnergyGrid g;
+    g.u = n < 8000 ? 2 : 4;
+    g.blocks = (n + EN_THREADS * g.u - 1) / (EN_THREADS * g.u);
+    const int64_t tiles = (n + EN_THREADS - 1) / EN_THREADS;
+    // half the blocks lie below the diagonal and end at once
+    int64_t ns = ((int64_t)16 * c->sm_count + g.blocks - 1) / g.blocks;
+    ns = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(ns, tiles), 64));
+    g.slice_len = (tiles + ns - 1) / ns * EN_THREADS;
+    g.slices = (n + g.slice_len - 1) / g.slice_len;
+    return g;
 }
 
 // Partials (5 doubles each) that aster_energy_enqueue writes.
-int64_t aster_energy_parts(const aster_ctx* c) { return (c->n + 255) / 256 * energy_slices(c, c->n); }
+int64_t aster_energy_parts(const aster_ctx* c) {
+    const EnergyGrid g = energy_grid(c, c->n);
+    return g.blocks * g.slices;
+}
 
+// FP64 energy and momentum of the resident state into out4 (device:
+// energy, px, py, pz); part holds aster_energy_parts * 5 doubles. No sync.
 int aster_energy_enqueue(aster_ctx* c, const aster_params* p, int ref_form, double* part, double* out4) {
     const int64_t n = c->n;
-    const int nb = (int)((n + 255) / 256);
-    const int ns = energy_slices(c, n);
-    const int64_t slice_len = (nb + ns - 1) / ns * (int64_t)256;
-    const dim3 grid((unsigned)nb, (unsigned)ns);
-    if (ref_form)
-        k_energy_partial<true><<<grid, 256, 0, c->stream>>>(n, c->pm.as<double4>(), c->vel.as<double4>(), p->eps2,
-                                                            slice_len, part);
-    else
-        k_energy_partial<false><<<grid, 256, 0, c->stream>>>(n, c->pm.as<double4>(), c->vel.as<double4>(), p->eps2,
-                                                             slice_len, part);
+    const EnergyGrid g = energy_grid(c, n);
+    const dim3 grid((unsigned)g.blocks, (unsigned)g.slices);
+    const double4 *pm = c->pm.as<double4>(), *vel = c->vel.as<double4>();
+    if (ref_form && g.u == 2) k_energy_partial<true, 2><<<grid, EN_THREADS, 0, c->stream>>>(n, pm, vel, p->eps2, g.slice_len, part);
+    else if (ref_form) k_energy_partial<true, 4><<<grid, EN_THREADS, 0, c->stream>>>(n, pm, vel, p->eps2, g.slice_len, part);
+    else if (g.u == 2) k_energy_partial<false, 2><<<grid, EN_THREADS, 0, c->stream>>>(n, pm, vel, p->eps2, g.slice_len, part);
+    else k_energy_partial<false, 4><<<grid, EN_THREADS, 0, c->stream>>>(n, pm, vel, p->eps2, g.slice_len, part);
     ASTER_CUDA(cudaGetLastError());
-    k_energy_final<<<1, 160, 0, c->stream>>>(nb * ns, part, p->G, out4);
+    k_energy_final<<<1, 160, 0, c->stream>>>((int)(g.blocks * g.slices), part, p->G, out4);
     ASTER_CUDA(cudaGetLastError());
     return ASTER_OK;
 }
@@ -822,11 +888,11 @@ extern "C" int aster_energy_noalloc(int64_t n, const double* pm_dev, const doubl
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const double4* pm = reinterpret_cast<const double4*>(pm_dev);
     const double4* vel = reinterpret_cast<const double4*>(vel_dev);
-    const int64_t whole = (int64_t)nb * 256;  // one slice: every source
+    const int64_t whole = (int64_t)nb * 256;  // one slice: every source; 2 bodies per thread, 256 per block
     if (ref_form)
-        k_energy_partial<true><<<nb, 256, 0, st>>>(n, pm, vel, p->eps2, whole, part);
+        k_energy_partial<true, 2><<<nb, EN_THREADS, 0, st>>>(n, pm, vel, p->eps2, whole, part);
     else
-        k_energy_partial<false><<<nb, 256, 0, st>>>(n, pm, vel, p->eps2, whole, part);
+        k_energy_partial<false, 2><<<nb, EN_THREADS, 0, st>>>(n, pm, vel, p->eps2, whole, part);
     ASTER_CUDA(cudaGetLastError());
     k_energy_final<<<1, 160, 0, st>>>(nb, part, p->G, out_dev);
     ASTER_CUDA(cudaGetLastError());

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 from aster_b200 import gen
-from aster_b200.api import FP64, NEWTON, PN1, SOLVER_ALLPAIRS, Params
+from aster_b200.api import FP64, MIXED, NEWTON, PN1, PN2, SOLVER_ALLPAIRS, Params
 from conftest import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -91,3 +91,56 @@ def test_repeated_evaluations_are_identical(ctx):
     ctx.upload(pos, vel, m)
     ctx.kdk_steps(p, 0, SOLVER_ALLPAIRS, FP64)
     np.testing.assert_array_equal(a, ctx.download()[2])
+
+
+@pytest.mark.parametrize("n", [1, 2, 127, 129, 256, 257, 7999, 8000, 8193])
+@pytest.mark.parametrize("ref_form", [False, True])
+@pytest.mark.parametrize("eps2", [0.0, 1e-4])
+def test_energy_of_every_pair_once(ctx, n, ref_form, eps2):
+    """Block and slice edges of the energy sum (2 and 4 bodies per thread), 1e-12 against numpy's sum over i < j."""
+    pos, vel, m = gen.plummer(n, 60 + n, masses="lognormal")
+    pot = 0.0
+    for i in range(n - 1):
+        r2 = ((pos[i + 1:] - pos[i]) ** 2).sum(1)
+        pot -= (m[i] * m[i + 1:] / (np.sqrt(r2) + eps2 if ref_form else np.sqrt(r2 + eps2))).sum()
+    ke = 0.5 * (m * (vel * vel).sum(1)).sum()
+    ctx.upload(pos, vel, m)
+    e, mom = ctx.energy(Params(eps2=eps2), ref_form=ref_form)
+    assert abs(e - (ke + pot)) <= 1e-12 * (ke + abs(pot))
+    np.testing.assert_allclose(mom, (m[:, None] * vel).sum(0), rtol=0, atol=1e-14)
+
+
+def test_energy_of_bodies_in_one_place(ctx):
+    """1 / r of two bodies in one place: infinite without softening, 1 / eps2 in the reference formula, 1 / eps
+    otherwise; and squared distances far outside the series step's range."""
+    pos = np.array([[0.5, 0.25, 0.0], [0.5, 0.25, 0.0], [1.5, 0.25, 0.0]])
+    m = np.array([2.0, 3.0, 1.0])
+    ctx.upload(pos, None, m)
+    assert ctx.energy(Params(eps2=0.0))[0] == -np.inf
+    assert abs(ctx.energy(Params(eps2=0.25), ref_form=True)[0] + 6.0 / 0.25 + 5.0 / 1.25) < 1e-14 * 28
+    assert abs(ctx.energy(Params(eps2=0.25))[0] + 6.0 / 0.5 + 5.0 / np.sqrt(1.25)) < 1e-14 * 16
+    for k in (2.0 ** 400, 2.0 ** -400):
+        ctx.upload(np.array([[0.0, 0.0, 0.0], [k, 0.0, 0.0]]), None, np.array([1.0, 1.0]))
+        assert abs(ctx.energy(Params())[0] * k + 1.0) < 1e-14
+        assert abs(ctx.energy(Params(), ref_form=True)[0] * k + 1.0) < 1e-14
+
+
+# every path that ends in a kernel adding partial sums: symmetric FP64 (small and large tiles, 1PN), directed FP64
+# (below the symmetric size, every PN term), mixed slices, mixed with PN terms; and mixed without slices
+@pytest.mark.parametrize("n,prec,law", [(100, FP64, NEWTON), (1000, FP64, NEWTON), (5000, FP64, NEWTON),
+                                        (5000, FP64, NEWTON | PN1), (700, FP64, NEWTON | PN1 | PN2),
+                                        (3000, MIXED, NEWTON), (3000, MIXED, NEWTON | PN1), (40, MIXED, NEWTON)])
+def test_fused_drift_equals_single_steps(ctx, n, prec, law):
+    """A multi-step run applies each next step's opening kick and drift where the forces are added up; single-step
+    calls run the kick-drift kernel. The same state bit for bit."""
+    pos, vel, m = gen.plummer(n, 70 + n, masses="lognormal")
+    p = Params(eps2=1e-4, dt=1e-3, c=50.0, force_law=law)
+    out = []
+    for split in ((7,), (1,) * 7, (2, 5)):
+        ctx.upload(pos, vel, m)
+        for k in split:
+            ctx.kdk_steps(p, k, SOLVER_ALLPAIRS, prec)
+        out.append(ctx.download())
+    for o in out[1:]:
+        for a, b in zip(out[0], o):
+            np.testing.assert_array_equal(a, b)
