@@ -27,18 +27,22 @@
 #include <algorithm>
 
 #include "aster_internal.cuh"
+#include "fp64_pair.cuh"
 
 namespace {
 
 constexpr int WH_BLOCK = 256;
+constexpr int WH_SRC = 64;  // massive bodies up to which k_wh_cba forms the interaction itself
 
-// state scalars in ctx->wh after the partials: [0] m0, [1] M, [2..4] x_cm,
+// ctx->wh: two copies of the massive bodies (positions before and after a
+// step's drift, WH_SRC each), the reduction partials, then the state scalars: [0] m0, [1] M, [2..4] x_cm,
 // [5..7] v_cm, [8..11] reduction result (sum m a.x, .y, .z, sum m), [12..14]
 // sum m v, [16..18] sum m Q, [20..22] sum m x, [24..27] the second slot for P
 // (k_wh_cba reads P from one slot and writes the next P to the other), [30] the
 // reductions' block counter (an unsigned int, zero between launches)
 struct WhLayout {
     int64_t nb;  // reduction blocks
+    double4* src[2];
     double* part;
     double* st;
 };
@@ -47,7 +51,9 @@ WhLayout wh_layout(aster_ctx* c) {
     WhLayout L;
     L.nb = std::min<int64_t>((c->n + WH_BLOCK - 1) / WH_BLOCK, (int64_t)c->sm_count * 4);
     if (L.nb < 1) L.nb = 1;
-    L.part = c->wh.as<double>();
+    L.src[0] = c->wh.as<double4>();
+    L.src[1] = L.src[0] + WH_SRC;
+    L.part = reinterpret_cast<double*>(L.src[1] + WH_SRC);
     L.st = L.part + 4 * L.nb;
     return L;
 }
@@ -171,7 +177,13 @@ __device__ bool kepler_drift(double3& r, double3& v, double mu, double dt) {
     const double s0 = (r.x * v.x + r.y * v.y + r.z * v.z) / smu;
     const double a = 2.0 / r0 - v2 / mu;
     const double b = 1.0 - a * r0;
-    double chi = smu * dt / r0, c2 = 0.5, c3 = 1.0 / 6.0;
+    // start: the universal Kepler equation r0 chi + s0 chi^2/2 + b chi^3/6 + ... =
+    // sqrt(mu) dt inverted as a series in q = sqrt(mu) dt / r0 to q^3, where that
+    // is small; q itself otherwise
+    const double q = smu * dt / r0, ir0 = 1.0 / r0, sg = s0 * ir0;
+    const double g3 = 0.5 * sg * sg - b * ir0 * (1.0 / 6.0);
+    const double dq = q * q * fma(g3, q, -0.5 * sg);
+    double chi = fabs(dq) < 0.2 * fabs(q) ? q + dq : q, c2 = 0.5, c3 = 1.0 / 6.0;
     bool ok = false;
     for (int it = 0; it < 64; ++it) {
         const double z = a * chi * chi;
@@ -183,7 +195,9 @@ __device__ bool kepler_drift(double3& r, double3& v, double mu, double dt) {
         const double den = Fp + (Fp >= 0.0 ? 1.0 : -1.0) * sqrt(disc);
         const double d = den != 0.0 ? 5.0 * F / den : F / Fp;
         chi -= d;
-        if (fabs(d) <= 1e-15 * (1.0 + fabs(chi))) {
+        // Laguerre's iteration converges cubically at a simple root: a correction
+        // of 1e-8 leaves an error far below the rounding of chi
+        if (fabs(d) <= 1e-8 * fabs(chi) || fabs(d) <= 1e-15 * (1.0 + fabs(chi))) {
             ok = true;
             break;
         }
@@ -202,28 +216,75 @@ __device__ bool kepler_drift(double3& r, double3& v, double mu, double dt) {
     return true;
 }
 
-// Per body i >= 1: C(hc) with P = pin[0..2], B(hb) with the cached
-// interaction acc, A(dt); then P = sum m_i V_i after the drift into pout[0..2]
-// (pout[3] = sum m_i), pin and pout distinct slots of the state scalars.
+// Interaction of the massive bodies src[1 .. nsrc) (shared memory) on the body
+// at p, FP64 (the operations of the all-pairs kernel; the body itself gives 0).
+__device__ __forceinline__ double4 wh_interaction(const double4* __restrict__ src, int nsrc, const double4 p, double G,
+                                                  double eps2) {
+    double ax = 0.0, ay = 0.0, az = 0.0;
+    for (int j = 1; j < nsrc; ++j) {
+        const double4 s = src[j];
+        const double dx = s.x - p.x, dy = s.y - p.y, dz = s.z - p.z;
+        const double t = m_inv_r3(s.w, fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
+        ax = fma(dx, t, ax); ay = fma(dy, t, ay); az = fma(dz, t, az);
+    }
+    return make_double4(G * ax, G * ay, G * az, 0.0);
+}
+
+// Per body i >= 1: C(hc) with P = pin[0..2], B(hb) with the interaction, A(dt);
+// then P = sum m_i V_i after the drift into pout[0..2] (pout[3] = sum m_i), pin
+// and pout distinct slots of the state scalars. FUSED (at most WH_SRC massive
+// bodies, FP64): the interaction is formed here from src_in, the massive bodies'
+// positions before this step, and src_out gets those after it (blocks move pm
+// under one another); otherwise it is the cached acc. With a handful of planets
+// a separate interaction kernel was a launch and 64 bytes a body (7.9 us of a
+// step's 30 at 262,144 test particles) for nine sources.
+template <bool FUSED>
 __global__ void __launch_bounds__(WH_BLOCK) k_wh_cba(int64_t n, double4* __restrict__ pm, double4* __restrict__ vel,
                                                      const double4* __restrict__ acc, const double* st,
                                                      const double* pin, double hc, double hb, double mu, double dt,
                                                      int* __restrict__ err, double* part, unsigned int* done,
-                                                     double* pout) {
+                                                     double* pout, int nsrc, const double4* __restrict__ src_in,
+                                                     double4* __restrict__ src_out, double G, double eps2) {
+    __shared__ double4 src[FUSED ? WH_SRC : 1];
+    if (FUSED) {
+        if ((int)threadIdx.x < nsrc) src[threadIdx.x] = src_in[threadIdx.x];
+        __syncthreads();
+    }
     const double m0 = st[0];
     const double px = pin[0] / m0 * hc, py = pin[1] / m0 * hc, pz = pin[2] / m0 * hc;
     double sum[4] = {0, 0, 0, 0};
     for (int64_t i = 1 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double4 p = pm[i], v = vel[i];
-        const double4 a = acc[i];
+        const double4 a = FUSED ? wh_interaction(src, nsrc, p, G, eps2) : acc[i];
         double3 r = make_double3(p.x + px, p.y + py, p.z + pz);
         double3 u = make_double3(v.x + a.x * hb, v.y + a.y * hb, v.z + a.z * hb);
         if (!kepler_drift(r, u, mu, dt)) atomicOr(err, ASTER_DEVERR_KEPLER);
-        pm[i] = make_double4(r.x, r.y, r.z, p.w);
+        p = make_double4(r.x, r.y, r.z, p.w);
+        pm[i] = p;
+        if (FUSED && i < nsrc) src_out[i] = p;
         vel[i] = make_double4(u.x, u.y, u.z, v.w);
         sum[0] += p.w * u.x; sum[1] += p.w * u.y; sum[2] += p.w * u.z; sum[3] += p.w;
     }
     block_sum4_last(sum, part, done, pout);
+}
+
+// The run's last C(h) and B(h) with the interaction of src_in.
+__global__ void __launch_bounds__(WH_BLOCK) k_wh_cb(int64_t n, double4* __restrict__ pm, double4* __restrict__ vel,
+                                                    const double* st, const double* pin, double h, int nsrc,
+                                                    const double4* __restrict__ src_in, double G, double eps2) {
+    __shared__ double4 src[WH_SRC];
+    if ((int)threadIdx.x < nsrc) src[threadIdx.x] = src_in[threadIdx.x];
+    __syncthreads();
+    const double m0 = st[0];
+    const double px = pin[0] / m0 * h, py = pin[1] / m0 * h, pz = pin[2] / m0 * h;
+    for (int64_t i = 1 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        double4 p = pm[i], v = vel[i];
+        const double4 a = wh_interaction(src, nsrc, p, G, eps2);
+        v.x += a.x * h; v.y += a.y * h; v.z += a.z * h;
+        p.x += px; p.y += py; p.z += pz;
+        pm[i] = p;
+        vel[i] = v;
+    }
 }
 
 // C(h) alone with P = pin[0..2] (a run's last half step; B follows in the
@@ -319,7 +380,7 @@ int aster_wh_enqueue(aster_ctx* c, const aster_params* p, int precision, int nst
     ASTER_TRY(wh_check(c, p, precision, nsteps));
     const int64_t n = c->n;
     const int64_t nbmax = std::min<int64_t>((n + WH_BLOCK - 1) / WH_BLOCK, (int64_t)c->sm_count * 4);
-    ASTER_TRY(c->wh.ensure((size_t)(4 * std::max<int64_t>(nbmax, 1) + 32) * sizeof(double)));
+    ASTER_TRY(c->wh.ensure(2 * WH_SRC * sizeof(double4) + (size_t)(4 * std::max<int64_t>(nbmax, 1) + 32) * sizeof(double)));
     const WhLayout L = wh_layout(c);
     ASTER_CUDA(cudaMemsetAsync(L.st + 30, 0, sizeof(double), c->stream));  // arm the reduction counter
     c->mixed_valid = false;  // the steps move positions and velocities (mixed runs refresh as they go)
@@ -347,19 +408,37 @@ int aster_wh_enqueue(aster_ctx* c, const aster_params* p, int precision, int nst
     unsigned int* cnt = reinterpret_cast<unsigned int*>(L.st + 30);
     double* pslot[2] = {L.st + 8, L.st + 24};
     int cur = 0;
+    // few massive bodies: the interaction inside the drift kernel
+    const int nsrc = (int)std::min<int64_t>(c->n_src, WH_SRC + 1);
+    const bool fused = precision == ASTER_FP64 && nsrc <= WH_SRC;
+    if (fused && nsteps > 0)
+        ASTER_CUDA(cudaMemcpyAsync(L.src[0], pm, (size_t)nsrc * sizeof(double4), cudaMemcpyDeviceToDevice, c->stream));
     for (int s = 0; s < nsteps && st == ASTER_OK; ++s) {
         if (precision == ASTER_MIXED && (st = aster_refresh_mixed(c)) != ASTER_OK) break;
-        if ((st = aster_allpairs_launch(c, p, precision, false, n, nullptr, nullptr)) != ASTER_OK) break;
+        if (!fused && (st = aster_allpairs_launch(c, p, precision, false, n, nullptr, nullptr)) != ASTER_OK) break;
         if (s == 0 && (st = wh_reduce(c, L, 1, vel)) != ASTER_OK) break;  // P of the initial state
         const double hcb = s == 0 ? h : dt;
-        k_wh_cba<<<grid, WH_BLOCK, 0, c->stream>>>(n, pm, vel, c->acc.as<double4>(), L.st, pslot[cur], hcb, hcb, mu,
-                                                   dt, c->err_dev, L.part, cnt, pslot[cur ^ 1]);
+        if (fused) {
+            k_wh_cba<true><<<grid, WH_BLOCK, 0, c->stream>>>(n, pm, vel, nullptr, L.st, pslot[cur], hcb, hcb, mu, dt,
+                                                             c->err_dev, L.part, cnt, pslot[cur ^ 1], nsrc, L.src[s & 1],
+                                                             L.src[(s & 1) ^ 1], p->G, p->eps2);
+            c->stats.interactions += (double)n * (double)nsrc;
+        } else {
+            k_wh_cba<false><<<grid, WH_BLOCK, 0, c->stream>>>(n, pm, vel, c->acc.as<double4>(), L.st, pslot[cur], hcb,
+                                                              hcb, mu, dt, c->err_dev, L.part, cnt, pslot[cur ^ 1], 0,
+                                                              nullptr, nullptr, p->G, p->eps2);
+        }
         if ((st = wh_launch_status()) != ASTER_OK) break;
         cur ^= 1;
         ++done;
         c->stats.kernels += 1;
     }
-    if (st == ASTER_OK && done > 0) {  // the last C(h) B(h)
+    if (st == ASTER_OK && done > 0 && fused) {  // the last C(h) B(h)
+        k_wh_cb<<<grid, WH_BLOCK, 0, c->stream>>>(n, pm, vel, L.st, pslot[cur], h, nsrc, L.src[done & 1], p->G, p->eps2);
+        st = wh_launch_status();
+        c->stats.kernels += 1;
+        c->stats.interactions += (double)n * (double)nsrc;
+    } else if (st == ASTER_OK && done > 0) {
         k_wh_c<<<grid, WH_BLOCK, 0, c->stream>>>(n, pm, L.st, pslot[cur], h);
         st = wh_launch_status();
         c->stats.kernels += 1;
