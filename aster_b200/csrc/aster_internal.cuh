@@ -146,6 +146,8 @@ struct aster_ctx {
     // [0], [1] timing; [2] final positions ready; [3] upload copies issued;
     // [4] masses copied (overlapped upload)
     cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t dl_ev[16] = {};  // pieces of a staged copy to the host (created on first use)
+    bool counted = false;        // one of the contexts that keep the copies' slab
     // masses still on their way (overlapped upload): staging copy on the
     // device, applied to pm[].w before the tree build reads them
     const double* mass_pending = nullptr;
@@ -180,6 +182,8 @@ int aster_download_va_enqueue(aster_ctx* c, double* vel, double* acc, cudaStream
 // applies masses still on their way (waits for their copy); no-op otherwise
 int aster_apply_pending_mass(aster_ctx* c);
 int aster_copy_acc_out(aster_ctx* ctx, double* acc_out);
+// device arrays -> host arrays (null destinations skipped) after the stream's work; synchronised on return
+int aster_copy_to_host(aster_ctx* c, void* const* dst, const void* const* src, const size_t* bytes, int count);
 
 // ---- kernels exposed across translation units ------------------------------
 // allpairs.cu

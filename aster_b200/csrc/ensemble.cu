@@ -823,18 +823,16 @@ extern "C" int aster_ensemble_download(aster_ctx* c, double* pos, double* vel) {
     ASTER_TRY(c->stage.ensure(2 * v3));
     double* st = c->stage.as<double>();
     const int grid = (int)std::min<int64_t>((nb + 255) / 256, (int64_t)c->sm_count * 16);
-    if (pos) {
-        k_unpack_ens<<<grid, 256, 0, c->stream>>>(nb, e.pm.as<double4>(), st);
+    void* const dsts[2] = {pos, vel};
+    const void* const stage[2] = {st, st + 3 * nb};
+    const size_t bytes[2] = {v3, v3};
+    const DevBuf* srcs[2] = {&e.pm, &e.vel};
+    for (int k = 0; k < 2; ++k) {
+        if (!dsts[k]) continue;
+        k_unpack_ens<<<grid, 256, 0, c->stream>>>(nb, srcs[k]->as<double4>(), st + 3 * nb * k);
         ASTER_CUDA(cudaGetLastError());
-        ASTER_CUDA(cudaMemcpyAsync(pos, st, v3, cudaMemcpyDeviceToHost, c->stream));
     }
-    if (vel) {
-        k_unpack_ens<<<grid, 256, 0, c->stream>>>(nb, e.vel.as<double4>(), st + 3 * nb);
-        ASTER_CUDA(cudaGetLastError());
-        ASTER_CUDA(cudaMemcpyAsync(vel, st + 3 * nb, v3, cudaMemcpyDeviceToHost, c->stream));
-    }
-    ASTER_CUDA(cudaStreamSynchronize(c->stream));
-    return ASTER_OK;
+    return aster_copy_to_host(c, dsts, stage, bytes, 2);
 }
 
 extern "C" int aster_ensemble_run(aster_ctx* c, const aster_params* p, int integrator, int precision, int64_t nsteps,
