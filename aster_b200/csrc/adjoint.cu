@@ -263,15 +263,45 @@ __global__ void __launch_bounds__(BLOCK) k_adj_pair_fp64(int64_t n, const double
         if (kk[q] < n) adj_store(kk[q], ax[q], ay[q], az[q], ag[q], G, nslices, slice, n, partial, lx, lm);
 }
 
-__global__ void k_adj_reduce(int64_t n, int nslices, const double4* __restrict__ partial, double G,
-                             double4* __restrict__ lx, double* __restrict__ lm) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-        double jx = 0, jy = 0, jz = 0, g = 0;
-        for (int s = 0; s < nslices; ++s) {
-            const double4 p = partial[(int64_t)s * n + k];
-            jx += p.x; jy += p.y; jz += p.z; g += p.w;
+// What k_adj_pre does for the next (earlier) step, applied where the slices are
+// added: lv' = lv + dt lx, w = scale lv'.
+struct AdjNext {
+    bool on, mixed;
+    double4* lv;
+    void* w;
+    double dt, scale;
+};
+
+// One thread per body and component (the fourth is the mass gradient).
+__global__ void __launch_bounds__(256) k_adj_reduce(int64_t n, int nslices, const double4* __restrict__ partial,
+                                                    double G, double4* __restrict__ lx, double* __restrict__ lm,
+                                                    AdjNext next) {
+    const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, b = id >> 2;
+    const int k = (int)(id & 3);
+    if (b >= n) return;
+    const double* p = reinterpret_cast<const double*>(partial) + id;
+    double j = 0.0;
+#pragma unroll 8
+    for (int s = 0; s < nslices; ++s) j += p[(int64_t)s * n * 4];
+    if (k == 3) {
+        lm[b] += G * j;
+        if (next.on) {
+            if (next.mixed) static_cast<float*>(next.w)[id] = 0.f;
+            else static_cast<double*>(next.w)[id] = 0.0;
         }
-        adj_store(k, jx, jy, jz, g, G, 1, 0, n, nullptr, lx, lm);
+        return;
+    }
+    double* xp = reinterpret_cast<double*>(lx + b) + k;
+    double a = *xp;
+    a += G * j;
+    *xp = a;
+    if (next.on) {
+        double* vp = reinterpret_cast<double*>(next.lv + b) + k;
+        double v = *vp;
+        v += next.dt * a;
+        *vp = v;
+        if (next.mixed) static_cast<float*>(next.w)[id] = (float)(next.scale * v);
+        else static_cast<double*>(next.w)[id] = next.scale * v;
     }
 }
 
@@ -282,16 +312,14 @@ __global__ void k_unpack_d4(int64_t n, const double4* __restrict__ src, double* 
     }
 }
 
-int adj_pair_launch(aster_ctx* c, const aster_params* p, int precision, const double4* xs) {
+// *next: in, the pre-step of the next sweep step to apply; out, on = whether it
+// was (not without slices).
+int adj_pair_launch(aster_ctx* c, const aster_params* p, int precision, const double4* xs, AdjNext* next) {
     AdjBufs& a = c->adj;
     const int64_t n = c->n;
     const int64_t iblocks = (n + BLOCK * IPT - 1) / (BLOCK * IPT);
-    int64_t want = ASTER_SLICE_BLOCKS_PER_SM * (int64_t)c->sm_count;
-    int64_t ns = iblocks >= want ? 1 : (want + iblocks - 1) / iblocks;
-    const int64_t max_ns = (n + BLOCK - 1) / BLOCK;
-    ns = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(ns, max_ns), 64));
-    const int64_t slice_len = ((n + ns - 1) / ns + BLOCK - 1) / BLOCK * BLOCK;
-    ns = (n + slice_len - 1) / slice_len;
+    const int64_t slice_len = aster_slice_tiles(iblocks, (n + BLOCK - 1) / BLOCK, c->sm_count) * BLOCK;
+    const int64_t ns = (n + slice_len - 1) / slice_len;
     double4* partial = nullptr;
     if (ns > 1) {
         ASTER_TRY(a.part.ensure((size_t)ns * n * sizeof(double4)));
@@ -321,18 +349,16 @@ int adj_pair_launch(aster_ctx* c, const aster_params* p, int precision, const do
     ASTER_CUDA(cudaGetLastError());
     c->stats.kernels += 1;
     if (ns > 1) {
-        k_adj_reduce<<<(int)((n + 255) / 256), 256, 0, c->stream>>>(n, (int)ns, partial, p->G, a.lx.as<double4>(),
-                                                                  a.lm.as<double>());
+        const int rb = n < 10000 ? 64 : 256;
+        k_adj_reduce<<<(unsigned)((4 * n + rb - 1) / rb), rb, 0, c->stream>>>(n, (int)ns, partial, p->G,
+                                                                             a.lx.as<double4>(), a.lm.as<double>(),
+                                                                             *next);
         ASTER_CUDA(cudaGetLastError());
         c->stats.kernels += 1;
+    } else {
+        next->on = false;
     }
     return ASTER_OK;
-}
-
-// One forward KDK step of the context state (the aster_kdk_steps step).
-int forward_step(aster_ctx* c, const aster_params* p, int precision) {
-    ASTER_TRY(aster_kick_drift_launch(c, p, false, precision == ASTER_MIXED));
-    return aster_allpairs_launch(c, p, precision, true, c->n, nullptr, nullptr);
 }
 
 int copy_d2d(aster_ctx* c, void* dst, const void* src, size_t bytes) {
@@ -378,13 +404,19 @@ extern "C" int aster_adjoint_leapfrog(aster_ctx* c, const aster_params* p, int p
     // forward pass with checkpoints
     if (precision == ASTER_MIXED) ASTER_TRY(aster_refresh_mixed(c));
     ASTER_TRY(aster_allpairs_launch(c, p, precision, false, n, nullptr, nullptr));  // a(x0)
+    // (a force evaluation also applies the next step's opening kick and drift
+    // unless a checkpoint of the state between the steps is due)
+    const bool mixed = precision == ASTER_MIXED, can_fuse = aster_allpairs_can_fuse(c, p, precision);
+    bool drifted = false;
     for (int64_t s = 0; s < nsteps; ++s) {
         if (s % K == 0) {
             ASTER_TRY(copy_d2d(c, ck_x(s / K), c->pm.ptr, v4));
             ASTER_TRY(copy_d2d(c, ck_v(s / K), c->vel.ptr, v4));
             ASTER_TRY(copy_d2d(c, ck_a(s / K), c->acc.ptr, v4));
         }
-        ASTER_TRY(forward_step(c, p, precision));
+        if (!drifted) ASTER_TRY(aster_kick_drift_launch(c, p, false, mixed));
+        drifted = can_fuse && s + 1 < nsteps && (s + 1) % K != 0;
+        ASTER_TRY(aster_allpairs_launch(c, p, precision, true, n, nullptr, nullptr, drifted));
     }
     // loss and seeds
     k_adj_seed<<<nb, 256, 0, c->stream>>>(n, c->pm.as<double4>(), a.target.as<double>(), a.lx.as<double4>(),
@@ -396,6 +428,7 @@ extern "C" int aster_adjoint_leapfrog(aster_ctx* c, const aster_params* p, int p
 
     // reverse pass, segment by segment
     const int eg = (int)std::min<int64_t>((n + 255) / 256, (int64_t)c->sm_count * 8);
+    bool pre_done = false;  // the step's lv' and w were formed by the previous reduction
     for (int64_t seg = nseg - 1; seg >= 0; --seg) {
         const int64_t start = seg * K, len = std::min<int64_t>(K, nsteps - start);
         ASTER_TRY(copy_d2d(c, c->pm.ptr, ck_x(seg), v4));
@@ -403,22 +436,28 @@ extern "C" int aster_adjoint_leapfrog(aster_ctx* c, const aster_params* p, int p
         ASTER_TRY(copy_d2d(c, c->acc.ptr, ck_a(seg), v4));
         if (precision == ASTER_MIXED) ASTER_TRY(aster_refresh_mixed(c));
         ASTER_TRY(copy_d2d(c, a.segx.ptr, c->pm.ptr, v4));
-        for (int64_t t = 0; t + 1 < len; ++t) {  // positions x_start .. x_{start+len-1}
-            ASTER_TRY(forward_step(c, p, precision));
+        // positions x_start .. x_{start+len-1}; the last drift needs no force after it
+        for (int64_t t = 0; t + 1 < len; ++t) {
+            if (t == 0 || !can_fuse) ASTER_TRY(aster_kick_drift_launch(c, p, false, mixed));
             ASTER_TRY(copy_d2d(c, a.segx.as<char>() + (size_t)(t + 1) * v4, c->pm.ptr, v4));
+            if (t + 2 < len) ASTER_TRY(aster_allpairs_launch(c, p, precision, true, n, nullptr, nullptr, can_fuse));
         }
         for (int64_t t = len - 1; t >= 0; --t) {
             const int64_t step = start + t;
-            const double scale = (step >= 1 ? 2.0 : 1.0) * h;
-            if (precision == ASTER_MIXED)
-                k_adj_pre<true><<<eg, 256, 0, c->stream>>>(n, a.lx.as<double4>(), a.lv.as<double4>(), a.w.ptr, p->dt,
-                                                           scale);
-            else
-                k_adj_pre<false><<<eg, 256, 0, c->stream>>>(n, a.lx.as<double4>(), a.lv.as<double4>(), a.w.ptr,
-                                                            p->dt, scale);
-            ASTER_CUDA(cudaGetLastError());
+            if (!pre_done) {
+                const double scale = (step >= 1 ? 2.0 : 1.0) * h;
+                if (mixed)
+                    k_adj_pre<true><<<eg, 256, 0, c->stream>>>(n, a.lx.as<double4>(), a.lv.as<double4>(), a.w.ptr,
+                                                               p->dt, scale);
+                else
+                    k_adj_pre<false><<<eg, 256, 0, c->stream>>>(n, a.lx.as<double4>(), a.lv.as<double4>(), a.w.ptr,
+                                                                p->dt, scale);
+                ASTER_CUDA(cudaGetLastError());
+            }
+            AdjNext next{step > 0, mixed, a.lv.as<double4>(), a.w.ptr, p->dt, (step >= 2 ? 2.0 : 1.0) * h};
             ASTER_TRY(adj_pair_launch(c, p, precision, reinterpret_cast<const double4*>(a.segx.as<char>() +
-                                                                                        (size_t)t * v4)));
+                                                                                        (size_t)t * v4), &next));
+            pre_done = next.on;
         }
     }
     cudaEventRecord(c->ev[1], c->stream);

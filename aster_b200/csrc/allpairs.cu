@@ -23,6 +23,8 @@
 // Each thread owns IPT targets; a block of BLOCK threads owns BLOCK*IPT targets
 // and walks one j-slice; small n use several j-slices whose partial sums are
 // added by k_reduce_slices (scratch memory).
+#include <algorithm>
+
 #include "aster_internal.cuh"
 #include "fp64_pair.cuh"
 #include "pn.cuh"
@@ -331,38 +333,52 @@ struct NextDrift {
     float4 *phi, *plo, *vf;
 };
 
-__global__ void k_reduce_slices(int64_t nt, int nslices, const double4* __restrict__ partial,
-                                const int32_t* __restrict__ targets, double G, double4* __restrict__ acc,
-                                double* __restrict__ out3, KickArgs kick, NextDrift next) {
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nt; t += (int64_t)gridDim.x * blockDim.x) {
-        double ax = 0, ay = 0, az = 0;
-#pragma unroll 4
-        for (int s = 0; s < nslices; ++s) {
-            double4 p = partial[(int64_t)s * nt + t];
-            ax += p.x; ay += p.y; az += p.z;
+// One thread per target and component (the fourth writes the padding), so that
+// small systems still spread over the SMs: every operation is per component.
+__global__ void __launch_bounds__(256) k_reduce_slices(int64_t nt, int nslices, const double4* __restrict__ partial,
+                                                       const int32_t* __restrict__ targets, double G,
+                                                       double4* __restrict__ acc, double* __restrict__ out3,
+                                                       KickArgs kick, NextDrift next) {
+    const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, t = id >> 2;
+    const int k = (int)(id & 3);
+    if (t >= nt) return;
+    const int64_t body = targets ? (int64_t)targets[t] : t;
+    double a = 0.0;
+    if (k < 3) {
+        const double* p = reinterpret_cast<const double*>(partial) + id;
+#pragma unroll 8
+        for (int s = 0; s < nslices; ++s) a += p[(int64_t)s * nt * 4];
+        a *= G;
+    }
+    if (out3) {
+        if (k < 3) out3[3 * t + k] = a;
+        return;
+    }
+    reinterpret_cast<double*>(acc + body)[k] = a;
+    if (!kick.on) return;
+    double* vp = reinterpret_cast<double*>(kick.vel + body) + k;
+    double v = 0.0;
+    if (k < 3) {
+        v = *vp;
+        v += a * kick.half_dt;
+    }
+    if (next.pm) {
+        double* xp = reinterpret_cast<double*>(next.pm + body) + k;
+        double x = *xp;
+        if (k < 3) {
+            v += a * kick.half_dt;
+            x += v * next.dt;
+            *xp = x;
         }
-        int64_t body = targets ? (int64_t)targets[t] : t;
-        store_result(t, body, ax, ay, az, G, 1, 0, nt, nullptr, acc, out3, kick);
-        if (next.pm) {
-            const double4 a = acc[body];
-            double4 p = next.pm[body], v = kick.vel[body];
-            v.x += a.x * kick.half_dt; v.y += a.y * kick.half_dt; v.z += a.z * kick.half_dt;
-            p.x += v.x * next.dt; p.y += v.y * next.dt; p.z += v.z * next.dt;
-            next.pm[body] = p;
-            kick.vel[body] = v;
-            if (next.phi) {
-                float4 h, l;
-                ds_split(p.x, h.x, l.x);
-                ds_split(p.y, h.y, l.y);
-                ds_split(p.z, h.z, l.z);
-                h.w = __double2float_rn(p.w);
-                l.w = 0.f;
-                next.phi[body] = h;
-                next.plo[body] = l;
-                next.vf[body] = make_float4((float)v.x, (float)v.y, (float)v.z, 0.f);
-            }
+        if (next.phi) {
+            float h = __double2float_rn(x), l = 0.f;  // the mass, for k = 3
+            if (k < 3) ds_split(x, h, l);
+            reinterpret_cast<float*>(next.phi + body)[k] = h;
+            reinterpret_cast<float*>(next.plo + body)[k] = l;
+            reinterpret_cast<float*>(next.vf + body)[k] = k < 3 ? (float)v : 0.f;
         }
     }
+    if (k < 3) *vp = v;
 }
 
 template <int PNL, bool GUARD>
@@ -409,26 +425,13 @@ struct SliceGrid {
 };
 static SliceGrid slice_grid(const aster_ctx* c, const aster_params* p, int precision, int64_t nt, int64_t len) {
     SliceGrid g;
+    const int pnl = pn_level(p);
     // one target per thread in the mixed post-Newtonian kernel, two elsewhere
-    const int64_t per_block = (int64_t)BLOCK * (precision == ASTER_MIXED && pn_level(p) > 0 ? IPT_PN : IPT);
+    const int64_t per_block = (int64_t)BLOCK * (precision == ASTER_MIXED && pnl > 0 ? IPT_PN : IPT);
     g.iblocks = (nt + per_block - 1) / per_block;
-    // j-slices so that small n still fill the GPU (>= ASTER_SLICE_BLOCKS_PER_SM blocks per SM).
-    int64_t want = ASTER_SLICE_BLOCKS_PER_SM * (int64_t)c->sm_count;
-    int64_t ns = g.iblocks >= want ? 1 : (want + g.iblocks - 1) / g.iblocks;
-    // each slice at least one j-tile; the mixed kernel's at least
-    // ASTER_SLICE_MIN_MIXED sources (its partial-sum reduction outweighs more
-    // parallelism below that)
-    const int64_t min_len = precision == ASTER_MIXED ? ASTER_SLICE_MIN_MIXED : BLOCK;
-    int64_t max_ns = (len + min_len - 1) / min_len;
-    if (ns > max_ns) ns = max_ns;
-    if (ns > 64) ns = 64;
-    if (ns < 1) ns = 1;
-    int64_t slice_len = ((len + ns - 1) / ns + BLOCK - 1) / BLOCK * BLOCK;
-    if (slice_len < BLOCK) slice_len = BLOCK;
-    ns = (len + slice_len - 1) / slice_len;
-    if (ns < 1) ns = 1;  // no sources: one slice that writes zeros
-    g.ns = ns;
-    g.slice_len = slice_len;
+    const int64_t t = aster_slice_tiles(g.iblocks, (len + BLOCK - 1) / BLOCK, c->sm_count);
+    g.slice_len = std::max<int64_t>(t, 1) * BLOCK;
+    g.ns = std::max<int64_t>(1, (len + g.slice_len - 1) / g.slice_len);  // no sources: one slice that writes zeros
     return g;
 }
 
@@ -451,12 +454,18 @@ int aster_allpairs_launch_range(aster_ctx* c, const aster_params* p, int precisi
         if (st != ASTER_ERR_OOM || fuse_next) return st;
     }
     const SliceGrid sg = slice_grid(c, p, precision, nt, len);
-    const int64_t ns = sg.ns, slice_len = sg.slice_len;
+    int64_t ns = sg.ns, slice_len = sg.slice_len;
     if (fuse_next && (ns < 2 || !closing_kick || out_dev || targets_dev)) return ASTER_ERR_UNSUPPORTED;
     double4* partial = nullptr;
     if (ns > 1) {
-        ASTER_TRY(c->scratch.ensure((size_t)ns * nt * sizeof(double4)));
-        partial = c->scratch.as<double4>();
+        const int st = c->scratch.ensure((size_t)ns * nt * sizeof(double4));
+        if (st == ASTER_ERR_OOM && !fuse_next) {  // no room for the partial sums: one slice
+            ns = 1;
+            slice_len = std::max<int64_t>((len + BLOCK - 1) / BLOCK, 1) * BLOCK;
+        } else {
+            ASTER_TRY(st);
+            partial = c->scratch.as<double4>();
+        }
     }
     KickArgs kick{closing_kick && !out_dev, 0.5 * p->dt, c->vel.as<double4>()};
     if (kick.on) c->mixed_valid = false;  // the closing kick moves the velocities
@@ -473,10 +482,9 @@ int aster_allpairs_launch_range(aster_ctx* c, const aster_params* p, int precisi
         const bool mixed = precision == ASTER_MIXED;
         const NextDrift next{fuse_next ? c->pm.as<double4>() : nullptr, p->dt, mixed ? c->phi.as<float4>() : nullptr,
                              mixed ? c->plo.as<float4>() : nullptr, mixed ? c->vf.as<float4>() : nullptr};
-        // few targets: small blocks, so that the reduction's latency spreads over the SMs
-        const int rb = nt < 40000 ? 64 : 256;
-        k_reduce_slices<<<(unsigned)((nt + rb - 1) / rb), rb, 0, c->stream>>>(nt, (int)ns, partial, targets_dev, p->G,
-                                                                             c->acc.as<double4>(), out_dev, kick, next);
+        const int rb = nt < 10000 ? 64 : 256;
+        k_reduce_slices<<<(unsigned)((4 * nt + rb - 1) / rb), rb, 0, c->stream>>>(
+            nt, (int)ns, partial, targets_dev, p->G, c->acc.as<double4>(), out_dev, kick, next);
         ASTER_CUDA(cudaGetLastError());
         c->stats.kernels += 1;
         if (fuse_next && mixed) c->mixed_valid = true;  // refreshed with the drift

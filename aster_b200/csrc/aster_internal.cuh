@@ -21,20 +21,22 @@
 #define ASTER_DEVERR_KEPLER 0x20
 
 // The O(N^2) kernels (all-pairs forces, adjoint pair terms) split the sources
-// into slices when there are too few target blocks to give every SM this many
-// blocks (small N), and add the slices' partial sums afterwards. Measured
-// (same-box A/B, 2 / 4 / 6 / 8 / 12): 12 took the C5 adjoint (N = 16384,
-// 1000 steps) from 1021 to 744 ms mixed and 2057 to 1400 ms FP64, and the C1
-// FP64 step (N = 4096) from 0.048 to 0.040 ms. The mixed all-pairs kernel
-// keeps at least ASTER_SLICE_MIN_MIXED sources per slice: with 128 the C1
-// mixed step slowed from 0.0255 to 0.0274 ms, the reduction of 32 partial
-// sums per body outweighing the parallelism.
-#ifndef ASTER_SLICE_BLOCKS_PER_SM
-#define ASTER_SLICE_BLOCKS_PER_SM 12
-#endif
-#ifndef ASTER_SLICE_MIN_MIXED
-#define ASTER_SLICE_MIN_MIXED 256
-#endif
+// into slices, and add the slices' partial sums afterwards: 32 slices (64 where
+// that is needed for 12 blocks an SM), so that the SMs' shares of the blocks
+// come out even and the last blocks are short. Mixed forces, us, with the slices
+// that give 12 blocks an SM and with 32: 16,384 bodies 182 / 176, 65,536 2686 /
+// 2490, 100,003 6166 / 5718, 262,144 40,350 / 39,100; 1PN at 30,000 1382 / 1334.
+// From ASTER_SLICE_MAX_BLOCKS target blocks on (614,400 bodies) one slice: the
+// blocks alone are 16 an SM, and the partial sums would take a gigabyte. Returns
+// the tiles (128 sources) of a slice.
+constexpr int64_t ASTER_SLICE_MAX_BLOCKS = 2400;
+inline int64_t aster_slice_tiles(int64_t iblocks, int64_t tiles, int64_t sms) {
+    if (tiles < 1) return 1;
+    if (iblocks >= ASTER_SLICE_MAX_BLOCKS) return tiles;
+    int64_t ns = (12 * sms + iblocks - 1) / iblocks;
+    ns = ns < 32 ? 32 : ns > 64 ? 64 : ns;
+    return (tiles + ns - 1) / ns;
+}
 
 #define ASTER_TRY(...)                                    \
     do {                                                  \
