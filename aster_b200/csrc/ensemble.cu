@@ -31,14 +31,15 @@
 // entire run; per force evaluation every lane publishes its bodies to the
 // warp's shared-memory slab and sums over the slab. Systems are taken largest
 // first from a global work counter (longest-processing-time order), so the
-// uneven sizes balance across warps. The kernel polls a host-written cancel
-// flag every check_every steps; it never waits on anything.
+// uneven sizes balance across warps. The kernel polls a cancel flag every
+// check_every steps; it never waits on anything.
 #include <algorithm>
 #include <cmath>
 #include <numeric>
 #include <vector>
 
 #include "aster_internal.cuh"
+#include "fp64_pair.cuh"
 #include "pn.cuh"
 
 namespace {
@@ -263,7 +264,8 @@ __device__ __forceinline__ void accel_f64(const EnsSlab<false>& s, int n, int j0
         const double4 xj = s.x[j];
         const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
         const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-        double inv = r2 > 0.0 ? rsqrt(r2) : 0.0;
+        // (the series step's registers cost the longer PN bodies more than it saves: 1PN unrolled 4, 7.4 -> 8.0 ms)
+        const double inv = PNL == 0 ? inv_r_or_0(r2) : r2 > 0.0 ? rsqrt(r2) : 0.0;
         const double inv2 = inv * inv;
         const double sN = xj.w * inv * inv2;
         ax = fma(dx, sN, ax); ay = fma(dy, sN, ay); az = fma(dz, sN, az);
@@ -495,11 +497,36 @@ __device__ __forceinline__ void eih_accel(const EnsSlab<MIXED>& slab, typename E
     }
 }
 
+// The launch's counters in device memory, zero before it.
+struct EnsWork {
+    unsigned int next;             // the next system to take
+    int cancelled;                 // the host's flag was seen
+    unsigned long long polled_ns;  // when it was last read
+};
+
+// Whether the run is cancelled. The host writes its flag to mapped memory, and
+// reads of that go over PCIe one after another, 0.9 us each: with every warp
+// reading it for every system (and every check_every steps), 16,384 systems took
+// 14.8 ms for any number of steps whose arithmetic was shorter (40 Newtonian
+// steps: 14.8 -> 2.6 ms, 40 1PN steps 14.9 -> 5.8). Now one warp reads it for all
+// once in CANCEL_POLL_NS and passes it on in device memory.
+constexpr unsigned long long CANCEL_POLL_NS = 20000;
+__device__ __forceinline__ int poll_cancel(EnsWork* w, const volatile int* host_flag) {
+    if (*(volatile int*)&w->cancelled) return 1;
+    unsigned long long now;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+    const unsigned long long last = *(volatile unsigned long long*)&w->polled_ns;
+    if (now - last < CANCEL_POLL_NS || atomicCAS(&w->polled_ns, last, now) != last) return 0;
+    if (!*host_flag) return 0;
+    *(volatile int*)&w->cancelled = 1;
+    return 1;
+}
+
 template <bool MIXED, int PNL, int UNROLL, int NST>
 __global__ void k_ensemble(int32_t nsys, const int32_t* __restrict__ order, const int32_t* __restrict__ off,
                            double4* __restrict__ pm, double4* __restrict__ vel, double G, double eps2, PnK<double> pk,
-                           Coeffs k, int64_t nsteps, int check_every, unsigned int* __restrict__ work,
-                           const volatile int* __restrict__ cancel, int* __restrict__ err) {
+                           Coeffs k, int64_t nsteps, int check_every, EnsWork* work, const volatile int* cancel,
+                           int* __restrict__ err) {
     extern __shared__ __align__(16) unsigned char ens_smem[];
     EnsSlab<MIXED>& slab = reinterpret_cast<EnsSlab<MIXED>*>(ens_smem)[threadIdx.x >> 5];
     // level 3 only: 64 (A, Phi) records per warp after all the block's slabs
@@ -511,7 +538,7 @@ __global__ void k_ensemble(int32_t nsys, const int32_t* __restrict__ order, cons
     const PnK<float> pkf = pn_float(pk);
     for (;;) {
         unsigned int w = 0;
-        if (lane == 0) w = atomicAdd(work, 1u);
+        if (lane == 0) w = atomicAdd(&work->next, 1u);
         w = __shfl_sync(0xffffffffu, w, 0);
         if (w >= (unsigned)nsys) break;
         const int sys = order ? order[w] : (int)w;  // no order: upload order
@@ -534,7 +561,7 @@ __global__ void k_ensemble(int32_t nsys, const int32_t* __restrict__ order, cons
         for (int64_t step = 0; step < nsteps; ++step) {
             if (step % check_every == 0) {
                 int cflag = 0;
-                if (lane == 0) cflag = *cancel;
+                if (lane == 0) cflag = poll_cancel(work, cancel);
                 cflag = __shfl_sync(0xffffffffu, cflag, 0);
                 if (cflag) {
                     if (lane == 0) atomicOr(err, ASTER_DEVERR_CANCEL);
@@ -700,9 +727,9 @@ int launch_ensemble(aster_ctx* c, const aster_params* p, const Coeffs& k, int64_
     const int64_t need = (e.nsys + wpb - 1) / wpb;
     if (blocks > need) blocks = need;
     const PnK<double> pk = make_pn(p);
-    unsigned int* work = e.counter.as<unsigned int>();
+    EnsWork* work = e.counter.as<EnsWork>();
     auto enqueue = [&](cudaStream_t s) -> int {
-        ASTER_CUDA(cudaMemsetAsync(work, 0, sizeof(unsigned int), s));
+        ASTER_CUDA(cudaMemsetAsync(work, 0, sizeof(EnsWork), s));
         kern<<<(unsigned)blocks, wpb * 32, smem, s>>>(e.nsys, lpt ? e.order.as<int32_t>() : nullptr, e.off.as<int32_t>(),
                                                      e.pm.as<double4>(), e.vel.as<double4>(), p->G, p->eps2, pk, k,
                                                      nsteps, check_every, work, e.cancel_dev, c->err_dev);
@@ -844,7 +871,9 @@ extern "C" int aster_ensemble_run(aster_ctx* c, const aster_params* p, int integ
     if (integrator != ASTER_INTEGRATOR_LEAPFROG && integrator != ASTER_INTEGRATOR_YOSHIDA4) return ASTER_ERR_INVALID_ARG;
     if (precision != ASTER_FP64 && precision != ASTER_MIXED) return ASTER_ERR_INVALID_ARG;
     int wpb = cfg && cfg->warps_per_block ? cfg->warps_per_block : 4;
-    int unroll = cfg && cfg->unroll ? cfg->unroll : 2;
+    // the flagged PN terms' and EIH's loop bodies are long: 16,384 systems, 40 mixed steps, unroll 1 / 2 / 4:
+    // every PN term 14.6 / 17.2 / 22.4 ms, EIH 8.7 / 9.9 / 11.5; 1PN 5.84 / 5.83 / 6.33, Newton 2.83 / 2.59 / 2.61
+    int unroll = cfg && cfg->unroll ? cfg->unroll : pnl >= 2 ? 1 : 2;
     int check = cfg && cfg->check_every ? cfg->check_every : 256;
     // stream capture is not possible on the legacy default stream
     bool graph = (cfg ? cfg->use_graph != 0 : true) && c->stream != nullptr;

@@ -53,6 +53,14 @@ __device__ __forceinline__ double inv_r(double x) {
     return y;
 }
 
+// inv_r where x = 0 is common (a body among its own sources): no branch for it
+__device__ __forceinline__ double inv_r_or_0(double x) {
+    const bool zero = (__double2hiint(x) | __double2loint(x)) == 0;
+    double y = inv_r_fast(x);
+    if (!r2_ordinary(x) && !zero) y = inv_r_any(x);
+    return zero ? 0.0 : y;
+}
+
 // m x^(-3/2), 0 for x = 0; the mass first where r^-3 alone may leave the range
 __device__ __forceinline__ double m_inv_r3(double m, double x) {
     double s = m * inv_r3_fast(x);
