@@ -156,7 +156,7 @@ struct aster_ctx {
     // executable graphs of the last call's repeated steps; destroyed by the
     // next call's aster_begin (its work has finished by then) or at destroy
     std::vector<std::pair<cudaGraph_t, cudaGraphExec_t>> graphs;
-    // the tree KDK's middle step (kick-fused build + walk), kept across calls;
+    // the KDK's middle step (forces with the next kick and drift), kept across calls;
     // a replaced one moves to `graphs`
     StepGraph kdk_graph;
 };

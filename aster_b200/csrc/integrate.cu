@@ -340,20 +340,22 @@ static int no_replay(cudaGraph_t, cudaGraphExec_t) { return ASTER_OK; }
 
 // The key of a cached step graph: everything the captured launches depend on
 // besides the data in device memory (parameters, solver, precision, body
-// count, the addresses of the context's buffers through their generation,
-// whether the step carries timing marks).
+// count, the sources among them and whether partial sums found room (which
+// choose the all-pairs kernel and its grid), the addresses of the context's
+// buffers through their generation, whether the step carries timing marks).
 static std::vector<unsigned char> step_key(const aster_ctx* c, const aster_params* p, int solver, int precision,
                                            bool timed) {
     std::vector<unsigned char> k(sizeof(aster_params));
     std::memcpy(k.data(), p, sizeof(aster_params));
-    const int64_t w[] = {solver, precision, timed ? 1 : 0, c->n, c->device, c->walk_stack_limit,
-                         (int64_t)aster_devbuf_epoch()};
+    const int64_t w[] = {solver, precision, timed ? 1 : 0, c->n, c->n_src, c->sym_oom_n, c->device,
+                         c->walk_stack_limit, (int64_t)aster_devbuf_epoch()};
     const unsigned char* wb = reinterpret_cast<const unsigned char*>(w);
     k.insert(k.end(), wb, wb + sizeof(w));
     return k;
 }
 
-// Launches `count` more of the tree KDK's middle step from the context's
+// Launches `count` more of a KDK run's middle step (its force evaluation ends
+// in the next step's kick and drift) from the context's
 // cached graph, capturing it first (one step, `middle`) when the cached one
 // does not match this call. The cached graph survives the call, so a later
 // call with the same key captures and instantiates nothing: its steps are

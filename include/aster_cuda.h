@@ -174,8 +174,8 @@ int aster_lbvh_forces(aster_ctx* ctx, const aster_params* p, int precision,
 /* nsteps kick-drift-kick leapfrog steps of the resident state with one force
  * evaluation per step (the acceleration is cached across steps; the reference
  * update_leapfrog evaluates twice per step). solver: ASTER_SOLVER_*. With
- * the tree solver, the steps between the first and the last run as launches
- * of one CUDA graph that the context keeps until it is destroyed: a later call
+ * the tree solver, and with all-pairs where the sums are made in parts, the
+ * steps between the first and the last run as launches of one CUDA graph that the context keeps until it is destroyed: a later call
  * with the same parameters, body count and device buffers launches it again
  * instead of capturing a new one. */
 int aster_kdk_steps(aster_ctx* ctx, const aster_params* p, int solver, int precision,
@@ -343,8 +343,8 @@ int aster_adjoint_leapfrog(aster_ctx* ctx, const aster_params* p, int precision,
  * make that first call before any stream capture. The address is kept for the
  * life of the process: calling cudaDeviceReset after the first call on that
  * device is not supported (the module is reloaded elsewhere and the kept
- * address goes stale). Every block adds up 256 bodies against all sources in
- * one launch, so below about 40,000 bodies the GPU is only partly filled and
+ * address goes stale). Every block adds up 256 bodies against all bodies after
+ * them in one launch, so below about 40,000 bodies the GPU is only partly filled and
  * this call is several times slower than aster_energy, which also splits the
  * sources over blocks. All calls share the one
  * array: calls that overlap on the GPU (on different streams) race and give
