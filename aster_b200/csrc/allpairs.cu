@@ -501,12 +501,14 @@ int aster_allpairs_launch(aster_ctx* c, const aster_params* p, int precision, bo
 
 // Whether an evaluation of all bodies ends in a kernel that adds partial sums,
 // where the next step's opening kick and drift can follow (no other block then
-// reads positions any more). Allocates the symmetric path's partials.
+// reads positions any more). Allocates the partial sums; where there is no room
+// for them the evaluation runs in one slice, and nothing can follow.
 bool aster_allpairs_can_fuse(aster_ctx* c, const aster_params* p, int precision) {
     if (precision == ASTER_FP64 && aster_allpairs_sym_fits(c, p))
         if (aster_allpairs_sym_prepare(c, p) == ASTER_OK) return true;
     const int64_t n_src = c->n_src > 0 ? c->n_src : c->n;
-    return slice_grid(c, p, precision, c->n, n_src).ns > 1;
+    const int64_t ns = slice_grid(c, p, precision, c->n, n_src).ns;
+    return ns > 1 && c->scratch.ensure((size_t)ns * c->n * sizeof(double4)) == ASTER_OK;
 }
 
 extern "C" int aster_allpairs(aster_ctx* c, const aster_params* p, int precision, double* acc_out) {

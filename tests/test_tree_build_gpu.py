@@ -24,8 +24,10 @@ def _same(ctx, orc, pos, m, bits=30):
         np.testing.assert_array_equal(t[a], o[b], err_msg=a)
 
 
-# one block, two, the last merge alone (up to 13k bodies), one middle merge, two middle merges (above 450k)
-@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 128, 129, 4095, 12500, 14500, 100001, 470001])
+# sort: a cluster's block of 1024 bodies, its 16 blocks with one and with two bodies a thread, the sort of many launches;
+# tree: one block, two, the last merge alone (up to 13k bodies), one middle merge, two middle merges (above 450k)
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 128, 129, 1024, 1025, 4095, 12500, 14500, 16384, 16385, 32768,
+                               32769, 100001, 470001])
 @pytest.mark.parametrize("bits", [30, 63])
 def test_tree_bit_exact(ctx, orc, n, bits):
     pos, _, m = gen.plummer(n, 40 + n, masses="lognormal")
