@@ -1252,6 +1252,53 @@ __device__ __forceinline__ float max3_f32(float a, float b, float c) {
     return d;
 }
 
+// Pairs q0i, q0i + step, ... < np of a list with velocities acting on one body,
+// two entries per paired FP32 instruction: the Newtonian sum into sx, sy, sz,
+// the 1PN sum into p and the 2PN + 2.5PN sum into qq. PNL = 1: Newton + 1PN;
+// 2: the terms that pk.f selects.
+template <int PNL, bool GUARD>
+__device__ __forceinline__ void pn_list(const float4* LA, const float4* LB, const float4* LVA, const float4* LVB,
+                                        int np, int q0i, int step, const float2 nbx, const float2 nby,
+                                        const float2 nbz, const float4 vf, float mi, const float2 e2, double G,
+                                        const PnK<double>& pk, CompSum& sx, CompSum& sy, CompSum& sz, float3& p,
+                                        float3& qq) {
+    const float Gf = (float)G, mc2 = -(float)pk.c2;
+    const float2 G4 = make_float2(4.f * Gf, 4.f * Gf);
+    const float2 vix = make_float2(vf.x, vf.x), viy = make_float2(vf.y, vf.y), viz = make_float2(vf.z, vf.z),
+                 nvi2 = make_float2(-vf.w, -vf.w), vi4x = make_float2(4.f * vf.x, 4.f * vf.x),
+                 vi4y = make_float2(4.f * vf.y, 4.f * vf.y), vi4z = make_float2(4.f * vf.z, 4.f * vf.z),
+                 mi5G = make_float2(5.f * Gf * mi, 5.f * Gf * mi);
+    float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax, px = ax, py = ax, pz = ax;
+    if constexpr (PNL == 1) {
+#pragma unroll 2
+        for (int q = q0i; q < np; q += step)
+            interact2_pn1_f32<GUARD>(LA[q], LB[q], LVA[q], LVB[q], nbx, nby, nbz, vix, viy, viz, vi4x, vi4y, vi4z,
+                                     nvi2, mi5G, e2, G4, ax, ay, az, px, py, pz);
+    } else {
+        const float mc4 = -(float)pk.c4, nkf = -0.8f * (float)pk.ic;
+        const float2 G2 = make_float2(Gf, Gf), nk = make_float2(nkf, nkf), vi2 = make_float2(vf.w, vf.w),
+                     Gmi = make_float2(Gf * mi, Gf * mi);
+        float2 qx = make_float2(0.f, 0.f), qy = qx, qz = qx;
+        for (int q = q0i; q < np; q += step) {
+            const float4 A = LA[q], B = LB[q], VA = LVA[q], VB = LVB[q];
+            const float2 dx = __fadd2_rn(make_float2(A.x, A.y), nbx);  // entry - body
+            const float2 dy = __fadd2_rn(make_float2(A.z, A.w), nby);
+            const float2 dz = __fadd2_rn(make_float2(B.x, B.y), nbz);
+            newton_pn_all_x2<GUARD>(dx, dy, dz, make_float2(B.z, B.w), make_float2(VA.x, VA.y),
+                                    make_float2(VA.z, VA.w), make_float2(VB.x, VB.y), make_float2(VB.z, VB.w), vix,
+                                    viy, viz, vi4x, vi4y, vi4z, nvi2, vi2, mi5G, Gmi, e2, G4, G2, nk, pk.f, ax, ay,
+                                    az, px, py, pz, qx, qy, qz);
+        }
+        qq.x = fmaf(mc4, qx.x + qx.y, qq.x);
+        qq.y = fmaf(mc4, qy.x + qy.y, qq.y);
+        qq.z = fmaf(mc4, qz.x + qz.y, qq.z);
+    }
+    sx.add(ax.x + ax.y); sy.add(ay.x + ay.y); sz.add(az.x + az.y);
+    p.x = fmaf(mc2, px.x + px.y, p.x);
+    p.y = fmaf(mc2, py.x + py.y, p.y);
+    p.z = fmaf(mc2, pz.x + pz.y, p.z);
+}
+
 // Opening test of both children of a node for the whole group, FP32
 // round-to-nearest without FMA (the CPU restatement reproduces it bit for
 // bit), the two children in the halves of paired FP32 operations: the squared
@@ -1406,74 +1453,15 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, PNL ? 4 : ASTER_WALK_MINBLOCK
             }
         };
 
-        auto evaluate = [&](int cnt) {
+        auto evaluate = [&](int cnt) __attribute__((always_inline)) {
             if constexpr (PNL > 0) {
-                if constexpr (MIXED && PNL == 1) {  // Newton + 1PN only: two entries per paired instruction
-                    // an odd cnt has its last slot half zero-padded by the caller
-                    const int np = (cnt + 1) >> 1;
-                    const float Gf = (float)G, mc2 = -(float)pk.c2;
-                    const float2 G4 = make_float2(4.f * Gf, 4.f * Gf);
-                    auto body = [&](const float2 nbx, const float2 nby, const float2 nbz, const float4 vf, float mi,
-                                    int q0i, int step, CompSum& sx, CompSum& sy, CompSum& sz, float3& p) {
-                        const float2 vix = make_float2(vf.x, vf.x), viy = make_float2(vf.y, vf.y),
-                                     viz = make_float2(vf.z, vf.z), nvi2 = make_float2(-vf.w, -vf.w),
-                                     vi4x = make_float2(4.f * vf.x, 4.f * vf.x),
-                                     vi4y = make_float2(4.f * vf.y, 4.f * vf.y),
-                                     vi4z = make_float2(4.f * vf.z, 4.f * vf.z),
-                                     mi5G = make_float2(5.f * Gf * mi, 5.f * Gf * mi);
-                        float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax, px = ax, py = ax, pz = ax;
-#pragma unroll 2
-                        for (int q = q0i; q < np; q += step)
-                            interact2_pn1_f32<GUARD>(sm.lpa[warp][q], sm.lpb[warp][q], sm.lva[warp][q],
-                                                     sm.lvb[warp][q], nbx, nby, nbz, vix, viy, viz, vi4x, vi4y,
-                                                     vi4z, nvi2, mi5G, eps2f2, G4, ax, ay, az, px, py, pz);
-                        sx.add(ax.x + ax.y); sy.add(ay.x + ay.y); sz.add(az.x + az.y);
-                        p.x = fmaf(mc2, px.x + px.y, p.x);
-                        p.y = fmaf(mc2, py.x + py.y, p.y);
-                        p.z = fmaf(mc2, pz.x + pz.y, p.z);
-                    };
-                    body(nb0x, nb0y, nb0z, vf0, h0.w, 0, 1, sx0, sy0, sz0, p0);
-                    if (two) body(nb1x, nb1y, nb1z, vf1, h1.w, sub, lps, sx1, sy1, sz1, p1);
-                } else if (MIXED) {  // any of the PN terms by flags: two entries per paired instruction as well
+                if constexpr (MIXED) {
                     const int np = (cnt + 1) >> 1;  // an odd cnt: last slot half zero-padded by the caller
-                    const float Gf = (float)G, mc2 = -(float)pk.c2, mc4 = -(float)pk.c4;
-                    const float2 G4 = make_float2(4.f * Gf, 4.f * Gf), G2 = make_float2(Gf, Gf);
-                    const float nkf = -0.8f * (float)pk.ic;
-                    const float2 nk = make_float2(nkf, nkf);
-                    auto body = [&](const float2 nbx, const float2 nby, const float2 nbz, const float4 vf, float mi,
-                                    int q0i, int step, CompSum& sx, CompSum& sy, CompSum& sz, float3& p, float3& qq) {
-                        const float2 vix = make_float2(vf.x, vf.x), viy = make_float2(vf.y, vf.y),
-                                     viz = make_float2(vf.z, vf.z), nvi2 = make_float2(-vf.w, -vf.w),
-                                     vi2 = make_float2(vf.w, vf.w),
-                                     vi4x = make_float2(4.f * vf.x, 4.f * vf.x),
-                                     vi4y = make_float2(4.f * vf.y, 4.f * vf.y),
-                                     vi4z = make_float2(4.f * vf.z, 4.f * vf.z),
-                                     mi5G = make_float2(5.f * Gf * mi, 5.f * Gf * mi),
-                                     Gmi = make_float2(Gf * mi, Gf * mi);
-                        float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax, px = ax, py = ax, pz = ax, qx = ax,
-                               qy = ax, qz = ax;
-                        for (int q = q0i; q < np; q += step) {
-                            const float4 A = sm.lpa[warp][q], B = sm.lpb[warp][q], VA = sm.lva[warp][q],
-                                         VB = sm.lvb[warp][q];
-                            const float2 dx = __fadd2_rn(make_float2(A.x, A.y), nbx);  // entry - body
-                            const float2 dy = __fadd2_rn(make_float2(A.z, A.w), nby);
-                            const float2 dz = __fadd2_rn(make_float2(B.x, B.y), nbz);
-                            newton_pn_all_x2<GUARD>(dx, dy, dz, make_float2(B.z, B.w), make_float2(VA.x, VA.y),
-                                                    make_float2(VA.z, VA.w), make_float2(VB.x, VB.y),
-                                                    make_float2(VB.z, VB.w), vix, viy, viz, vi4x, vi4y, vi4z, nvi2,
-                                                    vi2, mi5G, Gmi, eps2f2, G4, G2, nk, pk.f, ax, ay, az, px, py, pz,
-                                                    qx, qy, qz);
-                        }
-                        sx.add(ax.x + ax.y); sy.add(ay.x + ay.y); sz.add(az.x + az.y);
-                        p.x = fmaf(mc2, px.x + px.y, p.x);
-                        p.y = fmaf(mc2, py.x + py.y, p.y);
-                        p.z = fmaf(mc2, pz.x + pz.y, p.z);
-                        qq.x = fmaf(mc4, qx.x + qx.y, qq.x);
-                        qq.y = fmaf(mc4, qy.x + qy.y, qq.y);
-                        qq.z = fmaf(mc4, qz.x + qz.y, qq.z);
-                    };
-                    body(nb0x, nb0y, nb0z, vf0, h0.w, 0, 1, sx0, sy0, sz0, p0, q0);
-                    if (two) body(nb1x, nb1y, nb1z, vf1, h1.w, sub, lps, sx1, sy1, sz1, p1, q1);
+                    pn_list<PNL, GUARD>(sm.lpa[warp], sm.lpb[warp], sm.lva[warp], sm.lvb[warp], np, 0, 1, nb0x, nb0y,
+                                        nb0z, vf0, h0.w, eps2f2, G, pk, sx0, sy0, sz0, p0, q0);
+                    if (two)
+                        pn_list<PNL, GUARD>(sm.lpa[warp], sm.lpb[warp], sm.lva[warp], sm.lvb[warp], np, sub, lps, nb1x,
+                                            nb1y, nb1z, vf1, h1.w, eps2f2, G, pk, sx1, sy1, sz1, p1, q1);
                 } else {
                     for (int e = 0; e < cnt; ++e)
                         interact_pn_f64<PNL>(sm.lcm[warp][e], sm.lvd[warp][e], c0, vd0, eps2, G, pk, dx0, dy0,
@@ -1738,45 +1726,51 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, PNL ? 4 : ASTER_WALK_MINBLOCK
 // in which the chunks' sums are added differs (compensated FP32 per warp, FP64
 // over the warps). FP64: the list holds node ids, and each evaluating warp
 // gathers the nodes of its chunk 32 at a time, so that the traversal does not
-// wait for them. Bound by the traversal's ~85 dependent rounds a group (mixed)
+// wait for them; post-Newtonian velocities come the same way in both
+// precisions. Bound by the traversal's ~85 dependent rounds a group (mixed)
 // or by the FP64 pipe (FP64); chunk, warps and resident teams are the best of
 // 64 / 96 / 128 entries, 3 to 8 warps and 2 to 6 teams per SM at 1000 to
 // 262,144 bodies (fewer teams leave FP64 the registers it would spill).
-template <bool MIXED>
+template <bool MIXED, int PNL = 0>
 struct TeamSize {
     static constexpr int WARPS = MIXED ? 4 : 5;
-    static constexpr int CHUNK = MIXED ? WALK_FLUSH_MIXED : 64;
+    static constexpr int PER_SM = MIXED ? (PNL ? 4 : 5) : 3;
+    static constexpr int CHUNK = MIXED && PNL == 0 ? WALK_FLUSH_MIXED : 64;
     static constexpr int BATCH = (WARPS - 1) * CHUNK;
     static constexpr int LIST = BATCH + 64;  // a round appends up to 64 entries
     static_assert(CHUNK >= 64 && CHUNK % 32 == 0, "the rest of a list is at most WARPS chunks");
 };
 
-template <bool MIXED>
+template <bool MIXED, int PNL>
 struct TeamShared {
+    using Size = TeamSize<MIXED, PNL>;
     int stack[WALK_STACK];
-    float4 lpa[2][MIXED ? TeamSize<MIXED>::LIST / 2 : 1];  // as WalkShared::lpa, lpb
-    float4 lpb[2][MIXED ? TeamSize<MIXED>::LIST / 2 : 1];
-    int lid[2][MIXED ? 1 : TeamSize<MIXED>::LIST];                // node ids
-    double4 lcm[TeamSize<MIXED>::WARPS][MIXED ? 1 : 32];          // the entries a warp evaluates
-    double sum[TeamSize<MIXED>::WARPS][6][32];
+    float4 lpa[2][MIXED ? Size::LIST / 2 : 1];  // as WalkShared::lpa, lpb
+    float4 lpb[2][MIXED ? Size::LIST / 2 : 1];
+    int lid[2][MIXED && PNL == 0 ? 1 : Size::LIST];  // node ids
+    double4 lcm[Size::WARPS][MIXED ? 1 : 32];        // the entries a warp evaluates
+    double4 lvd[Size::WARPS][!MIXED && PNL ? 32 : 1];  // and their velocities
+    float4 lva[Size::WARPS][MIXED && PNL ? Size::CHUNK / 2 : 1];  // mixed: paired as in WalkSharedPn
+    float4 lvb[Size::WARPS][MIXED && PNL ? Size::CHUNK / 2 : 1];
+    double sum[Size::WARPS][6][32];
     int cnt[2];    // entries in each buffer
     int state[2];  // of each buffer: 0 more to come, 1 last batch, 2 stack overflow
     unsigned int next;
 };
 
-template <bool MIXED, bool GUARD, bool KICK>
-__global__ void __launch_bounds__(TeamSize<MIXED>::WARPS * 32, MIXED ? 5 : 3) k_walk_team(
+template <bool MIXED, bool GUARD, bool KICK, int PNL>
+__global__ void __launch_bounds__(TeamSize<MIXED, PNL>::WARPS * 32, TeamSize<MIXED, PNL>::PER_SM) k_walk_team(
     int64_t n, const int2* __restrict__ groups, const unsigned int* __restrict__ ngroups_p,
     unsigned int* __restrict__ work, const float4* __restrict__ crec, const double4* __restrict__ node_cm,
     const int2* __restrict__ child, const int32_t* __restrict__ perm, double G, double eps2, double half_dt,
     double4* __restrict__ acc, double4* __restrict__ vel, int* __restrict__ err, int* __restrict__ stack_hw,
     int stack_limit, int32_t* __restrict__ body_counts, unsigned long long* __restrict__ inter_count,
-    double4* __restrict__ pm_next, double dt_next, unsigned long long* __restrict__ box_next,
-    const float4* __restrict__ bmin, const float4* __restrict__ bmax) {
-    __shared__ TeamShared<MIXED> sm;
-    constexpr int TEAM_WARPS = TeamSize<MIXED>::WARPS, TEAM_CHUNK = TeamSize<MIXED>::CHUNK,
-                  TEAM_BATCH = TeamSize<MIXED>::BATCH;
-    const bool plain = !MIXED && walk_r2_ordinary(n, bmin, bmax, eps2);
+    const double4* __restrict__ node_v, PnK<double> pk, double4* __restrict__ pm_next, double dt_next,
+    unsigned long long* __restrict__ box_next, const float4* __restrict__ bmin, const float4* __restrict__ bmax) {
+    __shared__ TeamShared<MIXED, PNL> sm;
+    using Size = TeamSize<MIXED, PNL>;
+    constexpr int TEAM_WARPS = Size::WARPS, TEAM_CHUNK = Size::CHUNK, TEAM_BATCH = Size::BATCH;
+    const bool plain = !MIXED && PNL == 0 && walk_r2_ordinary(n, bmin, bmax, eps2);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
     const unsigned int nbig = ngroups_p[0], ngroups = nbig + ngroups_p[3];
@@ -1815,9 +1809,22 @@ __global__ void __launch_bounds__(TeamSize<MIXED>::WARPS * 32, MIXED ? 5 : 3) k_
         const float3 b1 = make_float3((h1.x - cgx) + l1.x, (h1.y - cgy) + l1.y, (h1.z - cgz) + l1.z);
         CompSum sx0, sy0, sz0, sx1, sy1, sz1;
         double dx0 = 0, dy0 = 0, dz0 = 0, dx1 = 0, dy1 = 0, dz1 = 0;
+        // the bodies' velocities and the 1PN (p) and 2PN + 2.5PN (q) sums, as in k_walk
+        float4 vf0 = make_float4(0.f, 0.f, 0.f, 0.f), vf1 = vf0;
+        double4 vd0 = make_double4(0, 0, 0, 0), vd1 = vd0;
+        float3 p0 = make_float3(0.f, 0.f, 0.f), q0 = p0, p1 = p0, q1 = p0;
+        if constexpr (PNL > 0) {
+            if (MIXED) {
+                vf0 = vel_f4(node_v[k0]);
+                vf1 = two ? vel_f4(node_v[k1]) : vf0;
+            } else {
+                vd0 = vel_d4(node_v[k0]);
+                vd1 = two ? vel_d4(node_v[k1]) : vd0;
+            }
+        }
 
         // one chunk: cnt entries from entry `from` of buffer b
-        auto evaluate = [&](int b, int from, int cnt) {
+        auto evaluate = [&](int b, int from, int cnt) __attribute__((always_inline)) {
             if constexpr (MIXED) {
                 const float4* A = sm.lpa[b] + from / 2;
                 const float4* B = sm.lpb[b] + from / 2;
@@ -1827,6 +1834,28 @@ __global__ void __launch_bounds__(TeamSize<MIXED>::WARPS * 32, MIXED ? 5 : 3) k_
                 const float2 nb1x = make_float2(-b1.x, -b1.x), nb1y = make_float2(-b1.y, -b1.y),
                              nb1z = make_float2(-b1.z, -b1.z);
                 const int np = (cnt + 1) >> 1;  // an odd list has its last half slot zeroed
+                if constexpr (PNL > 0) {  // the warp fetches its chunk's velocities, the traversal only lists the nodes
+                    const int* id = sm.lid[b] + from;
+                    float* VA = reinterpret_cast<float*>(sm.lva[warp]);
+                    float* VB = reinterpret_cast<float*>(sm.lvb[warp]);
+                    __syncwarp();
+#pragma unroll
+                    for (int e = lane; e < TEAM_CHUNK; e += 32) {
+                        const float4 v = vel_f4(e < cnt ? node_v[id[e]] : make_double4(0, 0, 0, 0));
+                        const int o = ((e >> 1) << 2) | (e & 1);
+                        VA[o] = v.x;
+                        VA[o + 2] = v.y;
+                        VB[o] = v.z;
+                        VB[o + 2] = v.w;
+                    }
+                    __syncwarp();
+                    pn_list<PNL, GUARD>(A, B, sm.lva[warp], sm.lvb[warp], np, 0, 1, nb0x, nb0y, nb0z, vf0, h0.w, e2, G,
+                                        pk, sx0, sy0, sz0, p0, q0);
+                    if (two)
+                        pn_list<PNL, GUARD>(A, B, sm.lva[warp], sm.lvb[warp], np, sub, lps, nb1x, nb1y, nb1z, vf1,
+                                            h1.w, e2, G, pk, sx1, sy1, sz1, p1, q1);
+                    return;
+                }
                 float2 ax0 = make_float2(0.f, 0.f), ay0 = ax0, az0 = ax0, ax1 = ax0, ay1 = ax0, az1 = ax0;
                 if (two && lps == 1) {
 #pragma unroll 4
@@ -1849,6 +1878,24 @@ __global__ void __launch_bounds__(TeamSize<MIXED>::WARPS * 32, MIXED ? 5 : 3) k_
             } else {
                 const int* id = sm.lid[b] + from;
                 double4* st = sm.lcm[warp];
+                if constexpr (PNL > 0) {
+                    double4* sv = sm.lvd[warp];
+                    for (int e0 = 0; e0 < cnt; e0 += 32) {
+                        __syncwarp();
+                        if (e0 + lane < cnt) {
+                            st[lane] = node_cm[id[e0 + lane]];
+                            sv[lane] = vel_d4(node_v[id[e0 + lane]]);
+                        }
+                        __syncwarp();
+                        const int m = cnt - e0 < 32 ? cnt - e0 : 32;
+                        for (int e = 0; e < m; ++e)
+                            interact_pn_f64<PNL>(st[e], sv[e], c0, vd0, eps2, G, pk, dx0, dy0, dz0);
+                        if (two)
+                            for (int e = sub; e < m; e += lps)
+                                interact_pn_f64<PNL>(st[e], sv[e], c1, vd1, eps2, G, pk, dx1, dy1, dz1);
+                    }
+                    return;
+                }
                 double4 nx = lane < cnt ? node_cm[id[lane]] : make_double4(0, 0, 0, 0);
                 for (int e0 = 0; e0 < cnt; e0 += 32) {
                     __syncwarp();
@@ -1884,7 +1931,7 @@ __global__ void __launch_bounds__(TeamSize<MIXED>::WARPS * 32, MIXED ? 5 : 3) k_
             } else {
                 if (lane == 0) {
                     if (MIXED) put(0, 0, b0.x, b0.y, b0.z, h0.w);
-                    else sm.lid[0][0] = 0;
+                    if (!MIXED || PNL > 0) sm.lid[0][0] = 0;
                 }
                 lc = 1;
             }
@@ -1927,7 +1974,8 @@ __global__ void __launch_bounds__(TeamSize<MIXED>::WARPS * 32, MIXED ? 5 : 3) k_
                     const float2 ez = __fadd2_rn(__fadd2_rn(cz, ncgz2), make_float2(r3.x, r3.y));
                     if (aL) put(b, pos, ex.x, ey.x, ez.x, r1.z);
                     if (aR) put(b, pos + (aL ? 1 : 0), ex.y, ey.y, ez.y, r1.w);
-                } else {
+                }
+                if (!MIXED || PNL > 0) {
                     if (aL) sm.lid[b][pos] = ch.x;
                     if (aR) sm.lid[b][pos + (aL ? 1 : 0)] = ch.y;
                 }
@@ -1965,7 +2013,8 @@ __global__ void __launch_bounds__(TeamSize<MIXED>::WARPS * 32, MIXED ? 5 : 3) k_
                         sm.lpa[b ^ 1][lane] = sm.lpa[b][TEAM_BATCH / 2 + lane];
                         sm.lpb[b ^ 1][lane] = sm.lpb[b][TEAM_BATCH / 2 + lane];
                     }
-                } else {
+                }
+                if (!MIXED || PNL > 0) {
                     if (lane < rest) sm.lid[b ^ 1][lane] = sm.lid[b][TEAM_BATCH + lane];
                     if (lane + 32 < rest) sm.lid[b ^ 1][lane + 32] = sm.lid[b][TEAM_BATCH + 32 + lane];
                 }
@@ -1985,6 +2034,11 @@ __global__ void __launch_bounds__(TeamSize<MIXED>::WARPS * 32, MIXED ? 5 : 3) k_
             s[0][lane] = MIXED ? sx0.value() : dx0; s[1][lane] = MIXED ? sy0.value() : dy0;
             s[2][lane] = MIXED ? sz0.value() : dz0; s[3][lane] = MIXED ? sx1.value() : dx1;
             s[4][lane] = MIXED ? sy1.value() : dy1; s[5][lane] = MIXED ? sz1.value() : dz1;
+            if (MIXED && PNL > 0) {
+                s[0][lane] += (double)p0.x + (double)q0.x; s[1][lane] += (double)p0.y + (double)q0.y;
+                s[2][lane] += (double)p0.z + (double)q0.z; s[3][lane] += (double)p1.x + (double)q1.x;
+                s[4][lane] += (double)p1.y + (double)q1.y; s[5][lane] += (double)p1.z + (double)q1.z;
+            }
         }
         __syncthreads();
         if (warp == 0) wtotal += (unsigned long long)total * (unsigned long long)gr.y;
@@ -2039,23 +2093,26 @@ __global__ void __launch_bounds__(TeamSize<MIXED>::WARPS * 32, MIXED ? 5 : 3) k_
 // Walk at theta = 0.5, k_walk against the team, us: mixed 5000 bodies 82, 46;
 // 20,011: 125, 66; 60,000: 196, 135; 100,000: 238, 201; 131,073: 244, 248;
 // 262,144: 432, 480. FP64 5000: 164, 64; 20,011: 225, 98; 60,000: 391, 236;
-// 131,073: 580, 492; 262,144: 942, 948; 1,048,576: 3556, 4002.
+// 131,073: 580, 492; 262,144: 942, 948; 1,048,576: 3556, 4002. 1PN mixed 3000:
+// 253, 117; 20,011: 475, 191; 60,000: 597, 370; 119,000: 689, 629; FP64 20,011:
+// 1066, 399; 119,000: 1685, 1527; 190,000: 2490, 2396. Every term, mixed 20,011:
+// 1177, 437; 119,000: 1766, 1572; FP64 20,011: 2237, 804; 190,000: 5588, 5020.
 constexpr int64_t TEAM_MAX_MIXED = 120000, TEAM_MAX_FP64 = 200000;
 
-template <bool MIXED, bool GUARD, bool KICK>
+template <bool MIXED, bool GUARD, bool KICK, int PNL>
 int launch_team(aster_ctx* c, const aster_params* p, int32_t* counts, bool fuse_next) {
     LbvhBufs& t = c->tree;
-    auto kern = k_walk_team<MIXED, GUARD, KICK>;
+    auto kern = k_walk_team<MIXED, GUARD, KICK, PNL>;
     int per_sm = 0;
-    ASTER_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TeamSize<MIXED>::WARPS * 32, 0));
+    ASTER_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TeamSize<MIXED, PNL>::WARPS * 32, 0));
     if (per_sm < 1) per_sm = 1;
     const int64_t blocks = std::min<int64_t>((int64_t)c->sm_count * per_sm, c->n);  // groups <= n
     unsigned int* gcount = red_groups(c);
-    kern<<<(unsigned)blocks, TeamSize<MIXED>::WARPS * 32, 0, c->stream>>>(
+    kern<<<(unsigned)blocks, TeamSize<MIXED, PNL>::WARPS * 32, 0, c->stream>>>(
         c->n, t.groups.as<int2>(), gcount, gcount + 1, t.crec.as<float4>(), t.node_cm.as<double4>(),
         t.child.as<int2>(), t.perm.as<int32_t>(), p->G, p->eps2, 0.5 * p->dt, c->acc.as<double4>(),
         c->vel.as<double4>(), c->err_dev, c->stack_hw_dev, c->walk_stack_limit, counts, red_inter(c),
-        KICK && fuse_next ? c->pm.as<double4>() : nullptr, p->dt, KICK && fuse_next ? red_box(c) : nullptr,
+        PNL > 0 ? t.node_v.as<double4>() : nullptr, make_pn(p), KICK && fuse_next ? c->pm.as<double4>() : nullptr, p->dt, KICK && fuse_next ? red_box(c) : nullptr,
         t.bmin.as<float4>(), t.bmax.as<float4>());
     ASTER_CUDA(cudaGetLastError());
     return ASTER_OK;
@@ -2064,9 +2121,8 @@ int launch_team(aster_ctx* c, const aster_params* p, int32_t* counts, bool fuse_
 template <bool MIXED, bool GUARD, bool KICK, int PNL = 0>
 int launch_walk(aster_ctx* c, const aster_params* p, int32_t* counts, bool fuse_next) {
     LbvhBufs& t = c->tree;
-    if constexpr (PNL == 0) {
-        if (c->n <= (MIXED ? TEAM_MAX_MIXED : TEAM_MAX_FP64)) return launch_team<MIXED, GUARD, KICK>(c, p, counts, fuse_next);
-    }
+    if (c->n <= (MIXED ? TEAM_MAX_MIXED : TEAM_MAX_FP64))
+        return launch_team<MIXED, GUARD, KICK, PNL>(c, p, counts, fuse_next);
     auto kern = k_walk<MIXED, GUARD, KICK, PNL>;
     int per_sm = 0;
     ASTER_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WALK_WARPS * 32, 0));
