@@ -62,7 +62,7 @@ FLOP_PER_EIH_PAIR = 95
 FLOP_PER_ADJ_PAIR = 48
 # Tree build, algorithmic bytes per body: Morton 32 (read the position 24,
 # write code and index 8) + sort 16 (one read and one write of the 8-byte
-# key/value, whatever the pass count) + Karras 24 (read the code, write links
+# key/value, whatever the pass count) + tree links 24 (read the code, write links
 # and ranges) + leaf gather 48 (read position and mass 32, write 16) +
 # bottom-up 120 (per internal node: read two 40-byte child records, write 40)
 BUILD_BYTES_PER_BODY = 240
@@ -359,7 +359,7 @@ def run_ours(args):
                                         + " (no FP32 figure in MEASURED_PEAKS.json)",
                          "flop_per_interaction": FLOP_PER_PAIR},
             "build_roofline": None if build_gbs is None else {
-                "bound": "hbm", "kernels": "tree build (Morton, sort, Karras, bottom-up, node records)",
+                "bound": "hbm", "kernels": "tree build (Morton, sort, bottom-up tree with node records)",
                 "achieved": build_gbs, "peak": peaks.get("hbm_gbs", 6650.0), "unit": "GB/s",
                 "frac": build_gbs / peaks.get("hbm_gbs", 6650.0), "bytes_per_body": BUILD_BYTES_PER_BODY,
                 "peak_source": f"{src} copy bandwidth (MEASURED_PEAKS.json)" if src == "measured"
