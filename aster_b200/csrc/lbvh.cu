@@ -11,7 +11,7 @@
 //            bits per axis). IEEE FP64 add/div, no contraction: bit-exact.
 //   sort     stable LSD radix sort of (code, body index), 8-bit digits:
 //            per pass a tile histogram, a per-digit scan over tiles, a stable
-//            scatter (warp match-any ranking). Ties keep body-index order.
+//            scatter (ranked by warp ballots). Ties keep body-index order.
 //   tree     Karras' (2012) tree exactly as barnes_hut.cpp:338-396 (tie-break
 //            32 + clz(i ^ j) on sorted positions), built bottom up: climbs
 //            meet at their parent's split and the second arrival merges the
@@ -228,9 +228,24 @@ __global__ void __launch_bounds__(1024) k_scan_digits(uint32_t* __restrict__ his
     if (threadIdx.x == 0) digit_tot[blockIdx.x] = carry;
 }
 
+// The lanes of the warp whose keys have this lane's digit (ok: it has a key),
+// from a ballot per bit: match-any takes longer (build of 2^20 bodies 267.6
+// against 258.8 us, 32,768: 78.3 against 75.3).
+__device__ __forceinline__ uint32_t digit_peers(uint32_t d, bool ok) {
+    uint32_t peers = __ballot_sync(0xffffffffu, ok);
+    if (!ok) peers = ~peers;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool one = (d >> b) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, one);
+        peers &= one ? m : ~m;
+    }
+    return peers;
+}
+
 // Stable scatter of one 8-bit digit. Warp w of the block owns the 256 keys
 // [w*256, w*256+256) of the tile and ranks them round by round (32 consecutive
-// keys per round) with __match_any_sync, so ranks follow input order.
+// keys per round) by digit_peers, so ranks follow input order.
 // Global position = (keys of smaller digits) + (same digit in earlier tiles)
 // + (same digit earlier in this tile).
 template <class KeyT, bool IDENTITY_VALS>
@@ -271,7 +286,7 @@ __global__ void __launch_bounds__(SORT_THREADS, 4) k_sort_scatter(int64_t n, con
         const bool ok = i < n;
         const uint32_t d = ok ? ((uint32_t)(key[r] >> shift) & (RADIX - 1)) : 0xFFFFu;
         dig[r] = d;
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t peers = digit_peers(d, ok);
         uint32_t before = 0;
         if (ok) before = wh[warp][d];
         __syncwarp();
@@ -314,17 +329,20 @@ __global__ void __launch_bounds__(SORT_THREADS, 4) k_sort_scatter(int64_t n, con
 // Morton codes and their whole stable sort in one launch, for up to 16 blocks'
 // worth of bodies: a cluster of up to 16 blocks keeps the keys on chip (ITEMS
 // per thread) and exchanges them through distributed shared memory, one 8-bit
-// digit a pass. Per pass: warps rank their keys with match-any as k_sort_scatter
+// digit a pass. Per pass: warps rank their keys as k_sort_scatter
 // does, every block publishes its digit counts to the others, and the keys go
 // straight to their new block and place; the last pass writes to global memory.
-// Bound by latency (two cluster barriers a pass). The general sort takes three
+// Bound by latency (two cluster barriers a pass) and by the number of stores into
+// other blocks: a 32-bit key with its value in one store instead of two and counts
+// eight to a store took the build of 32,768 bodies from 75.3 to 68.1 us (2000: 42.6
+// to 41.0). The general sort takes three
 // launches a pass, ~3.3 us each below 10^5 keys, whatever the size.
 constexpr int CSORT_THREADS = 1024, CSORT_WARPS = CSORT_THREADS / 32, CSORT_BLOCKS = 16;
 
 template <class KeyT>
 constexpr size_t cluster_sort_smem(int items) {
     return (size_t)CSORT_THREADS * items * (sizeof(KeyT) + 4) + (size_t)CSORT_WARPS * RADIX * 2 +
-           (size_t)CSORT_BLOCKS * RADIX * 4 + 2 * RADIX * 4;
+           (size_t)CSORT_BLOCKS * RADIX * 2 + RADIX * 2 + RADIX * 4;
 }
 
 template <class KeyT, int MODE, int ITEMS>
@@ -339,10 +357,10 @@ __global__ void __launch_bounds__(CSORT_THREADS, 1) k_sort_cluster(int64_t n, co
     extern __shared__ __align__(16) unsigned char csort_smem[];
     KeyT* bkey = reinterpret_cast<KeyT*>(csort_smem);
     uint32_t* bval = reinterpret_cast<uint32_t*>(bkey + PER_BLOCK);
-    uint32_t* ctot = bval + PER_BLOCK;            // [block][digit] counts of every block
-    uint32_t* stot = ctot + CSORT_BLOCKS * RADIX;  // [digit] this block's counts
-    uint32_t* sbase = stot + RADIX;                // [digit] place of this block's first key
-    uint16_t* wh = reinterpret_cast<uint16_t*>(sbase + RADIX);  // [warp][digit]
+    uint32_t* sbase = bval + PER_BLOCK;                          // [digit] place of this block's first key
+    uint16_t* ctot = reinterpret_cast<uint16_t*>(sbase + RADIX);  // [block][digit] counts of every block (<= PER_BLOCK)
+    uint16_t* stot = ctot + CSORT_BLOCKS * RADIX;                // [digit] this block's counts
+    uint16_t* wh = stot + RADIX;                                 // [warp][digit]
     __shared__ uint32_t s32[32];
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), nblk = (int)cluster.num_blocks();
@@ -370,8 +388,14 @@ __global__ void __launch_bounds__(CSORT_THREADS, 1) k_sort_cluster(int64_t n, co
         if (pass > 0) {
 #pragma unroll
             for (int r = 0; r < ITEMS; ++r) {
-                key[r] = bkey[local0 + 32 * r];
-                val[r] = bval[local0 + 32 * r];
+                if constexpr (sizeof(KeyT) == 4) {
+                    const uint2 kv = reinterpret_cast<const uint2*>(csort_smem)[local0 + 32 * r];
+                    key[r] = kv.x;
+                    val[r] = kv.y;
+                } else {
+                    key[r] = bkey[local0 + 32 * r];
+                    val[r] = bval[local0 + 32 * r];
+                }
             }
         }
         for (int d = threadIdx.x; d < CSORT_WARPS * RADIX / 2; d += CSORT_THREADS) reinterpret_cast<uint32_t*>(wh)[d] = 0u;
@@ -383,7 +407,7 @@ __global__ void __launch_bounds__(CSORT_THREADS, 1) k_sort_cluster(int64_t n, co
             const bool ok = tile0 + local0 + 32 * r < n;
             const uint32_t d = ok ? (uint32_t)(key[r] >> (8 * pass)) & (RADIX - 1) : 0xFFFFu;
             dig[r] = d;
-            const uint32_t peers = __match_any_sync(0xffffffffu, d);
+            const uint32_t peers = digit_peers(d, ok);
             uint32_t before = 0;
             if (ok) before = w[d];
             __syncwarp();
@@ -400,11 +424,14 @@ __global__ void __launch_bounds__(CSORT_THREADS, 1) k_sort_cluster(int64_t n, co
                 wh[q * RADIX + threadIdx.x] = (uint16_t)tot;
                 tot += t;
             }
-            stot[threadIdx.x] = tot;
+            stot[threadIdx.x] = (uint16_t)tot;
         }
         __syncthreads();
-        for (int x = threadIdx.x; x < nblk * RADIX; x += CSORT_THREADS)
-            cluster.map_shared_rank(ctot, x / RADIX)[rank * RADIX + x % RADIX] = stot[x % RADIX];
+        if (threadIdx.x < nblk * (RADIX / 8)) {  // eight counts a store, one row to each block
+            const int to = threadIdx.x / (RADIX / 8), at = threadIdx.x % (RADIX / 8);
+            reinterpret_cast<uint4*>(cluster.map_shared_rank(ctot, to) + rank * RADIX)[at] =
+                reinterpret_cast<const uint4*>(stot)[at];
+        }
         cluster.sync();  // every block's counts are here; every block has read its keys
         uint32_t all = 0, mine = 0;
         if (threadIdx.x < RADIX) {
@@ -426,8 +453,12 @@ __global__ void __launch_bounds__(CSORT_THREADS, 1) k_sort_cluster(int64_t n, co
                 vout[g] = (int32_t)val[r];
             } else {
                 const int to = (int)(g / PER_BLOCK), at = (int)(g % PER_BLOCK);
-                cluster.map_shared_rank(bkey, to)[at] = key[r];
-                cluster.map_shared_rank(bval, to)[at] = val[r];
+                if constexpr (sizeof(KeyT) == 4) {
+                    cluster.map_shared_rank(reinterpret_cast<uint2*>(csort_smem), to)[at] = make_uint2(key[r], val[r]);
+                } else {
+                    cluster.map_shared_rank(bkey, to)[at] = key[r];
+                    cluster.map_shared_rank(bval, to)[at] = val[r];
+                }
             }
         }
         if (pass < PASSES - 1) cluster.sync();  // the keys have arrived
