@@ -112,26 +112,12 @@ __global__ void __launch_bounds__(BLOCK) k_allpairs_fp64(
             for (int k = 0; k < IPT; ++k) {
                 double dx = pj.x - xi[k], dy = pj.y - yi[k], dz = pj.z - zi[k];
                 double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-                double inv = 0.0, inv2 = 0.0, s;
-                if (PNL) {
-                    inv = inv_r(r2);
-                    inv2 = inv * inv;
-                    s = pj.w * inv * inv2;
+                if (PNL) {  // the sums are accelerations / G; G is applied in store_result
+                    newton_pn_f64<PNL>(pk, dx, dy, dz, inv_r(r2), mi[k], pj.w,
+                                       make_double4(vxi[k], vyi[k], vzi[k], v1sq[k]), sv[q], G, ax[k], ay[k], az[k]);
                 } else {
-                    s = m_inv_r3(pj.w, r2);
-                }
-                ax[k] = fma(dx, s, ax[k]); ay[k] = fma(dy, s, ay[k]); az[k] = fma(dz, s, az[k]);
-                if (PNL) {
-                    const double4 vj = sv[q];
-                    PnPair<double> w;
-                    w.nx = -dx * inv; w.ny = -dy * inv; w.nz = -dz * inv;
-                    w.dvx = vxi[k] - vj.x; w.dvy = vyi[k] - vj.y; w.dvz = vzi[k] - vj.z;
-                    w.inv = inv; w.inv2 = inv2; w.mi = mi[k]; w.mj = pj.w; w.vi2 = v1sq[k]; w.vj2 = vj.w;
-                    w.v12 = vxi[k] * vj.x + vyi[k] * vj.y + vzi[k] * vj.z;
-                    w.nv1 = w.nx * vxi[k] + w.ny * vyi[k] + w.nz * vzi[k];
-                    w.nv2 = w.nx * vj.x + w.ny * vj.y + w.nz * vj.z;
-                    w.G = G;  // the sums are accelerations / G; G is applied in store_result
-                    pn_terms<PNL>(pk, w, ax[k], ay[k], az[k], ax[k], ay[k], az[k]);
+                    const double s = m_inv_r3(pj.w, r2);
+                    ax[k] = fma(dx, s, ax[k]); ay[k] = fma(dy, s, ay[k]); az[k] = fma(dz, s, az[k]);
                 }
             }
         }

@@ -257,7 +257,6 @@ template <int PNL, int UNROLL>
 __device__ __forceinline__ void accel_f64(const EnsSlab<false>& s, int n, int j0, int js, double4 xi, double4 vi,
                                           double eps2, double G, const PnK<double>& k, double& ax, double& ay,
                                           double& az) {
-    double px = 0.0, py = 0.0, pz = 0.0, qx = 0.0, qy = 0.0, qz = 0.0;
     ax = ay = az = 0.0;
 #pragma unroll UNROLL
     for (int j = j0; j < n; j += js) {
@@ -266,23 +265,13 @@ __device__ __forceinline__ void accel_f64(const EnsSlab<false>& s, int n, int j0
         const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
         // (the series step's registers cost the longer PN bodies more than it saves: 1PN unrolled 4, 7.4 -> 8.0 ms)
         const double inv = PNL == 0 ? inv_r_or_0(r2) : r2 > 0.0 ? rsqrt(r2) : 0.0;
-        const double inv2 = inv * inv;
-        const double sN = xj.w * inv * inv2;
-        ax = fma(dx, sN, ax); ay = fma(dy, sN, ay); az = fma(dz, sN, az);
         if (PNL > 0) {
-            const double4 vj = s.v[j];
-            PnPair<double> q;
-            q.nx = -dx * inv; q.ny = -dy * inv; q.nz = -dz * inv;
-            q.dvx = vi.x - vj.x; q.dvy = vi.y - vj.y; q.dvz = vi.z - vj.z;
-            q.inv = inv; q.inv2 = inv2; q.mi = xi.w; q.mj = xj.w; q.vi2 = vi.w; q.vj2 = vj.w;
-            q.v12 = vi.x * vj.x + vi.y * vj.y + vi.z * vj.z;
-            q.nv1 = q.nx * vi.x + q.ny * vi.y + q.nz * vi.z;
-            q.nv2 = q.nx * vj.x + q.ny * vj.y + q.nz * vj.z;
-            q.G = G;
-            pn_terms<PNL>(k, q, px, py, pz, qx, qy, qz);
+            newton_pn_f64<PNL>(k, dx, dy, dz, inv, xi.w, xj.w, vi, s.v[j], G, ax, ay, az);
+        } else {
+            const double sN = xj.w * inv * (inv * inv);
+            ax = fma(dx, sN, ax); ay = fma(dy, sN, ay); az = fma(dz, sN, az);
         }
     }
-    ax += px + qx; ay += py + qy; az += pz + qz;
 }
 
 // EIH pass 1 (level 3): Newtonian sum m_j d / r^3 and potential sum m_j / r

@@ -1233,18 +1233,7 @@ __device__ __forceinline__ void interact_pn_f64(const double4 e, const double4 e
                                                 double& az) {
     const double dx = e.x - b.x, dy = e.y - b.y, dz = e.z - b.z;
     const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-    const double inv = inv_r(r2);
-    const double s = e.w * inv * inv * inv;
-    ax = fma(dx, s, ax); ay = fma(dy, s, ay); az = fma(dz, s, az);
-    PnPair<double> w;
-    w.nx = -dx * inv; w.ny = -dy * inv; w.nz = -dz * inv;
-    w.dvx = vi.x - ev.x; w.dvy = vi.y - ev.y; w.dvz = vi.z - ev.z;
-    w.inv = inv; w.inv2 = inv * inv; w.mi = b.w; w.mj = e.w; w.vi2 = vi.w; w.vj2 = ev.w;
-    w.v12 = vi.x * ev.x + vi.y * ev.y + vi.z * ev.z;
-    w.nv1 = w.nx * vi.x + w.ny * vi.y + w.nz * vi.z;
-    w.nv2 = w.nx * ev.x + w.ny * ev.y + w.nz * ev.z;
-    w.G = G;
-    pn_terms<PNL>(k, w, ax, ay, az, ax, ay, az);
+    newton_pn_f64<PNL>(k, dx, dy, dz, inv_r(r2), b.w, e.w, vi, ev, G, ax, ay, az);
 }
 
 // Two entries at once with the paired FP32 instructions, force law Newton +
@@ -2127,7 +2116,9 @@ __global__ void __launch_bounds__(TeamSize<MIXED, PNL>::WARPS * 32, TeamSize<MIX
 // 131,073: 580, 492; 262,144: 942, 948; 1,048,576: 3556, 4002. 1PN mixed 3000:
 // 253, 117; 20,011: 475, 191; 60,000: 597, 370; 119,000: 689, 629; FP64 20,011:
 // 1066, 399; 119,000: 1685, 1527; 190,000: 2490, 2396. Every term, mixed 20,011:
-// 1177, 437; 119,000: 1766, 1572; FP64 20,011: 2237, 804; 190,000: 5588, 5020.
+// 1177, 437; 119,000: 1766, 1572; FP64 20,011: 2237, 804; 190,000: 5588, 5020
+// (FP64 figures from before its pair terms were gathered, which took a fifth to a
+// third off both walks).
 constexpr int64_t TEAM_MAX_MIXED = 120000, TEAM_MAX_FP64 = 200000;
 
 template <bool MIXED, bool GUARD, bool KICK, int PNL>

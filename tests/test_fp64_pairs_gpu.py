@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 from aster_b200 import gen
-from aster_b200.api import FP64, MIXED, NEWTON, PN1, PN2, SOLVER_ALLPAIRS, Params
+from aster_b200.api import FP64, MIXED, NEWTON, PN1, PN2, PN25, SOLVER_ALLPAIRS, Params
 from conftest import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -144,3 +144,19 @@ def test_fused_drift_equals_single_steps(ctx, n, prec, law):
     for o in out[1:]:
         for a, b in zip(out[0], o):
             np.testing.assert_array_equal(a, b)
+
+
+# the gathered post-Newtonian pair (pn.cuh: newton_pn_f64), every set of terms, all-pairs and the tree with every node opened
+@pytest.mark.parametrize("terms", [PN2, PN25, PN1 | PN2, PN1 | PN25, PN2 | PN25, PN1 | PN2 | PN25])
+@pytest.mark.parametrize("n,eps2", [(1, 1e-4), (97, 0.0), (700, 1e-4)])
+def test_gathered_pn_terms(ctx, orc, n, eps2, terms):
+    pos, vel, m = gen.plummer(n, 500 + n, masses="lognormal")
+    vel = vel * 5.0
+    ref = orc.allpairs(pos, m, 1.0, eps2, vel=vel, inv_c=0.1, pn=NEWTON | terms)
+    ctx.upload(pos, vel, m)
+    p = Params(eps2=eps2, theta=0.0, c=10.0, force_law=NEWTON | terms)
+    for acc in (ctx.allpairs(p, FP64), ctx.lbvh_forces(p, FP64)):
+        if n == 1:
+            assert np.all(acc == 0.0)
+        else:
+            assert rel_l2(acc, ref) < 1e-12
