@@ -268,18 +268,26 @@ __global__ void __launch_bounds__(WH_BLOCK) k_wh_cba(int64_t n, double4* __restr
     block_sum4_last(sum, part, done, pout);
 }
 
-// The run's last C(h) and B(h) with the interaction of src_in.
+// The run's last C(h) and B(h) with the interaction of src_in (positions before
+// C, which moves all bodies but the central one by the same amount). The
+// interaction goes to acc, as the separate force launch leaves it there.
 __global__ void __launch_bounds__(WH_BLOCK) k_wh_cb(int64_t n, double4* __restrict__ pm, double4* __restrict__ vel,
-                                                    const double* st, const double* pin, double h, int nsrc,
-                                                    const double4* __restrict__ src_in, double G, double eps2) {
+                                                    double4* __restrict__ acc, const double* st, const double* pin,
+                                                    double h, int nsrc, const double4* __restrict__ src_in, double G,
+                                                    double eps2) {
     __shared__ double4 src[WH_SRC];
     if ((int)threadIdx.x < nsrc) src[threadIdx.x] = src_in[threadIdx.x];
     __syncthreads();
     const double m0 = st[0];
     const double px = pin[0] / m0 * h, py = pin[1] / m0 * h, pz = pin[2] / m0 * h;
-    for (int64_t i = 1 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double4 p = pm[i], v = vel[i];
+        if (i == 0) {  // not moved by C: the sources are after it, seen from here
+            acc[0] = wh_interaction(src, nsrc, make_double4(p.x - px, p.y - py, p.z - pz, p.w), G, eps2);
+            continue;
+        }
         const double4 a = wh_interaction(src, nsrc, p, G, eps2);
+        acc[i] = a;
         v.x += a.x * h; v.y += a.y * h; v.z += a.z * h;
         p.x += px; p.y += py; p.z += pz;
         pm[i] = p;
@@ -434,7 +442,8 @@ int aster_wh_enqueue(aster_ctx* c, const aster_params* p, int precision, int nst
         c->stats.kernels += 1;
     }
     if (st == ASTER_OK && done > 0 && fused) {  // the last C(h) B(h)
-        k_wh_cb<<<grid, WH_BLOCK, 0, c->stream>>>(n, pm, vel, L.st, pslot[cur], h, nsrc, L.src[done & 1], p->G, p->eps2);
+        k_wh_cb<<<grid, WH_BLOCK, 0, c->stream>>>(n, pm, vel, c->acc.as<double4>(), L.st, pslot[cur], h, nsrc,
+                                                  L.src[done & 1], p->G, p->eps2);
         st = wh_launch_status();
         c->stats.kernels += 1;
         c->stats.interactions += (double)n * (double)nsrc;
