@@ -391,7 +391,7 @@ extern "C" int aster_adjoint_leapfrog(aster_ctx* c, const aster_params* p, int p
     ASTER_TRY(a.target.ensure((size_t)n * 3 * sizeof(double)));
     ASTER_TRY(c->red.ensure(4096));
     const int nb = (int)std::min<int64_t>((n + 255) / 256, 1024);
-    ASTER_TRY(c->scratch.ensure((size_t)nb * sizeof(double) + 64));
+    ASTER_TRY(a.loss.ensure((size_t)nb * sizeof(double)));  // not in scratch: a force evaluation may have to give that up
     ASTER_CUDA(cudaMemcpyAsync(a.target.ptr, target, (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice,
                                c->stream));
     char* ck = a.ckpt.as<char>();
@@ -420,10 +420,10 @@ extern "C" int aster_adjoint_leapfrog(aster_ctx* c, const aster_params* p, int p
     }
     // loss and seeds
     k_adj_seed<<<nb, 256, 0, c->stream>>>(n, c->pm.as<double4>(), a.target.as<double>(), a.lx.as<double4>(),
-                                          a.lv.as<double4>(), a.lm.as<double>(), c->scratch.as<double>());
+                                          a.lv.as<double4>(), a.lm.as<double>(), a.loss.as<double>());
     ASTER_CUDA(cudaGetLastError());
     double* loss_dev = red_energy(c) + 4;
-    k_adj_loss_final<<<1, 32, 0, c->stream>>>(nb, c->scratch.as<double>(), 1.0 / (double)n, loss_dev);
+    k_adj_loss_final<<<1, 32, 0, c->stream>>>(nb, a.loss.as<double>(), 1.0 / (double)n, loss_dev);
     ASTER_CUDA(cudaGetLastError());
 
     // reverse pass, segment by segment

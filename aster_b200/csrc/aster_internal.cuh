@@ -90,7 +90,7 @@ struct EnsBufs {
 
 // Adjoint (reverse-mode) buffers.
 struct AdjBufs {
-    DevBuf ckpt, segx, lx, lv, lm, w, target, part;
+    DevBuf ckpt, segx, lx, lv, lm, w, target, part, loss;
 };
 
 // An executable graph of one repeated step, kept across calls: replayed by

@@ -146,7 +146,7 @@ extern "C" int aster_ctx_destroy(aster_ctx* c) {
     for (DevBuf* b : bufs) b->release();
     DevBuf* ens[] = {&c->ens.pm, &c->ens.vel, &c->ens.off, &c->ens.order, &c->ens.counter,
                      &c->adj.ckpt, &c->adj.segx, &c->adj.lx, &c->adj.lv, &c->adj.lm, &c->adj.w,
-                     &c->adj.target, &c->adj.part};
+                     &c->adj.target, &c->adj.part, &c->adj.loss};
     for (DevBuf* b : ens) b->release();
     if (c->ens.cancel_host) cudaFreeHost((void*)c->ens.cancel_host);
     for (int i = 0; i < 6; ++i)

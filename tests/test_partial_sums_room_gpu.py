@@ -1,0 +1,67 @@
+"""Force and adjoint calls when the device has little memory left: the kernels'
+partial sums find no room and the sums are made in one piece.
+
+The other tensors take the memory (torch allocations); what is left free is a
+fixed number of megabytes, enough for everything but the partial sums."""
+import numpy as np
+import pytest
+
+from aster_b200 import gen
+from aster_b200.api import MIXED, AsterError, Context, Params
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+MB = 1 << 20
+ERR_OOM = 3
+
+
+class Crowd:
+    """Takes all device memory but `leave` bytes while it lasts."""
+
+    def __init__(self, leave):
+        self.leave = leave
+
+    def __enter__(self):
+        import torch
+        torch.cuda.empty_cache()
+        self.held = []
+        while True:
+            free = torch.cuda.mem_get_info()[0]
+            if free <= self.leave + 32 * MB:
+                return self
+            size = min(free - self.leave, 8192 * MB) // (2 * MB) * (2 * MB)
+            self.held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+
+    def __exit__(self, *exc):
+        import torch
+        self.held = None
+        torch.cuda.empty_cache()
+
+
+def test_adjoint_without_room_is_an_error_or_right():
+    """131,072 bodies: 32 slices of sums take 134 MB, the call's other arrays 60."""
+    n = 131072
+    pos, vel, m = gen.plummer(n, 41)
+    target = pos + 0.01
+    p = Params(eps2=1e-4, dt=1e-3)
+    with Context(0) as roomy:  # (and every kernel has been loaded)
+        ref = roomy.upload(pos, vel, m).adjoint(p, 3, target, MIXED, 2)
+        small = Context(0).upload(pos[:70], vel[:70], m[:70])  # one slice
+        small.adjoint(p, 3, target[:70], MIXED, 2)
+        small.close()
+    with Context(0) as c:
+        c.upload(pos, vel, m)
+        with Crowd(100 * MB):
+            try:
+                got = c.adjoint(p, 3, target, MIXED, 2)
+            except AsterError as e:
+                assert e.status == ERR_OOM
+                got = None
+        if got is not None:
+            assert abs(got[0] - ref[0]) <= 1e-9 * ref[0]
+            for g, r in zip(got[1:], ref[1:]):
+                assert rel_l2(g, r) < 1e-5
+        again = c.upload(pos, vel, m).adjoint(p, 3, target, MIXED, 2)
+        assert again[0] == ref[0]
+        for g, r in zip(again[1:], ref[1:]):
+            np.testing.assert_array_equal(g, r)
