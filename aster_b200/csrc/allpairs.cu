@@ -444,7 +444,7 @@ int aster_allpairs_launch_range(aster_ctx* c, const aster_params* p, int precisi
     if (fuse_next && (ns < 2 || !closing_kick || out_dev || targets_dev)) return ASTER_ERR_UNSUPPORTED;
     double4* partial = nullptr;
     if (ns > 1) {
-        const int st = c->scratch.ensure((size_t)ns * nt * sizeof(double4));
+        const int st = aster_sums_ensure(c, c->scratch, (size_t)ns * nt * sizeof(double4));
         if (st == ASTER_ERR_OOM && !fuse_next) {  // no room for the partial sums: one slice
             ns = 1;
             slice_len = std::max<int64_t>((len + BLOCK - 1) / BLOCK, 1) * BLOCK;
@@ -494,7 +494,7 @@ bool aster_allpairs_can_fuse(aster_ctx* c, const aster_params* p, int precision)
         if (aster_allpairs_sym_prepare(c, p) == ASTER_OK) return true;
     const int64_t n_src = c->n_src > 0 ? c->n_src : c->n;
     const int64_t ns = slice_grid(c, p, precision, c->n, n_src).ns;
-    return ns > 1 && c->scratch.ensure((size_t)ns * c->n * sizeof(double4)) == ASTER_OK;
+    return ns > 1 && aster_sums_ensure(c, c->scratch, (size_t)ns * c->n * sizeof(double4)) == ASTER_OK;
 }
 
 extern "C" int aster_allpairs(aster_ctx* c, const aster_params* p, int precision, double* acc_out) {

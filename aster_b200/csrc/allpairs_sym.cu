@@ -309,7 +309,7 @@ constexpr int64_t SYM_MIN = 128;
 // Newtonian and 1PN laws from SYM_MIN bodies on. Trailing massless bodies
 // (n_src < n) stay with the directed kernel, whose source loop leaves them out.
 bool aster_allpairs_sym_fits(const aster_ctx* c, const aster_params* p) {
-    return pn_level(p) <= 1 && c->n >= SYM_MIN && c->n_src == c->n && c->n < c->sym_oom_n;
+    return pn_level(p) <= 1 && c->n >= SYM_MIN && c->n_src == c->n;
 }
 
 static SymArgs sym_args(const aster_ctx* c, const aster_params* p) {
@@ -331,13 +331,11 @@ static SymArgs sym_args(const aster_ctx* c, const aster_params* p) {
     return g;
 }
 
-// Room for the partial array. ASTER_ERR_OOM: there is none, and the context's
-// evaluations of this size go to the directed kernel from then on.
+// Room for the partial array. ASTER_ERR_OOM: there is none, and the evaluation
+// goes to the directed kernel.
 int aster_allpairs_sym_prepare(aster_ctx* c, const aster_params* p) {
     const SymArgs g = sym_args(c, p);
-    const int st = c->scratch.ensure((size_t)g.slots * 3 * g.npad * sizeof(double));
-    if (st == ASTER_ERR_OOM) c->sym_oom_n = c->n;
-    return st;
+    return aster_sums_ensure(c, c->scratch, (size_t)g.slots * 3 * g.npad * sizeof(double));
 }
 
 // One evaluation (ASTER_ERR_OOM: nothing was launched), with the closing kick

@@ -133,8 +133,9 @@ struct aster_ctx {
     // pm/vel; anything that moves positions or velocities without refreshing
     // them clears it, and a mixed all-pairs launch refreshes them first
     bool mixed_valid = false;
-    // smallest body count whose symmetric FP64 all-pairs partials did not fit
-    int64_t sym_oom_n = INT64_MAX;
+    // smallest size (bytes) at which partial sums found no room: not tried again
+    // (a captured step may not allocate)
+    size_t sums_oom = SIZE_MAX;
     int* err_dev = nullptr;     // device error flags
     int* err_host = nullptr;    // pinned copy
     int* stack_hw_dev = nullptr;  // tree-walk stack high-water mark
@@ -181,6 +182,9 @@ int aster_upload_enqueue_overlapped(aster_ctx* c, int64_t n, const double* pos, 
                                     const double* acc, const aster_params* kick_drift = nullptr);
 // velocities and accelerations -> host (one unpack, two back-to-back copies)
 int aster_download_va_enqueue(aster_ctx* c, double* vel, double* acc, cudaStream_t stream);
+// Room for `want` bytes of partial sums in b. ASTER_ERR_OOM: there is none, and
+// the caller makes its sums in one piece.
+int aster_sums_ensure(aster_ctx* c, DevBuf& b, size_t want);
 // applies masses still on their way (waits for their copy); no-op otherwise
 int aster_apply_pending_mass(aster_ctx* c);
 int aster_copy_acc_out(aster_ctx* ctx, double* acc_out);

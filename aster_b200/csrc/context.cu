@@ -57,6 +57,14 @@ void DevBuf::release() {
     bytes = 0;
 }
 
+int aster_sums_ensure(aster_ctx* c, DevBuf& b, size_t want) {
+    if (b.ptr && want <= b.bytes) return ASTER_OK;
+    if (want >= c->sums_oom) return ASTER_ERR_OOM;
+    const int st = b.ensure(want);
+    if (st == ASTER_ERR_OOM) c->sums_oom = want;
+    return st;
+}
+
 extern "C" const char* aster_strerror(int s) {
     switch (s) {
         case ASTER_OK: return "ok";

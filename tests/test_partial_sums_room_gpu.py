@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from aster_b200 import gen
-from aster_b200.api import MIXED, AsterError, Context, Params
+from aster_b200.api import FP64, MIXED, SOLVER_ALLPAIRS, AsterError, Context, Params
 from conftest import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +65,26 @@ def test_adjoint_without_room_is_an_error_or_right():
         assert again[0] == ref[0]
         for g, r in zip(again[1:], ref[1:]):
             np.testing.assert_array_equal(g, r)
+
+
+@pytest.mark.parametrize("prec,tol", [(MIXED, 1e-6), (FP64, 1e-12)])
+@pytest.mark.parametrize("steps", [1, 2, 3, 6])
+def test_steps_without_room_run_in_one_piece(prec, tol, steps):
+    """All-pairs steps, the later ones captured: a step that finds no room for its sums looks for it once, before the
+    capture. 131,072 bodies need 134 MB (slices) or 403 MB (tile pairs), 64 are free. Accelerations as far apart as
+    two orders of one sum (mixed: FP32 pair terms)."""
+    n = 131072
+    pos, vel, m = gen.plummer(n, 42)
+    p = Params(eps2=1e-4, dt=1e-3)
+    with Context(0) as roomy:
+        roomy.upload(pos, vel, m).kdk_steps(p, steps, SOLVER_ALLPAIRS, prec)
+        ref = roomy.download()
+        kernels = roomy.stats()["kernels"]
+    with Context(0) as c:
+        c.upload(pos, vel, m)
+        with Crowd(64 * MB):
+            c.kdk_steps(p, steps, SOLVER_ALLPAIRS, prec)
+            assert c.stats()["kernels"] == kernels - 2  # a kick-drift in every step, and no reductions
+            got = c.download()
+    for g, r in zip(got, ref):
+        assert rel_l2(g, r) < tol
