@@ -134,7 +134,8 @@ struct aster_ctx {
     // them clears it, and a mixed all-pairs launch refreshes them first
     bool mixed_valid = false;
     // smallest size (bytes) at which partial sums found no room: not tried again
-    // (a captured step may not allocate)
+    // within the call (a captured step may not allocate), nor later while the
+    // device has less than that free
     size_t sums_oom = SIZE_MAX;
     int* err_dev = nullptr;     // device error flags
     int* err_host = nullptr;    // pinned copy

@@ -181,6 +181,11 @@ static void release_graphs(aster_ctx* c) {
 int aster_begin(aster_ctx* c) {
     ASTER_CUDA(cudaSetDevice(c->device));
     release_graphs(c);  // the previous call synchronised before returning
+    if (c->sums_oom != SIZE_MAX) {  // there may be room by now (what scratch holds is given up first)
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b + c->scratch.bytes >= c->sums_oom)
+            c->sums_oom = SIZE_MAX;
+    }
     ASTER_CUDA(cudaMemsetAsync(c->err_dev, 0, 2 * sizeof(int), c->stream));
     return ASTER_OK;
 }

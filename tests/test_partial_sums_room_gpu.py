@@ -88,3 +88,20 @@ def test_steps_without_room_run_in_one_piece(prec, tol, steps):
             got = c.download()
     for g, r in zip(got, ref):
         assert rel_l2(g, r) < tol
+
+
+def test_room_that_comes_free_is_used():
+    """FP64 forces of 300,000 bodies: 921 MB of tile-pair sums do not fit into 600; once the memory is free again the
+    same context takes the tile pairs (the sums of a fresh context, bit for bit)."""
+    n = 300000
+    pos, vel, m = gen.plummer(n, 43)
+    p = Params(eps2=1e-4)
+    with Context(0) as roomy:
+        ref = roomy.upload(pos, vel, m).allpairs(p, FP64)
+    with Context(0) as c:
+        c.upload(pos, vel, m)
+        with Crowd(600 * MB):
+            tight = c.allpairs(p, FP64)
+            np.testing.assert_array_equal(c.allpairs(p, FP64), tight)
+        assert not np.array_equal(tight, ref) and rel_l2(tight, ref) < 1e-12
+        np.testing.assert_array_equal(c.allpairs(p, FP64), ref)
