@@ -318,12 +318,18 @@ int adj_pair_launch(aster_ctx* c, const aster_params* p, int precision, const do
     AdjBufs& a = c->adj;
     const int64_t n = c->n;
     const int64_t iblocks = (n + BLOCK * IPT - 1) / (BLOCK * IPT);
-    const int64_t slice_len = aster_slice_tiles(iblocks, (n + BLOCK - 1) / BLOCK, c->sm_count) * BLOCK;
-    const int64_t ns = (n + slice_len - 1) / slice_len;
+    int64_t slice_len = aster_slice_tiles(iblocks, (n + BLOCK - 1) / BLOCK, c->sm_count) * BLOCK;
+    int64_t ns = (n + slice_len - 1) / slice_len;
     double4* partial = nullptr;
     if (ns > 1) {
-        ASTER_TRY(a.part.ensure((size_t)ns * n * sizeof(double4)));
-        partial = a.part.as<double4>();
+        const int st = aster_sums_ensure(c, a.part, (size_t)ns * n * sizeof(double4));
+        if (st == ASTER_ERR_OOM) {  // no room for the partial sums: one slice
+            ns = 1;
+            slice_len = (n + BLOCK - 1) / BLOCK * BLOCK;
+        } else {
+            ASTER_TRY(st);
+            partial = a.part.as<double4>();
+        }
     }
     const dim3 grid((unsigned)iblocks, (unsigned)ns);
     const bool guard = !(p->eps2 > 0.0);

@@ -105,3 +105,23 @@ def test_room_that_comes_free_is_used():
             np.testing.assert_array_equal(c.allpairs(p, FP64), tight)
         assert not np.array_equal(tight, ref) and rel_l2(tight, ref) < 1e-12
         np.testing.assert_array_equal(c.allpairs(p, FP64), ref)
+
+
+@pytest.mark.parametrize("prec,tol", [(MIXED, 1e-5), (FP64, 1e-10)])
+def test_adjoint_without_room_runs_in_one_piece(prec, tol):
+    """Gradients as far from those with room as test_adjoint_steps_gpu.py lets either be from the oracle."""
+    n = 131072
+    pos, vel, m = gen.plummer(n, 44)
+    target = pos + 0.01
+    p = Params(eps2=1e-4, dt=1e-3)
+    with Context(0) as roomy:
+        ref = roomy.upload(pos, vel, m).adjoint(p, 3, target, prec, 2)
+        kernels = roomy.stats()["kernels"]
+    with Context(0) as c:
+        c.upload(pos, vel, m)
+        with Crowd(100 * MB):
+            got = c.adjoint(p, 3, target, prec, 2)
+            assert c.stats()["kernels"] < kernels  # no reductions
+        assert abs(got[0] - ref[0]) <= tol * ref[0]
+        for g, r in zip(got[1:], ref[1:]):
+            assert rel_l2(g, r) < tol
