@@ -43,7 +43,7 @@ constexpr double SYM_FAR = 1.0e99, SYM_EPS2 = 1.0e-199;
 
 struct SymArgs {
     int64_t n, npad;
-    int tile, slots;
+    int set, tile, slots;  // bodies of the i sets, bodies of a tile (whole sets), tiles
     const double4* pm;
     const double4* vel;
     double eps2, G, c2;
@@ -290,11 +290,16 @@ int launch_sym(aster_ctx* c, const SymArgs& g) {
     return ASTER_OK;
 }
 
-// Tiles: as many as SYM_SLOTS allows. The partial array is SYM_SLOTS x 24 bytes
-// a body, and every tile pair writes two of its rows; 128 slots give 8256 tile
-// pairs for the 296 resident blocks. 262,144 bodies with 64 / 128 / 256 slots:
-// 55.8 / 52.9 / 52.8 ms; 40,000 bodies: 1.37 / 1.30 / 1.31 ms (4 bodies per lane).
-constexpr int SYM_SLOTS = 128;
+// Tiles: as many as SYM_SLOTS and the limit on the partial sums (1 GB) allow. The
+// partial array is 24 bytes a body and slot, and every tile pair writes two of its
+// rows; 128 slots give 8256 tile pairs for the 296 resident blocks. 262,144 bodies
+// with 64 / 128 / 256 slots: 55.8 / 52.9 / 52.8 ms; 40,000 bodies: 1.37 / 1.30 /
+// 1.31 ms (4 bodies per lane). Beyond 349,525 bodies fewer slots fit: 699,050 with
+// 128 / 64 / 24 slots 342 / 353 / 386 ms, 2^20 with 128 / 42 / 24 765 / 831 / 946.
+// Fewer than SYM_SLOTS_MIN are fewer tile pairs than resident blocks, and the
+// directed kernel is as fast: 2^20 with 20 slots 1239 ms, directed 1243; 1PN at
+// 524,289 604 ms with 128 slots, 690 with 24, 962 with 20, directed 873.
+constexpr int SYM_SLOTS = 128, SYM_SLOTS_MIN = 24;
 // Smaller systems take tiles of 64 bodies (2 per lane, 2 warps), larger ones
 // of 256 (8 per lane, 4 warps; 1PN 128 and 4): Newton at 4096 bodies 0.033
 // against 0.029 ms, at 8192 0.087 against 0.076; 1PN at 1000 0.021 against
@@ -305,21 +310,16 @@ constexpr int64_t SYM_MIN = 128;
 
 }  // namespace
 
-// Whether an evaluation of all bodies on all bodies takes this path: the
-// Newtonian and 1PN laws from SYM_MIN bodies on. Trailing massless bodies
-// (n_src < n) stay with the directed kernel, whose source loop leaves them out.
-bool aster_allpairs_sym_fits(const aster_ctx* c, const aster_params* p) {
-    return pn_level(p) <= 1 && c->n >= SYM_MIN && c->n_src == c->n;
-}
-
 static SymArgs sym_args(const aster_ctx* c, const aster_params* p) {
     const int pnl = pn_level(p);
-    const int set = c->n < SYM_SMALL ? 64 : pnl ? 128 : 256;
     SymArgs g;
+    const int set = g.set = c->n < SYM_SMALL ? 64 : pnl ? 128 : 256;
     g.n = c->n;
     g.npad = (c->n + set - 1) / set * set;
     const int64_t sets = g.npad / set;
-    g.tile = (int)((sets + SYM_SLOTS - 1) / SYM_SLOTS) * set;
+    int64_t most = std::min<int64_t>(SYM_SLOTS, (int64_t)(c->sums_limit / (24 * (size_t)g.npad)));
+    if (most < 1) most = 1;
+    g.tile = (int)((sets + most - 1) / most) * set;
     if (g.tile > JT) g.tile = (g.tile + JT - 1) / JT * JT;
     g.slots = (int)((g.npad + g.tile - 1) / g.tile);
     g.pm = c->pm.as<double4>();
@@ -331,11 +331,22 @@ static SymArgs sym_args(const aster_ctx* c, const aster_params* p) {
     return g;
 }
 
+static size_t sym_bytes(const SymArgs& g) { return (size_t)g.slots * 3 * g.npad * sizeof(double); }
+
+// Whether an evaluation of all bodies on all bodies takes this path: the
+// Newtonian and 1PN laws from SYM_MIN bodies on. Trailing massless bodies
+// (n_src < n) stay with the directed kernel, whose source loop leaves them out, as
+// do systems for which the partial sums' limit allows too few slots.
+bool aster_allpairs_sym_fits(const aster_ctx* c, const aster_params* p) {
+    if (pn_level(p) > 1 || c->n < SYM_MIN || c->n_src != c->n) return false;
+    const SymArgs g = sym_args(c, p);
+    return g.tile == g.set || g.slots >= SYM_SLOTS_MIN;
+}
+
 // Room for the partial array. ASTER_ERR_OOM: there is none, and the evaluation
 // goes to the directed kernel.
 int aster_allpairs_sym_prepare(aster_ctx* c, const aster_params* p) {
-    const SymArgs g = sym_args(c, p);
-    return aster_sums_ensure(c, c->scratch, (size_t)g.slots * 3 * g.npad * sizeof(double));
+    return aster_sums_ensure(c, c->scratch, sym_bytes(sym_args(c, p)));
 }
 
 // One evaluation (ASTER_ERR_OOM: nothing was launched), with the closing kick

@@ -137,6 +137,9 @@ struct aster_ctx {
     // within the call (a captured step may not allocate), nor later while the
     // device has less than that free
     size_t sums_oom = SIZE_MAX;
+    // most bytes that one buffer of partial sums may take (it is kept until the
+    // context goes); ASTER_SUMS_LIMIT (megabytes) lowers it
+    size_t sums_limit = (size_t)1 << 30;
     int* err_dev = nullptr;     // device error flags
     int* err_host = nullptr;    // pinned copy
     int* stack_hw_dev = nullptr;  // tree-walk stack high-water mark

@@ -59,7 +59,7 @@ void DevBuf::release() {
 
 int aster_sums_ensure(aster_ctx* c, DevBuf& b, size_t want) {
     if (b.ptr && want <= b.bytes) return ASTER_OK;
-    if (want >= c->sums_oom) return ASTER_ERR_OOM;
+    if (want > c->sums_limit || want >= c->sums_oom) return ASTER_ERR_OOM;
     const int st = b.ensure(want);
     if (st == ASTER_ERR_OOM) c->sums_oom = want;
     return st;
@@ -130,6 +130,10 @@ extern "C" int aster_ctx_create(aster_ctx** out, int device, void* stream) {
     if (const char* lim = std::getenv("ASTER_WALK_STACK_LIMIT")) {
         const int v = std::atoi(lim);
         if (v >= 64 && v < c->walk_stack_limit) c->walk_stack_limit = v;
+    }
+    if (const char* lim = std::getenv("ASTER_SUMS_LIMIT")) {
+        const long long v = std::atoll(lim);
+        if (v >= 0 && v < 100000) c->sums_limit = (size_t)v << 20;
     }
     cudaMemset(c->err_dev, 0, 2 * sizeof(int));
     *out = c;

@@ -2,12 +2,13 @@
 partial sums find no room and the sums are made in one piece.
 
 The other tensors take the memory (torch allocations); what is left free is a
-fixed number of megabytes, enough for everything but the partial sums."""
+fixed number of megabytes, enough for everything but the partial sums. Last, the
+limit on the sums of a context that has all the room it could want."""
 import numpy as np
 import pytest
 
 from aster_b200 import gen
-from aster_b200.api import FP64, MIXED, SOLVER_ALLPAIRS, AsterError, Context, Params
+from aster_b200.api import FP64, MIXED, NEWTON, PN1, SOLVER_ALLPAIRS, AsterError, Context, Params
 from conftest import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -125,3 +126,44 @@ def test_adjoint_without_room_runs_in_one_piece(prec, tol):
         assert abs(got[0] - ref[0]) <= tol * ref[0]
         for g, r in zip(got[1:], ref[1:]):
             assert rel_l2(g, r) < tol
+
+
+def _free():
+    import torch
+    return torch.cuda.mem_get_info()[0]
+
+
+@pytest.mark.parametrize("limit,n,law", [(8, 12500, NEWTON), (8, 12500, NEWTON | PN1), (2, 20000, NEWTON), (2, 3900, NEWTON | PN1),
+                                         (0, 5000, NEWTON), (0, 130, NEWTON)])
+@pytest.mark.parametrize("prec,tol", [(MIXED, 1e-6), (FP64, 1e-12)])
+def test_limited_sums_give_the_same_results(monkeypatch, limit, n, law, prec, tol):
+    """Fewer tiles than without a limit (12,500 bodies: 25), the directed kernel with one slice (20,000; 3900), and no
+    sums at all: forces, steps and gradients, and the memory that the first of them takes."""
+    pos, vel, m = gen.plummer(n, 45 + n)
+    p = Params(eps2=1e-4, dt=1e-3, c=50.0, force_law=law)
+    out = []
+    for lim in (None, limit):
+        if lim is not None:
+            monkeypatch.setenv("ASTER_SUMS_LIMIT", str(lim))
+        with Context(0) as c:
+            c.upload(pos, vel, m)
+            free = _free()
+            a = c.allpairs(p, prec)
+            if lim is not None:
+                assert free - _free() <= (lim + 2) * MB  # (the device hands out 2 MB at a time)
+            c.kdk_steps(p, 5, SOLVER_ALLPAIRS, prec)
+            state = c.download()
+            grads = () if law != NEWTON else c.upload(pos, vel, m).adjoint(p, 3, pos + 0.01, prec, 2)[1:]
+        out.append((a, *state, *grads))
+    for k, (x, y) in enumerate(zip(*out)):
+        assert rel_l2(y, x) < (tol if k < 4 else 10 * tol), k
+
+
+def test_sums_of_a_large_system_stay_within_the_limit():
+    n = 1 << 20
+    pos, vel, m = gen.plummer(n, 46)
+    with Context(0) as c:
+        c.upload(pos, vel, m)
+        free = _free()
+        c.allpairs(Params(eps2=1e-4), FP64)
+        assert free - _free() <= 1026 * MB
