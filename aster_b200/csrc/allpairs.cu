@@ -405,6 +405,15 @@ void launch_pnl(int precision, bool guard, dim3 grid, cudaStream_t st, int64_t j
 
 }  // namespace
 
+// The first allocation that takes a context past the 2 MB its state shares costs
+// some 0.35 ms, six small evaluations. Where mixed slices of one tile make that
+// much partial sums and slices of two do not (2433 to 3072 bodies), two are
+// taken: first evaluation of a context 415 -> 75 us at 2500 bodies and 428 -> 78
+// at 3000, a step 14.4 -> 14.4 and 14.4 -> 16.4 us (1PN 20.5 -> 22.6, 22.6 ->
+// 22.6). With 2PN or 2.5PN terms the longer slices cost more than that (2500
+// bodies 39 -> 49 us a step).
+constexpr int64_t SUMS_LARGE = 1480000, SUMS_SMALL = 1180000;  // bytes
+
 // Source slices of an evaluation of nt targets against len sources.
 struct SliceGrid {
     int64_t iblocks, ns, slice_len;
@@ -415,7 +424,10 @@ static SliceGrid slice_grid(const aster_ctx* c, const aster_params* p, int preci
     // one target per thread in the mixed post-Newtonian kernel, two elsewhere
     const int64_t per_block = (int64_t)BLOCK * (precision == ASTER_MIXED && pnl > 0 ? IPT_PN : IPT);
     g.iblocks = (nt + per_block - 1) / per_block;
-    const int64_t t = aster_slice_tiles(g.iblocks, (len + BLOCK - 1) / BLOCK, c->sm_count);
+    const int64_t tiles = (len + BLOCK - 1) / BLOCK, one = nt * (int64_t)sizeof(double4);  // sums of a slice
+    int64_t t = aster_slice_tiles(g.iblocks, tiles, c->sm_count);
+    if (precision == ASTER_MIXED && pnl < 2 && t == 1 && tiles * one > SUMS_LARGE && (tiles + 1) / 2 * one <= SUMS_SMALL)
+        t = 2;
     g.slice_len = std::max<int64_t>(t, 1) * BLOCK;
     g.ns = std::max<int64_t>(1, (len + g.slice_len - 1) / g.slice_len);  // no sources: one slice that writes zeros
     return g;

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from aster_b200 import gen
-from aster_b200.api import FP64, MIXED, NEWTON, PN1, SOLVER_ALLPAIRS, AsterError, Context, Params
+from aster_b200.api import FP64, MIXED, NEWTON, PN1, PN2, SOLVER_ALLPAIRS, AsterError, Context, Params
 from conftest import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -167,3 +167,19 @@ def test_sums_of_a_large_system_stay_within_the_limit():
         free = _free()
         c.allpairs(Params(eps2=1e-4), FP64)
         assert free - _free() <= 1026 * MB
+
+
+@pytest.mark.parametrize("n,law,kernels", [(2432, NEWTON, 1), (2433, NEWTON, 2), (2750, NEWTON, 2), (2750, NEWTON | PN1, 2),
+                                           (2750, NEWTON | PN1 | PN2, 1), (1700, NEWTON, 2)])
+def test_middle_sizes_take_slices_of_two_tiles(monkeypatch, n, law, kernels):
+    """Mixed forces, 2433 to 3072 bodies: the sums of 256-source slices fit into 1 MB, those of 128-source slices,
+    which the sizes below and the longer force laws take, do not (one launch less: no reduction)."""
+    pos, vel, m = gen.plummer(n, 47)
+    p = Params(eps2=1e-4, c=50.0, force_law=law)
+    with Context(0) as c:
+        ref = c.upload(pos, vel, m).allpairs(p, FP64)
+    monkeypatch.setenv("ASTER_SUMS_LIMIT", "1")
+    with Context(0) as c:
+        acc = c.upload(pos, vel, m).allpairs(p, MIXED)
+        assert c.stats()["kernels"] == kernels
+    assert rel_l2(acc, ref) < 1e-6
