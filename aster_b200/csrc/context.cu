@@ -10,13 +10,11 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 #include <new>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "aster_internal.cuh"
+#include "staged_copy.cuh"
 
 static thread_local char g_last_error[256] = "";
 static void release_graphs(aster_ctx* c);
@@ -281,59 +279,19 @@ __global__ void k_pack3(int64_t n, const double* __restrict__ src, double4* __re
     }
 }
 
-// ---- results to pageable host memory ------------------------------------------
-// A copy from the device into pageable memory goes through the driver's staging
-// on one thread, which also takes the page faults of a caller's freshly
-// allocated array: 19 MB (three arrays of 262,153 bodies) took 1.1 to 4.5 ms on
-// different hosts, and up to 2.4 more with the faults. Here the bytes come through
-// a page-locked slab in 1 MB pieces, and several threads copy them on (on the
-// slower host, memory reused / fresh: 4.5 -> 1.4 and 6.9 -> 1.6 ms; 75 MB of 2^20
-// bodies 13.0 -> 3.7 and 21.3 -> 5.0; two threads 2.5 and 8.1 ms). The slab is the process's (16 MB,
-// allocated by the first large copy, freed with the last context); a copy that
-// finds it in use takes the driver's way.
+// ---- results to pageable host memory (staged_copy.cuh) -------------------------
 namespace {
-constexpr size_t kPiece = (size_t)1 << 20;
-constexpr int kSlots = 16;
-constexpr int kTeam = 8;                     // threads at most (with 2 of the host's left over)
-// Below this the driver's copy is used: starting the threads costs some 0.2 ms,
-// as much as 2.4 MB take on a fast host.
-constexpr size_t kLeast = (size_t)6 << 20;
-struct Slab {
-    std::mutex mu;
-    void* base = nullptr;
-    bool busy = false, failed = false;
-    int contexts = 0;
-} g_slab;
-
-char* slab_take() {
-    std::lock_guard<std::mutex> lock(g_slab.mu);
-    if (g_slab.busy || g_slab.failed) return nullptr;
-    if (!g_slab.base && cudaHostAlloc(&g_slab.base, kPiece * kSlots, cudaHostAllocPortable) != cudaSuccess) {
+struct PageLocked {
+    static void* alloc(size_t bytes) {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess) return p;
         cudaGetLastError();
-        g_slab.base = nullptr;
-        g_slab.failed = true;
         return nullptr;
     }
-    g_slab.busy = true;
-    return static_cast<char*>(g_slab.base);
-}
-void slab_give_back() {
-    std::lock_guard<std::mutex> lock(g_slab.mu);
-    g_slab.busy = false;
-    if (g_slab.contexts == 0 && g_slab.base) {
-        cudaFreeHost(g_slab.base);
-        g_slab.base = nullptr;
-    }
-}
-void slab_contexts(int by) {
-    std::lock_guard<std::mutex> lock(g_slab.mu);
-    g_slab.contexts += by;
-    if (g_slab.contexts == 0 && !g_slab.busy && g_slab.base) {
-        cudaFreeHost(g_slab.base);
-        g_slab.base = nullptr;
-        g_slab.failed = false;
-    }
-}
+    static void free(void* p) { cudaFreeHost(p); }
+};
+staged::Slab<PageLocked> g_slab;
+void slab_contexts(int by) { g_slab.contexts(by); }
 
 bool page_locked(const void* p) {
     cudaPointerAttributes at{};
@@ -344,72 +302,23 @@ bool page_locked(const void* p) {
     return at.type != cudaMemoryTypeUnregistered;
 }
 
-struct Piece {
-    char* dst;
-    const char* src;
-    size_t bytes;
+// Copies on the context's stream, an event a slot.
+struct StreamCopies {
+    aster_ctx* c;
+    cudaError_t e = cudaSuccess;
+    bool issue(int slot, char* to, const staged::Piece& p) {
+        e = cudaMemcpyAsync(to, p.src, p.bytes, cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = cudaEventRecord(c->dl_ev[slot], c->stream);
+        return e == cudaSuccess;
+    }
+    bool wait(int slot) { return (e = cudaEventSynchronize(c->dl_ev[slot])) == cudaSuccess; }
 };
 
-// The pieces through the slab, in order; returns when all have arrived.
-int staged_copy(aster_ctx* c, const std::vector<Piece>& pieces, char* slab) {
-    const int n = (int)pieces.size();
-    for (int k = 0; k < kSlots; ++k)
+int staged_copy(aster_ctx* c, const std::vector<staged::Piece>& pieces, char* slab) {
+    for (int k = 0; k < staged::kSlots; ++k)
         if (!c->dl_ev[k]) ASTER_CUDA(cudaEventCreateWithFlags(&c->dl_ev[k], cudaEventDisableTiming));
-    std::atomic<int> ready{0}, taken{0};
-    std::atomic<bool> stop{false};
-    std::vector<std::atomic<bool>> done(n);
-    for (auto& d : done) d.store(false, std::memory_order_relaxed);
-    auto copy_next = [&](bool wait) -> bool {  // one piece; false: none left (or, without wait, none ready)
-        int k = taken.load();
-        do {
-            if (k >= n || (!wait && k >= ready.load())) return false;
-        } while (!taken.compare_exchange_weak(k, k + 1));
-        while (ready.load(std::memory_order_acquire) <= k) {
-            if (stop.load()) return false;
-            std::this_thread::yield();
-        }
-        std::memcpy(pieces[k].dst, slab + (size_t)(k % kSlots) * kPiece, pieces[k].bytes);
-        done[k].store(true, std::memory_order_release);
-        return true;
-    };
-    std::vector<std::thread> team;
-    cudaError_t e = cudaSuccess;
-    int issued = 0, arrived = 0;
-    auto issue = [&]() {
-        for (; issued < n && e == cudaSuccess && (issued < kSlots || done[issued - kSlots].load(std::memory_order_acquire));
-             ++issued) {
-            e = cudaMemcpyAsync(slab + (size_t)(issued % kSlots) * kPiece, pieces[issued].src, pieces[issued].bytes,
-                                cudaMemcpyDeviceToHost, c->stream);
-            if (e == cudaSuccess) e = cudaEventRecord(c->dl_ev[issued % kSlots], c->stream);
-        }
-    };
-    issue();
-    const unsigned hw = std::thread::hardware_concurrency();
-    const int want = std::min<int>({n - 1, (int)(hw > 2 ? hw - 2 : 0), kTeam - 1});
-    team.reserve(std::max(want, 0));
-    try {
-        for (int k = 0; k < want; ++k)
-            team.emplace_back([&]() {
-                while (copy_next(true)) {
-                }
-            });
-    } catch (const std::system_error&) {  // fewer threads
-    }
-    while (arrived < n && e == cudaSuccess) {
-        issue();
-        if (e != cudaSuccess) break;
-        if (arrived < issued) {
-            e = cudaEventSynchronize(c->dl_ev[arrived % kSlots]);
-            if (e == cudaSuccess) ready.store(++arrived, std::memory_order_release);
-        } else if (!copy_next(false)) {
-            std::this_thread::yield();  // every slot is being copied on
-        }
-    }
-    if (e != cudaSuccess) stop.store(true);
-    while (e == cudaSuccess && copy_next(true)) {
-    }
-    for (std::thread& t : team) t.join();
-    return e == cudaSuccess ? ASTER_OK : aster_cuda_fail(e, "staged copy", __FILE__, __LINE__);
+    StreamCopies dev{c};
+    return staged::copy(dev, pieces, slab) ? ASTER_OK : aster_cuda_fail(dev.e, "staged copy", __FILE__, __LINE__);
 }
 }  // namespace
 
@@ -419,20 +328,20 @@ int aster_copy_to_host(aster_ctx* c, void* const* dst, const void* const* src, c
     size_t total = 0;
     for (int k = 0; k < count; ++k)
         if (dst[k] && !page_locked(dst[k])) total += bytes[k];
-    char* slab = total >= kLeast ? slab_take() : nullptr;
+    char* slab = total >= staged::kLeast ? g_slab.take() : nullptr;
     int st = ASTER_OK;
     if (slab) {
         try {
-            std::vector<Piece> pieces;
+            std::vector<staged::Piece> pieces;
             for (int k = 0; k < count; ++k)
-                for (size_t o = 0; dst[k] && o < bytes[k]; o += kPiece)
-                    pieces.push_back({(char*)dst[k] + o, (const char*)src[k] + o, std::min(kPiece, bytes[k] - o)});
+                for (size_t o = 0; dst[k] && o < bytes[k]; o += staged::kPiece)
+                    pieces.push_back({(char*)dst[k] + o, (const char*)src[k] + o, std::min(staged::kPiece, bytes[k] - o)});
             st = staged_copy(c, pieces, slab);
         } catch (const std::bad_alloc&) {
             st = ASTER_ERR_OOM;
         }
         if (st != ASTER_OK) cudaStreamSynchronize(c->stream);  // nothing may still write the slab
-        slab_give_back();
+        g_slab.give_back();
         if (st != ASTER_ERR_OOM) return st;
     }
     for (int k = 0; k < count; ++k)

@@ -1,0 +1,24 @@
+"""The staging of large results on the host (aster_b200/csrc/staged_copy.cuh),
+compiled alone with copies and allocations of its own: memory that runs out while
+the threads start, and copies that fail, end in a whole result or in an error,
+never in the process's end."""
+import subprocess
+from pathlib import Path
+
+import pytest
+
+SRC = Path(__file__).with_name("host") / "staged_copy_harness.cpp"
+
+
+@pytest.fixture(scope="module")
+def harness(tmp_path_factory):
+    out = tmp_path_factory.mktemp("staged") / "harness"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", str(SRC), "-o", str(out)], check=True)
+    return out
+
+
+@pytest.mark.parametrize("what", ["memory", "device"])
+@pytest.mark.parametrize("pieces", [1, 7, 16, 17, 40])
+def test_staged_copy(harness, what, pieces):
+    r = subprocess.run([str(harness), what, str(pieces)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout == "ok\n", (r.returncode, r.stdout, r.stderr)
