@@ -56,9 +56,8 @@ public:
     }
 
 private:
-    void drop() {
-        if (!base_) return;
-        Host::free(base_);
+    void drop() {  // (the next contexts may have the memory that these did not get)
+        if (base_) Host::free(base_);
         base_ = nullptr;
         failed_ = false;
     }

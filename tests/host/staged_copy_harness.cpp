@@ -2,6 +2,7 @@
 // of by a device, and allocations that can be made to fail. One command a run:
 //   memory N   for k = 0, 1, ..: the k-th allocation after the first copy was
 //              issued fails; every copy of N pieces must arrive whole all the same
+//   slab 0     the slab's life: refused, in use, given back, freed with the last context
 //   device N   for k = 0, 1, ..: the k-th copy, then the k-th wait, fails: reported
 // Prints "ok" and exits 0, or says what was wrong.
 #include <cstdio>
@@ -40,10 +41,56 @@ struct Fake {
     }
 };
 
+static bool g_refuse = false;
+static int g_held = 0;
+struct FakeHost {
+    static void* alloc(size_t n) {
+        if (g_refuse) return nullptr;
+        ++g_held;
+        return std::malloc(n);
+    }
+    static void free(void* p) {
+        --g_held;
+        std::free(p);
+    }
+};
+static int slab_life() {
+#define WANT(x)                                              \
+    do {                                                     \
+        if (!(x)) return std::printf("not so: %s\n", #x), 1; \
+    } while (0)
+    staged::Slab<FakeHost> s;
+    s.contexts(1);
+    s.contexts(1);
+    WANT(s.take() && g_held == 1);
+    WANT(!s.take());  // in use
+    s.contexts(-1);
+    s.give_back();
+    WANT(g_held == 1 && s.take());
+    s.contexts(-1);
+    WANT(g_held == 1);  // still in use
+    s.give_back();
+    WANT(g_held == 0);
+    g_refuse = true;
+    s.contexts(1);
+    WANT(!s.take());
+    g_refuse = false;
+    WANT(!s.take());  // not asked for again by these contexts
+    s.contexts(-1);
+    s.contexts(1);
+    WANT(s.take() && g_held == 1);  // by the next ones it is
+    s.give_back();
+    s.contexts(-1);
+    WANT(g_held == 0);
+    std::printf("ok\n");
+    return 0;
+}
+
 int main(int argc, char** argv) {
     if (argc != 3) return 2;
     const std::string what = argv[1];
     const int n = std::atoi(argv[2]);
+    if (what == "slab") return slab_life();
     const size_t bytes = (size_t)n * staged::kPiece - 12345;
     std::vector<char> src(bytes), dst(bytes), slab(staged::kPiece * staged::kSlots);
     for (size_t k = 0; k < bytes; ++k) src[k] = (char)(k * 2654435761u >> 11);

@@ -22,3 +22,8 @@ def harness(tmp_path_factory):
 def test_staged_copy(harness, what, pieces):
     r = subprocess.run([str(harness), what, str(pieces)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == "ok\n", (r.returncode, r.stdout, r.stderr)
+
+
+def test_slab_is_asked_for_again_by_later_contexts(harness):
+    r = subprocess.run([str(harness), "slab", "0"], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and r.stdout == "ok\n", (r.returncode, r.stdout, r.stderr)
