@@ -325,27 +325,36 @@ int staged_copy(aster_ctx* c, const std::vector<staged::Piece>& pieces, char* sl
 // Device arrays -> host arrays (null destinations skipped) after the work
 // queued on the context's stream; synchronised when it returns.
 int aster_copy_to_host(aster_ctx* c, void* const* dst, const void* const* src, const size_t* bytes, int count) {
+    constexpr int MOST = 4;
+    bool pageable[MOST];
+    if (count > MOST) return ASTER_ERR_INVALID_ARG;
     size_t total = 0;
-    for (int k = 0; k < count; ++k)
-        if (dst[k] && !page_locked(dst[k])) total += bytes[k];
-    char* slab = total >= staged::kLeast ? g_slab.take() : nullptr;
-    int st = ASTER_OK;
+    for (int k = 0; k < count; ++k) {
+        pageable[k] = dst[k] && !page_locked(dst[k]);
+        if (pageable[k]) total += bytes[k];
+    }
+    auto direct = [&](bool which) -> int {  // the pageable ones, or the others
+        for (int k = 0; k < count; ++k)
+            if (dst[k] && pageable[k] == which)
+                ASTER_CUDA(cudaMemcpyAsync(dst[k], src[k], bytes[k], cudaMemcpyDeviceToHost, c->stream));
+        return ASTER_OK;
+    };
+    int st = direct(false);
+    char* slab = st == ASTER_OK && total >= staged::kLeast ? g_slab.take() : nullptr;
+    bool rest = total > 0;
     if (slab) {
         try {
-            std::vector<staged::Piece> pieces;
-            for (int k = 0; k < count; ++k)
-                for (size_t o = 0; dst[k] && o < bytes[k]; o += staged::kPiece)
-                    pieces.push_back({(char*)dst[k] + o, (const char*)src[k] + o, std::min(staged::kPiece, bytes[k] - o)});
-            st = staged_copy(c, pieces, slab);
+            st = staged_copy(c, staged::pieces_of(dst, src, bytes, pageable, count), slab);
         } catch (const std::bad_alloc&) {
             st = ASTER_ERR_OOM;
         }
         if (st != ASTER_OK) cudaStreamSynchronize(c->stream);  // nothing may still write the slab
         g_slab.give_back();
-        if (st != ASTER_ERR_OOM) return st;
+        rest = st == ASTER_ERR_OOM;
+        if (rest) st = ASTER_OK;
     }
-    for (int k = 0; k < count; ++k)
-        if (dst[k]) ASTER_CUDA(cudaMemcpyAsync(dst[k], src[k], bytes[k], cudaMemcpyDeviceToHost, c->stream));
+    if (st == ASTER_OK && rest) st = direct(true);
+    ASTER_TRY(st);
     ASTER_CUDA(cudaStreamSynchronize(c->stream));
     return ASTER_OK;
 }

@@ -73,6 +73,17 @@ struct Piece {
     size_t bytes;
 };
 
+// The pieces of those arrays whose destination is pageable (null destinations
+// skipped): the others take one direct copy each.
+inline std::vector<Piece> pieces_of(void* const* dst, const void* const* src, const size_t* bytes, const bool* pageable,
+                                    int count) {
+    std::vector<Piece> p;
+    for (int k = 0; k < count; ++k)
+        for (size_t o = 0; dst[k] && pageable[k] && o < bytes[k]; o += kPiece)
+            p.push_back({(char*)dst[k] + o, (const char*)src[k] + o, std::min(kPiece, bytes[k] - o)});
+    return p;
+}
+
 // The pieces through the slab, in order. Dev: bool issue(slot, to, piece) starts
 // the copy of a piece's bytes to `to`, bool wait(slot) returns when it has
 // arrived; false: failed. Returns whether all have arrived at their

@@ -3,6 +3,7 @@
 //   memory N   for k = 0, 1, ..: the k-th allocation after the first copy was
 //              issued fails; every copy of N pieces must arrive whole all the same
 //   slab 0     the slab's life: refused, in use, given back, freed with the last context
+//   pieces 0   which arrays are cut, and how
 //   device N   for k = 0, 1, ..: the k-th copy, then the k-th wait, fails: reported
 // Prints "ok" and exits 0, or says what was wrong.
 #include <cstdio>
@@ -86,11 +87,37 @@ static int slab_life() {
     return 0;
 }
 
+static int pieces_of_arrays() {
+    static char a[3 * staged::kPiece], b[10], x[3 * staged::kPiece], y[10];
+    void* const dst[4] = {x, y, nullptr, x};
+    const void* const src[4] = {a, b, a, a};
+    const size_t bytes[4] = {2 * staged::kPiece + 5, 10, 7, 2 * staged::kPiece};
+    for (int m = 0; m < 16; ++m) {
+        const bool pageable[4] = {(m & 1) != 0, (m & 2) != 0, (m & 4) != 0, (m & 8) != 0};
+        size_t got[4] = {0, 0, 0, 0}, want = 0, sum = 0;
+        const auto p = staged::pieces_of(dst, src, bytes, pageable, 4);
+        int at = 0;  // pieces come in the arrays' order
+        for (const auto& q : p) {
+            while (at < 4 && (!pageable[at] || !dst[at] || got[at] == bytes[at])) ++at;
+            WANT(at < 4 && q.dst == (char*)dst[at] + got[at] && q.src == (const char*)src[at] + got[at]);
+            WANT(q.bytes > 0 && q.bytes <= staged::kPiece);
+            got[at] += q.bytes;
+            sum += q.bytes;
+        }
+        for (int k = 0; k < 4; ++k)
+            if (pageable[k] && dst[k]) want += bytes[k];
+        WANT(sum == want);
+    }
+    std::printf("ok\n");
+    return 0;
+}
+
 int main(int argc, char** argv) {
     if (argc != 3) return 2;
     const std::string what = argv[1];
     const int n = std::atoi(argv[2]);
     if (what == "slab") return slab_life();
+    if (what == "pieces") return pieces_of_arrays();
     const size_t bytes = (size_t)n * staged::kPiece - 12345;
     std::vector<char> src(bytes), dst(bytes), slab(staged::kPiece * staged::kSlots);
     for (size_t k = 0; k < bytes; ++k) src[k] = (char)(k * 2654435761u >> 11);

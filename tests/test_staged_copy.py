@@ -27,3 +27,29 @@ def test_staged_copy(harness, what, pieces):
 def test_slab_is_asked_for_again_by_later_contexts(harness):
     r = subprocess.run([str(harness), "slab", "0"], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0 and r.stdout == "ok\n", (r.returncode, r.stdout, r.stderr)
+
+
+def test_only_pageable_destinations_are_staged(harness):
+    r = subprocess.run([str(harness), "pieces", "0"], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and r.stdout == "ok\n", (r.returncode, r.stdout, r.stderr)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("locked", [(), (0,), (1, 2), (0, 1, 2)])
+@pytest.mark.parametrize("n", [1000, 262153])
+def test_mixed_destinations_arrive_whole(locked, n):
+    import ctypes
+
+    import numpy as np
+    import torch
+
+    from aster_b200.api import Context
+    rng = np.random.default_rng(5)
+    pos, vel, m = rng.normal(size=(n, 3)), rng.normal(size=(n, 3)), rng.uniform(1, 2, n)
+    out = [torch.full((n, 3), float("nan"), dtype=torch.float64, pin_memory=k in locked).numpy() for k in range(3)]
+    with Context(0) as c:
+        c.upload(pos, vel, m)
+        assert c.lib.aster_state_download(c.h, *[ctypes.c_void_p(o.ctypes.data) for o in out]) == 0
+    np.testing.assert_array_equal(out[0], pos)
+    np.testing.assert_array_equal(out[1], vel)
+    assert not out[2].any()
