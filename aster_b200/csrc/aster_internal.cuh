@@ -161,9 +161,9 @@ struct aster_ctx {
     // executable graphs of the last call's repeated steps; destroyed by the
     // next call's aster_begin (its work has finished by then) or at destroy
     std::vector<std::pair<cudaGraph_t, cudaGraphExec_t>> graphs;
-    // the KDK's middle step (forces with the next kick and drift), kept across calls;
-    // a replaced one moves to `graphs`
-    StepGraph kdk_graph;
+    // the KDK's middle step (forces with the next kick and drift) of either solver
+    // (ASTER_SOLVER_*), kept across calls; a replaced one moves to `graphs`
+    StepGraph kdk_graph[2];
 };
 
 // Layout of ctx->red (4 KB of small device scalars).

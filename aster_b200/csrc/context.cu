@@ -143,9 +143,11 @@ extern "C" int aster_ctx_destroy(aster_ctx* c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     release_graphs(c);
-    if (c->kdk_graph.ge) cudaGraphExecDestroy(c->kdk_graph.ge);
-    if (c->kdk_graph.g) cudaGraphDestroy(c->kdk_graph.g);
-    if (c->kdk_graph.park) cudaEventDestroy(c->kdk_graph.park);
+    for (StepGraph& sg : c->kdk_graph) {
+        if (sg.ge) cudaGraphExecDestroy(sg.ge);
+        if (sg.g) cudaGraphDestroy(sg.g);
+        if (sg.park) cudaEventDestroy(sg.park);
+    }
     DevBuf* bufs[] = {&c->pm, &c->vel, &c->acc, &c->phi, &c->plo, &c->vf, &c->scratch, &c->targets,
                       &c->stage, &c->red, &c->wh, &c->rec,
                       &c->tree.codes, &c->tree.codes_alt, &c->tree.sorted_codes, &c->tree.perm,
