@@ -146,6 +146,10 @@ struct aster_ctx {
     // usable tree-walk stack entries per warp (<= the 1024 in shared memory);
     // ASTER_WALK_STACK_LIMIT lowers it, e.g. to exercise the overflow path
     int walk_stack_limit = 1024;
+    // largest tree that the walk by a block per group may take (where it is the
+    // faster one); ASTER_WALK_TEAM_LIMIT lowers it, so that the one-warp walk of
+    // the larger trees can be checked on small ones
+    int64_t walk_team_limit = INT64_MAX;
     LbvhBufs tree;
     EnsBufs ens;
     AdjBufs adj;

@@ -129,6 +129,10 @@ extern "C" int aster_ctx_create(aster_ctx** out, int device, void* stream) {
         const int v = std::atoi(lim);
         if (v >= 64 && v < c->walk_stack_limit) c->walk_stack_limit = v;
     }
+    if (const char* lim = std::getenv("ASTER_WALK_TEAM_LIMIT")) {
+        const long long v = std::atoll(lim);
+        if (v >= 0) c->walk_team_limit = v;
+    }
     if (const char* lim = std::getenv("ASTER_SUMS_LIMIT")) {
         const long long v = std::atoll(lim);
         if (v >= 0 && v < 100000) c->sums_limit = (size_t)v << 20;

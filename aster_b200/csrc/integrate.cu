@@ -348,7 +348,7 @@ static std::vector<unsigned char> step_key(const aster_ctx* c, const aster_param
     std::vector<unsigned char> k(sizeof(aster_params));
     std::memcpy(k.data(), p, sizeof(aster_params));
     const int64_t w[] = {solver, precision, timed ? 1 : 0, c->n, c->n_src, (int64_t)c->sums_oom, c->device,
-                         c->walk_stack_limit, (int64_t)aster_devbuf_epoch()};
+                         c->walk_stack_limit, c->walk_team_limit, (int64_t)aster_devbuf_epoch()};
     const unsigned char* wb = reinterpret_cast<const unsigned char*>(w);
     k.insert(k.end(), wb, wb + sizeof(w));
     return k;

@@ -2143,7 +2143,7 @@ int launch_team(aster_ctx* c, const aster_params* p, int32_t* counts, bool fuse_
 template <bool MIXED, bool GUARD, bool KICK, int PNL = 0>
 int launch_walk(aster_ctx* c, const aster_params* p, int32_t* counts, bool fuse_next) {
     LbvhBufs& t = c->tree;
-    if (c->n <= (MIXED ? TEAM_MAX_MIXED : TEAM_MAX_FP64))
+    if (c->n <= std::min(c->walk_team_limit, MIXED ? TEAM_MAX_MIXED : TEAM_MAX_FP64))
         return launch_team<MIXED, GUARD, KICK, PNL>(c, p, counts, fuse_next);
     auto kern = k_walk<MIXED, GUARD, KICK, PNL>;
     int per_sm = 0;
