@@ -67,8 +67,9 @@ __device__ __forceinline__ void store_result(int64_t t, int64_t body, double ax,
 }
 
 // ---------------------------------------------------------------- FP64 path
-// PNL: 0 Newton, 1 Newton + 1PN, 2 Newton + the PN terms pk.f selects.
-template <int PNL, bool GUARD>
+// PNL: 0 Newton, 1 Newton + 1PN, 2 Newton + the PN terms pk.f selects. (A zero
+// distance contributes nothing, softened or not: fp64_pair.cuh.)
+template <int PNL>
 __global__ void __launch_bounds__(BLOCK) k_allpairs_fp64(
     int64_t j_lo, int64_t n, int64_t nt, const int32_t* __restrict__ targets, const double4* __restrict__ pm,
     const double4* __restrict__ vel, double G, double eps2, PnK<double> pk, int64_t slice_len, int nslices,
@@ -367,12 +368,12 @@ __global__ void __launch_bounds__(256) k_reduce_slices(int64_t nt, int nslices, 
     if (k < 3) *vp = v;
 }
 
-template <int PNL, bool GUARD>
+template <int PNL>
 void launch_fp64(dim3 grid, cudaStream_t st, int64_t j_lo, int64_t n, int64_t nt, const int32_t* tg, aster_ctx* c,
                  const aster_params* p, int64_t slice_len, int ns, double4* partial, double* out3, KickArgs kick) {
-    k_allpairs_fp64<PNL, GUARD><<<grid, BLOCK, 0, st>>>(j_lo, n, nt, tg, c->pm.as<double4>(), c->vel.as<double4>(), p->G,
-                                                         p->eps2, make_pn(p), slice_len, ns, partial,
-                                                         c->acc.as<double4>(), out3, kick);
+    k_allpairs_fp64<PNL><<<grid, BLOCK, 0, st>>>(j_lo, n, nt, tg, c->pm.as<double4>(), c->vel.as<double4>(), p->G,
+                                                  p->eps2, make_pn(p), slice_len, ns, partial, c->acc.as<double4>(),
+                                                  out3, kick);
 }
 
 template <int PNL, bool GUARD>
@@ -395,8 +396,7 @@ void launch_pnl(int precision, bool guard, dim3 grid, cudaStream_t st, int64_t j
                 aster_ctx* c, const aster_params* p, int64_t slice_len, int ns, double4* partial, double* out3,
                 KickArgs kick) {
     if (precision == ASTER_FP64) {
-        if (guard) launch_fp64<PNL, true>(grid, st, j_lo, n, nt, tg, c, p, slice_len, ns, partial, out3, kick);
-        else       launch_fp64<PNL, false>(grid, st, j_lo, n, nt, tg, c, p, slice_len, ns, partial, out3, kick);
+        launch_fp64<PNL>(grid, st, j_lo, n, nt, tg, c, p, slice_len, ns, partial, out3, kick);
     } else {
         if (guard) launch_mixed<PNL, true>(grid, st, j_lo, n, nt, tg, c, p, slice_len, ns, partial, out3, kick);
         else       launch_mixed<PNL, false>(grid, st, j_lo, n, nt, tg, c, p, slice_len, ns, partial, out3, kick);

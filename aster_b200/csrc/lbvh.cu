@@ -1224,8 +1224,8 @@ __device__ __forceinline__ bool walk_r2_ordinary(int64_t n, const float4* __rest
            1e30f;
 }
 
-// One entry with a post-Newtonian force law, FP64: the Newtonian term as
-// interact_f64 forms it plus the terms pk selects (pn.cuh), all divided by G.
+// One entry with a post-Newtonian force law, FP64: the Newtonian term and the
+// terms pk selects (pn.cuh), all divided by G.
 // Entry e (position, mass; velocity ev) acts on the body b (velocity vi).
 template <int PNL>
 __device__ __forceinline__ void interact_pn_f64(const double4 e, const double4 ev, const double4 b, const double4 vi,
@@ -1355,7 +1355,8 @@ __device__ __forceinline__ float2 box_dist2_pair(const float2 cx, const float2 c
 // interaction needs one subtraction per axis; the group is compact, so the
 // relative coordinates keep FP32 precision of the separation.
 // PNL > 0: the post-Newtonian walk (the terms pk selects, with the nodes'
-// velocities node_v); PNL == 0 is the Newtonian kernel.
+// velocities node_v); PNL == 0 is the Newtonian kernel. GUARD (mixed): unsoftened,
+// a zero distance contributes nothing (the FP64 sums see to that by themselves).
 template <bool MIXED, bool GUARD, bool KICK, int PNL = 0>
 __global__ void __launch_bounds__(WALK_WARPS * 32, PNL ? 4 : ASTER_WALK_MINBLOCKS) k_walk(
     int64_t n, const int2* __restrict__ groups, const unsigned int* __restrict__ ngroups_p,
@@ -2114,11 +2115,11 @@ __global__ void __launch_bounds__(TeamSize<MIXED, PNL>::WARPS * 32, TeamSize<MIX
 // 20,011: 125, 66; 60,000: 196, 135; 100,000: 238, 201; 131,073: 244, 248;
 // 262,144: 432, 480. FP64 5000: 164, 64; 20,011: 225, 98; 60,000: 391, 236;
 // 131,073: 580, 492; 262,144: 942, 948; 1,048,576: 3556, 4002. 1PN mixed 3000:
-// 253, 117; 20,011: 475, 191; 60,000: 597, 370; 119,000: 689, 629; FP64 20,011:
-// 1066, 399; 119,000: 1685, 1527; 190,000: 2490, 2396. Every term, mixed 20,011:
-// 1177, 437; 119,000: 1766, 1572; FP64 20,011: 2237, 804; 190,000: 5588, 5020
-// (FP64 figures from before its pair terms were gathered, which took a fifth to a
-// third off both walks).
+// 183, 120; 20,011: 429, 191; 60,000: 595, 366; 119,000: 681, 622; FP64 20,011:
+// 796, 386; 119,000: 1465, 1379; 190,000: 2274, 2178. Every term, mixed 20,011:
+// 867, 419; 119,000: 1738, 1521; FP64 20,011: 1355, 597; 119,000: 2749, 2266;
+// 190,000: 3942, 3599. (At theta = 0.8 the two meet somewhat earlier: Newton mixed
+// 119,000 113, 119, FP64 190,000 309, 332.)
 constexpr int64_t TEAM_MAX_MIXED = 120000, TEAM_MAX_FP64 = 200000;
 
 template <bool MIXED, bool GUARD, bool KICK, int PNL>
@@ -2396,8 +2397,7 @@ int aster_lbvh_walk_launch(aster_ctx* c, const aster_params* p, int precision, b
             if (guard) { ASTER_TRY(kick ? launch_walk<true, true, true, 2>(c, p, counts, fuse_next) : launch_walk<true, true, false, 2>(c, p, counts, fuse_next)); }
             else       { ASTER_TRY(kick ? launch_walk<true, false, true, 2>(c, p, counts, fuse_next) : launch_walk<true, false, false, 2>(c, p, counts, fuse_next)); }
         } else {
-            if (guard) { ASTER_TRY(kick ? launch_walk<false, true, true, 2>(c, p, counts, fuse_next) : launch_walk<false, true, false, 2>(c, p, counts, fuse_next)); }
-            else       { ASTER_TRY(kick ? launch_walk<false, false, true, 2>(c, p, counts, fuse_next) : launch_walk<false, false, false, 2>(c, p, counts, fuse_next)); }
+            ASTER_TRY(kick ? launch_walk<false, false, true, 2>(c, p, counts, fuse_next) : launch_walk<false, false, false, 2>(c, p, counts, fuse_next));
         }
         c->stats.kernels += 1;
         return ASTER_OK;
@@ -2406,8 +2406,7 @@ int aster_lbvh_walk_launch(aster_ctx* c, const aster_params* p, int precision, b
         if (guard) { ASTER_TRY(kick ? launch_walk<true, true, true>(c, p, counts, fuse_next) : launch_walk<true, true, false>(c, p, counts, fuse_next)); }
         else       { ASTER_TRY(kick ? launch_walk<true, false, true>(c, p, counts, fuse_next) : launch_walk<true, false, false>(c, p, counts, fuse_next)); }
     } else {
-        if (guard) { ASTER_TRY(kick ? launch_walk<false, true, true>(c, p, counts, fuse_next) : launch_walk<false, true, false>(c, p, counts, fuse_next)); }
-        else       { ASTER_TRY(kick ? launch_walk<false, false, true>(c, p, counts, fuse_next) : launch_walk<false, false, false>(c, p, counts, fuse_next)); }
+        ASTER_TRY(kick ? launch_walk<false, false, true>(c, p, counts, fuse_next) : launch_walk<false, false, false>(c, p, counts, fuse_next));
     }
     c->stats.kernels += 1;
     return ASTER_OK;
