@@ -69,6 +69,13 @@ __device__ __forceinline__ void store_result(int64_t t, int64_t body, double ax,
 // ---------------------------------------------------------------- FP64 path
 // PNL: 0 Newton, 1 Newton + 1PN, 2 Newton + the PN terms pk.f selects. (A zero
 // distance contributes nothing, softened or not: fp64_pair.cuh.)
+// Newtonian sums take DQ sources at a time. With a range test and branch a pair,
+// few targets or sources, which leave a scheduler a warp or two, wait for every
+// pair's chain in turn: 100 targets among 50,000 bodies 174 us, 110 with four
+// sources a branch (two: 110), among 300,000 739 -> 379 (407); a KDK step of 100
+// bodies 18.6 -> 12.4 us; 100,000 massless bodies of 200,000, where the FP64 pipe
+// bounds it, 21.6 -> 20.2 ms (20.7). The terms and their order are the same.
+constexpr int DQ = 4;
 template <int PNL>
 __global__ void __launch_bounds__(BLOCK) k_allpairs_fp64(
     int64_t j_lo, int64_t n, int64_t nt, const int32_t* __restrict__ targets, const double4* __restrict__ pm,
@@ -106,8 +113,48 @@ __global__ void __launch_bounds__(BLOCK) k_allpairs_fp64(
         }
         __syncthreads();
         const int cnt = (int)min((int64_t)BLOCK, j1 - base);  // a partial last tile stops at its last source
-#pragma unroll 8
-        for (int q = 0; q < cnt; ++q) {
+        int q = 0;
+        if (PNL == 0) {  // DQ sources at a time: their chains overlap, with one branch for all
+#pragma unroll 1
+            for (; q + DQ <= cnt; q += DQ) {
+                double dx[DQ][IPT], dy[DQ][IPT], dz[DQ][IPT], s[DQ][IPT];
+                bool odd = false;
+#pragma unroll
+                for (int u = 0; u < DQ; ++u) {
+                    const double4 pj = sp[q + u];
+#pragma unroll
+                    for (int k = 0; k < IPT; ++k) {
+                        dx[u][k] = pj.x - xi[k]; dy[u][k] = pj.y - yi[k]; dz[u][k] = pj.z - zi[k];
+                        const double r2 = fma(dx[u][k], dx[u][k], fma(dy[u][k], dy[u][k], fma(dz[u][k], dz[u][k], eps2)));
+                        s[u][k] = pj.w * inv_r3_fast(r2);
+                        odd = odd || !r2_ordinary(r2);
+                    }
+                }
+                if (odd) {
+#pragma unroll 1
+                    for (int u = 0; u < DQ; ++u) {
+                        const double4 pj = sp[q + u];
+#pragma unroll
+                        for (int k = 0; k < IPT; ++k) {
+                            const double x = pj.x - xi[k], y = pj.y - yi[k], z = pj.z - zi[k];
+                            const double t = m_inv_r3(pj.w, fma(x, x, fma(y, y, fma(z, z, eps2))));
+                            ax[k] = fma(x, t, ax[k]); ay[k] = fma(y, t, ay[k]); az[k] = fma(z, t, az[k]);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int u = 0; u < DQ; ++u)
+#pragma unroll
+                        for (int k = 0; k < IPT; ++k) {
+                            ax[k] = fma(dx[u][k], s[u][k], ax[k]);
+                            ay[k] = fma(dy[u][k], s[u][k], ay[k]);
+                            az[k] = fma(dz[u][k], s[u][k], az[k]);
+                        }
+                }
+            }
+        }
+#pragma unroll (PNL ? 8 : 1)
+        for (; q < cnt; ++q) {
             const double4 pj = sp[q];
 #pragma unroll
             for (int k = 0; k < IPT; ++k) {
