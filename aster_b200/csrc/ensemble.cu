@@ -862,8 +862,12 @@ extern "C" int aster_ensemble_run(aster_ctx* c, const aster_params* p, int integ
     if (precision != ASTER_FP64 && precision != ASTER_MIXED) return ASTER_ERR_INVALID_ARG;
     int wpb = cfg && cfg->warps_per_block ? cfg->warps_per_block : 4;
     // the flagged PN terms' and EIH's loop bodies are long: 16,384 systems, 40 mixed steps, unroll 1 / 2 / 4:
-    // every PN term 14.6 / 17.2 / 22.4 ms, EIH 8.7 / 9.9 / 11.5; 1PN 5.84 / 5.83 / 6.33, Newton 2.83 / 2.59 / 2.61
-    int unroll = cfg && cfg->unroll ? cfg->unroll : pnl >= 2 ? 1 : 2;
+    // every PN term 14.6 / 17.2 / 22.4 ms, EIH 8.7 / 9.9 / 11.5; 1PN 5.84 / 5.83 / 6.33, Newton 2.83 / 2.59 / 2.61.
+    // With few systems a warp has its SM's pipes almost to itself and EIH's two loops a body overlap: 20 steps of
+    // systems of 3 to 64 bodies, unroll 1 / 2, us: 64 systems FP64 2242 / 2084, mixed 738 / 647; 1200 2580 / 2408 and
+    // 1060 / 964; 2400 3538 / 3482 and 1532 / 1601; 4800 3882 / 4061 and 1741 / 1866. (Every unrolling gives the same bits.)
+    const bool few = c->ens.nsys <= 16 * c->sm_count;
+    int unroll = cfg && cfg->unroll ? cfg->unroll : pnl == 2 || (pnl == 3 && !few) ? 1 : 2;
     int check = cfg && cfg->check_every ? cfg->check_every : 256;
     // stream capture is not possible on the legacy default stream
     bool graph = (cfg ? cfg->use_graph != 0 : true) && c->stream != nullptr;

@@ -279,8 +279,11 @@ int aster_energy(aster_ctx* ctx, const aster_params* p, int ref_form, double* en
 typedef struct aster_ensemble_config {
     int32_t warps_per_block; /* 1..16 (0: 4)                                  */
     int32_t unroll;          /* inner-loop unroll 1, 2 or 4 (0: 2, or 1 with
-                                2PN, 2.5PN or EIH terms)                    */
-    int32_t check_every;     /* steps between cancel-flag reads (0: 256)      */
+                                2PN or 2.5PN terms and, past some 2,400
+                                systems, with EIH; the results are the same) */
+    int32_t check_every;     /* steps of a system between looks at the cancel
+                                flag (0: 256); the host's flag itself is read
+                                at most every 20 us, for all systems         */
     int32_t use_graph;       /* 1: capture the launch in a CUDA graph         */
     int32_t schedule;        /* order warps take systems in: 0 largest first
                                 (longest-processing-time), 1 upload order     */
