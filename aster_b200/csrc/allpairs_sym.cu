@@ -297,8 +297,9 @@ int launch_sym(aster_ctx* c, const SymArgs& g) {
 // 1.31 ms (4 bodies per lane). Beyond 349,525 bodies fewer slots fit: 699,050 with
 // 128 / 64 / 24 slots 342 / 353 / 386 ms, 2^20 with 128 / 42 / 24 765 / 831 / 946.
 // Fewer than SYM_SLOTS_MIN are fewer tile pairs than resident blocks, and the
-// directed kernel is as fast: 2^20 with 20 slots 1239 ms, directed 1243; 1PN at
-// 524,289 604 ms with 128 slots, 690 with 24, 962 with 20, directed 873.
+// directed kernel is faster: 2^20 with 20 slots 1239 ms, directed 1141; 524,289
+// with 24 slots 221, with 20 308, directed 291; 1PN there 604 ms with 128 slots,
+// 688 with 24, 962 with 20, directed 872.
 constexpr int SYM_SLOTS = 128, SYM_SLOTS_MIN = 24;
 // Smaller systems take tiles of 64 bodies (2 per lane, 2 warps), larger ones
 // of 256 (8 per lane, 4 warps; 1PN 128 and 4): Newton at 4096 bodies 0.033

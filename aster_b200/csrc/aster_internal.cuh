@@ -26,9 +26,10 @@
 // come out even and the last blocks are short. Mixed forces, us, with the slices
 // that give 12 blocks an SM and with 32: 16,384 bodies 182 / 176, 65,536 2686 /
 // 2490, 100,003 6166 / 5718, 262,144 40,350 / 39,100; 1PN at 30,000 1382 / 1334.
-// From ASTER_SLICE_MAX_BLOCKS target blocks on (614,400 bodies) one slice: the
-// blocks alone are 16 an SM, and the partial sums would take a gigabyte. Returns
-// the tiles (128 sources) of a slice.
+// From ASTER_SLICE_MAX_BLOCKS target blocks on (614,400 bodies; 307,200 in the
+// mixed post-Newtonian kernel, one target a thread) one slice: the blocks alone are
+// 16 an SM, and the partial sums would take 0.3 to 0.6 GB. Returns the tiles (128
+// sources) of a slice.
 constexpr int64_t ASTER_SLICE_MAX_BLOCKS = 2400;
 inline int64_t aster_slice_tiles(int64_t iblocks, int64_t tiles, int64_t sms) {
     if (tiles < 1) return 1;
