@@ -496,7 +496,7 @@ int aster_allpairs_launch_range(aster_ctx* c, const aster_params* p, int precisi
     if (precision == ASTER_FP64 && !targets_dev && !out_dev && lo == 0 && len == nt && nt == c->n &&
         aster_allpairs_sym_fits(c, p)) {
         const int st = aster_allpairs_sym_launch(c, p, closing_kick, fuse_next);
-        if (st != ASTER_ERR_OOM || fuse_next) return st;
+        if (st != ASTER_ERR_OOM) return st;  // no room for its sums: slices, which take less
     }
     const SliceGrid sg = slice_grid(c, p, precision, nt, len);
     int64_t ns = sg.ns, slice_len = sg.slice_len;

@@ -91,8 +91,31 @@ def test_steps_without_room_run_in_one_piece(prec, tol, steps):
         assert rel_l2(g, r) < tol
 
 
+@pytest.mark.parametrize("steps", [1, 4])
+def test_room_for_slices_alone_takes_slices(steps):
+    """FP64, 180,000 bodies: 381 MB of tile-pair sums do not fit into 260, 184 MB of slices' sums do."""
+    n = 180000
+    pos, vel, m = gen.plummer(n, 48)
+    p = Params(eps2=1e-4, dt=1e-3)
+    out = []
+    for leave in (None, 260 * MB):
+        with Context(0) as c:
+            c.upload(pos, vel, m)
+            if leave is None:
+                c.kdk_steps(p, steps, SOLVER_ALLPAIRS, FP64)
+                kernels = c.stats()["kernels"]
+            else:
+                with Crowd(leave):
+                    c.kdk_steps(p, steps, SOLVER_ALLPAIRS, FP64)
+                    assert c.stats()["kernels"] == kernels  # reductions, and the drifts in them
+            out.append(c.download())
+    assert not np.array_equal(out[0][2], out[1][2])
+    for a, b in zip(*out):
+        assert rel_l2(b, a) < 1e-12
+
+
 def test_room_that_comes_free_is_used():
-    """FP64 forces of 300,000 bodies: 921 MB of tile-pair sums do not fit into 600; once the memory is free again the
+    """FP64 forces of 300,000 bodies: 706 MB of tile-pair sums do not fit into 600; once the memory is free again the
     same context takes the tile pairs (the sums of a fresh context, bit for bit)."""
     n = 300000
     pos, vel, m = gen.plummer(n, 43)
